@@ -16,9 +16,9 @@
 //
 // Field elements live in registers as 8 little-endian 32-bit limbs in
 // Montgomery form (R = 2^256). The modulus is sparse, limbs [1, 0, 0, 0, 0, 0,
-// 17, 2^27], and p = 1 mod 2^32, so the Montgomery quotient digit of each
-// reduction step is -t0 and adding m·p touches limbs 0, 6, 7 and 8. Hashes in
-// memory are the reference's device layout: 32 bytes, big-endian.
+// 17, 2^27], and p = 1 mod 2^192, so 192 bits of a product reduce in one step
+// of shifts and a subtraction. Hashes in memory are the reference's device
+// layout: 32 bytes, big-endian.
 #include "runtime.cuh"
 #include <cstring>
 
@@ -51,78 +51,323 @@ __device__ __forceinline__ void reduce_once(uint32_t t[8]) {
   for (int j = 0; j < 8; j++) t[j] = (t[j] & bw) | (d[j] & ~bw);  // borrow: t < p, keep it
 }
 
-// Montgomery product a·b·R^-1 mod p (CIOS), for a, b < p. Per limb b_i:
-// t += a·b_i, then t += m·p with m = -t0 (p = 1 mod 2^32), which zeroes
-// t0 and touches limbs 6, 7, 8 (17·2^192 and 2^251), then a one-limb shift.
-// t0 + m is 0 with a carry exactly when t0 != 0; that carry is fed into
-// limb 1 directly, and m·17 is formed outside the carry chain, which holds
-// plain add-with-carry only (a chain that mixed multiply-add-with-carry
-// with an immediate operand into the reduction produced wrong carries on
-// sm_100a). After each shift t < 2p < 2^253, so limb 8 is 0 before the next
-// product.
-template <bool FULL>
-__device__ __forceinline__ Felt fmul_t(const Felt& a, const Felt& b) {
-  uint32_t t[10];
-#pragma unroll
-  for (int j = 0; j < 10; j++) t[j] = 0;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    asm("mad.lo.cc.u32 %0, %10, %18, %0;\n\t"
-        "madc.lo.cc.u32 %1, %11, %18, %1;\n\t"
-        "madc.lo.cc.u32 %2, %12, %18, %2;\n\t"
-        "madc.lo.cc.u32 %3, %13, %18, %3;\n\t"
-        "madc.lo.cc.u32 %4, %14, %18, %4;\n\t"
-        "madc.lo.cc.u32 %5, %15, %18, %5;\n\t"
-        "madc.lo.cc.u32 %6, %16, %18, %6;\n\t"
-        "madc.lo.cc.u32 %7, %17, %18, %7;\n\t"
-        "addc.u32 %8, %8, 0;\n\t"
-        "mad.hi.cc.u32 %1, %10, %18, %1;\n\t"
-        "madc.hi.cc.u32 %2, %11, %18, %2;\n\t"
-        "madc.hi.cc.u32 %3, %12, %18, %3;\n\t"
-        "madc.hi.cc.u32 %4, %13, %18, %4;\n\t"
-        "madc.hi.cc.u32 %5, %14, %18, %5;\n\t"
-        "madc.hi.cc.u32 %6, %15, %18, %6;\n\t"
-        "madc.hi.cc.u32 %7, %16, %18, %7;\n\t"
-        "madc.hi.cc.u32 %8, %17, %18, %8;\n\t"
-        "addc.u32 %9, 0, 0;"
-        : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]),
-          "+r"(t[8]), "=r"(t[9])
-        : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]),
-          "r"(a.v[7]), "r"(b.v[i]));
-    // reduction with plain add-with-carry: t0 + m is 0 with a carry exactly
-    // when t0 != 0; m·17 at limb 6 (two words); m·2^251 at limbs 7 and 8
-    const uint32_t m = 0u - t[0];
-    const uint64_t m17 = (uint64_t)m * 17u;
-    asm("add.cc.u32 %0, %0, %9;\n\t"
-        "addc.cc.u32 %1, %1, 0;\n\t"
-        "addc.cc.u32 %2, %2, 0;\n\t"
-        "addc.cc.u32 %3, %3, 0;\n\t"
-        "addc.cc.u32 %4, %4, 0;\n\t"
-        "addc.cc.u32 %5, %5, %10;\n\t"
-        "addc.cc.u32 %6, %6, %11;\n\t"
-        "addc.cc.u32 %7, %7, 0;\n\t"
-        "addc.u32 %8, %8, 0;\n\t"
-        "add.cc.u32 %6, %6, %12;\n\t"
-        "addc.cc.u32 %7, %7, %13;\n\t"
-        "addc.u32 %8, %8, 0;"
-        : "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]), "+r"(t[8]),
-          "+r"(t[9])
-        : "r"(t[0] != 0u ? 1u : 0u), "r"((uint32_t)m17), "r"((uint32_t)(m17 >> 32)), "r"(m << 27), "r"(m >> 5));
-#pragma unroll
-    for (int j = 0; j < 9; j++) t[j] = t[j + 1];
-  }
-  if (FULL) reduce_once(t);
-  Felt r;
-#pragma unroll
-  for (int j = 0; j < 8; j++) r.v[j] = t[j];
-  return r;
+// Products. p = 1 + q·2^192 with q = 2^59 + 17, so the Montgomery reduction
+// needs no product by p: T - x·p with x = the low 192 bits of T is divisible
+// by 2^192 and leaves (T >> 192) - x·q, a shift by 4 added to x, a shift by
+// 59, and one subtraction; a second step takes 64 bits the same way. So a
+// product is a plain 512-bit product, then one lump reduction by R = 2^256.
+//
+// The 512-bit product runs in rows over two accumulators, one for the
+// products that land on even 32-bit columns (E) and one for odd columns (O):
+// neighbouring products of a row then fill separate 64-bit columns, and each
+// is one wide multiply-add with the carry of its row (mad.lo.cc / madc.hi.cc
+// on one column pair): 64 wide multiplies instead of 64 low and 64 high ones,
+// which cost 4 against 2 + 4 issue cycles per warp. A square takes 28 + 8.
+//
+// The subtractions can leave a negative value, so a multiple of p is added to
+// T: k·p·2^256 + p·2^192 (its limbs enter as the starting values of the
+// accumulators' fresh columns, at no instruction). The result is then at
+// least (k - 1)·p and below T / 2^256 + (k + 1/1000)·p.
+//
+// Measured against a limb-by-limb reduction (CIOS, low and high multiplies):
+// 97 k -> 37.7 k warp instructions per permutation, so a lone warp, which a
+// small tree level is, takes 105 -> 60 us (it now waits on the carry chains:
+// 3.1 cycles per instruction, the multiplier busy for half of them), and a
+// Wide-Fibonacci 2^16 x 100 proof over this hash 30.5 -> 16.1 ms.
+
+// Columns t[0..2n) += (a0, a1, ...) · b, one wide multiply-add per pair of
+// columns; in the c forms the carry of the last goes to `top` (= top0 + carry).
+__device__ __forceinline__ void wchain1c(uint32_t* t, uint32_t a0, uint32_t b, uint32_t& top, uint32_t top0) {
+  asm("mad.lo.cc.u32 %0, %3, %4, %0;\n\t"
+      "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+      "addc.u32 %2, %5, 0;"
+      : "+r"(t[0]), "+r"(t[1]), "=r"(top)
+      : "r"(a0), "r"(b), "r"(top0));
+}
+__device__ __forceinline__ void wchain1(uint32_t* t, uint32_t a0, uint32_t b) {
+  asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\t"
+      "madc.hi.u32 %1, %2, %3, %1;"
+      : "+r"(t[0]), "+r"(t[1])
+      : "r"(a0), "r"(b));
+}
+__device__ __forceinline__ void wchain2c(uint32_t* t, uint32_t a0, uint32_t a1, uint32_t b, uint32_t& top, uint32_t top0) {
+  asm("mad.lo.cc.u32 %0, %5, %7, %0;\n\t"
+      "madc.hi.cc.u32 %1, %5, %7, %1;\n\t"
+      "madc.lo.cc.u32 %2, %6, %7, %2;\n\t"
+      "madc.hi.cc.u32 %3, %6, %7, %3;\n\t"
+      "addc.u32 %4, %8, 0;"
+      : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "=r"(top)
+      : "r"(a0), "r"(a1), "r"(b), "r"(top0));
+}
+__device__ __forceinline__ void wchain2(uint32_t* t, uint32_t a0, uint32_t a1, uint32_t b) {
+  asm("mad.lo.cc.u32 %0, %4, %6, %0;\n\t"
+      "madc.hi.cc.u32 %1, %4, %6, %1;\n\t"
+      "madc.lo.cc.u32 %2, %5, %6, %2;\n\t"
+      "madc.hi.u32 %3, %5, %6, %3;"
+      : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3])
+      : "r"(a0), "r"(a1), "r"(b));
+}
+__device__ __forceinline__ void wchain3c(uint32_t* t, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t b, uint32_t& top, uint32_t top0) {
+  asm("mad.lo.cc.u32 %0, %7, %10, %0;\n\t"
+      "madc.hi.cc.u32 %1, %7, %10, %1;\n\t"
+      "madc.lo.cc.u32 %2, %8, %10, %2;\n\t"
+      "madc.hi.cc.u32 %3, %8, %10, %3;\n\t"
+      "madc.lo.cc.u32 %4, %9, %10, %4;\n\t"
+      "madc.hi.cc.u32 %5, %9, %10, %5;\n\t"
+      "addc.u32 %6, %11, 0;"
+      : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "=r"(top)
+      : "r"(a0), "r"(a1), "r"(a2), "r"(b), "r"(top0));
+}
+__device__ __forceinline__ void wchain3(uint32_t* t, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t b) {
+  asm("mad.lo.cc.u32 %0, %6, %9, %0;\n\t"
+      "madc.hi.cc.u32 %1, %6, %9, %1;\n\t"
+      "madc.lo.cc.u32 %2, %7, %9, %2;\n\t"
+      "madc.hi.cc.u32 %3, %7, %9, %3;\n\t"
+      "madc.lo.cc.u32 %4, %8, %9, %4;\n\t"
+      "madc.hi.u32 %5, %8, %9, %5;"
+      : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(b));
+}
+__device__ __forceinline__ void wchain4c(uint32_t* t, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b, uint32_t& top, uint32_t top0) {
+  asm("mad.lo.cc.u32 %0, %9, %13, %0;\n\t"
+      "madc.hi.cc.u32 %1, %9, %13, %1;\n\t"
+      "madc.lo.cc.u32 %2, %10, %13, %2;\n\t"
+      "madc.hi.cc.u32 %3, %10, %13, %3;\n\t"
+      "madc.lo.cc.u32 %4, %11, %13, %4;\n\t"
+      "madc.hi.cc.u32 %5, %11, %13, %5;\n\t"
+      "madc.lo.cc.u32 %6, %12, %13, %6;\n\t"
+      "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"
+      "addc.u32 %8, %14, 0;"
+      : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]), "=r"(top)
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b), "r"(top0));
+}
+__device__ __forceinline__ void wchain4(uint32_t* t, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b) {
+  asm("mad.lo.cc.u32 %0, %8, %12, %0;\n\t"
+      "madc.hi.cc.u32 %1, %8, %12, %1;\n\t"
+      "madc.lo.cc.u32 %2, %9, %12, %2;\n\t"
+      "madc.hi.cc.u32 %3, %9, %12, %3;\n\t"
+      "madc.lo.cc.u32 %4, %10, %12, %4;\n\t"
+      "madc.hi.cc.u32 %5, %10, %12, %5;\n\t"
+      "madc.lo.cc.u32 %6, %11, %12, %6;\n\t"
+      "madc.hi.u32 %7, %11, %12, %7;"
+      : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b));
 }
 
-// Fully reduced product (inputs below 2p): below p.
-__device__ __forceinline__ Felt fmul(const Felt& a, const Felt& b) { return fmul_t<true>(a, b); }
-// Lazy product: for inputs below 5.6p the result a·b/R + (< p) stays below
-// 2p; the permutation keeps every product input below 4.5p.
-__device__ __forceinline__ Felt fmul_l(const Felt& a, const Felt& b) { return fmul_t<false>(a, b); }
+// the same over the eight squares, no carry out
+__device__ __forceinline__ void sqchain8(uint32_t t[16], const Felt& a) {
+  asm("mad.lo.cc.u32 %0, %16, %16, %0;\n\t"
+      "madc.hi.cc.u32 %1, %16, %16, %1;\n\t"
+      "madc.lo.cc.u32 %2, %17, %17, %2;\n\t"
+      "madc.hi.cc.u32 %3, %17, %17, %3;\n\t"
+      "madc.lo.cc.u32 %4, %18, %18, %4;\n\t"
+      "madc.hi.cc.u32 %5, %18, %18, %5;\n\t"
+      "madc.lo.cc.u32 %6, %19, %19, %6;\n\t"
+      "madc.hi.cc.u32 %7, %19, %19, %7;\n\t"
+      "madc.lo.cc.u32 %8, %20, %20, %8;\n\t"
+      "madc.hi.cc.u32 %9, %20, %20, %9;\n\t"
+      "madc.lo.cc.u32 %10, %21, %21, %10;\n\t"
+      "madc.hi.cc.u32 %11, %21, %21, %11;\n\t"
+      "madc.lo.cc.u32 %12, %22, %22, %12;\n\t"
+      "madc.hi.cc.u32 %13, %22, %22, %13;\n\t"
+      "madc.lo.cc.u32 %14, %23, %23, %14;\n\t"
+      "madc.hi.u32 %15, %23, %23, %15;"
+      : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]), "+r"(t[8]),
+        "+r"(t[9]), "+r"(t[10]), "+r"(t[11]), "+r"(t[12]), "+r"(t[13]), "+r"(t[14]), "+r"(t[15])
+      : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]));
+}
+// T[j] = e[j] + o[j - 1], columns 1..15
+__device__ __forceinline__ void add_columns(uint32_t T[16], const uint32_t e[16], const uint32_t o[16]) {
+  asm("add.cc.u32 %0, %15, %30;\n\t"
+      "addc.cc.u32 %1, %16, %31;\n\t"
+      "addc.cc.u32 %2, %17, %32;\n\t"
+      "addc.cc.u32 %3, %18, %33;\n\t"
+      "addc.cc.u32 %4, %19, %34;\n\t"
+      "addc.cc.u32 %5, %20, %35;\n\t"
+      "addc.cc.u32 %6, %21, %36;\n\t"
+      "addc.cc.u32 %7, %22, %37;\n\t"
+      "addc.cc.u32 %8, %23, %38;\n\t"
+      "addc.cc.u32 %9, %24, %39;\n\t"
+      "addc.cc.u32 %10, %25, %40;\n\t"
+      "addc.cc.u32 %11, %26, %41;\n\t"
+      "addc.cc.u32 %12, %27, %42;\n\t"
+      "addc.cc.u32 %13, %28, %43;\n\t"
+      "addc.u32 %14, %29, %44;"
+      : "=&r"(T[1]), "=&r"(T[2]), "=&r"(T[3]), "=&r"(T[4]), "=&r"(T[5]), "=&r"(T[6]), "=&r"(T[7]), "=&r"(T[8]),
+        "=&r"(T[9]), "=&r"(T[10]), "=&r"(T[11]), "=&r"(T[12]), "=&r"(T[13]), "=&r"(T[14]), "=&r"(T[15])
+      : "r"(e[1]), "r"(e[2]), "r"(e[3]), "r"(e[4]), "r"(e[5]), "r"(e[6]), "r"(e[7]), "r"(e[8]), "r"(e[9]), "r"(e[10]),
+        "r"(e[11]), "r"(e[12]), "r"(e[13]), "r"(e[14]), "r"(e[15]), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]),
+        "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]), "r"(o[8]), "r"(o[9]), "r"(o[10]), "r"(o[11]), "r"(o[12]),
+        "r"(o[13]), "r"(o[14]));
+}
+
+// T = a·b + (k·p·2^64 + p)·2^192. a, b < 2^255 with a·b < 2^510.
+template <uint32_t K>
+__device__ __forceinline__ void mul_wide8(const Felt& a, const Felt& b, uint32_t T[16]) {
+  uint32_t e[16], o[16];
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const uint64_t pe = (uint64_t)a.v[2 * j] * b.v[0] + (j == 3 ? 1u : 0u);  // column 6: + 1
+    const uint64_t po = (uint64_t)a.v[2 * j + 1] * b.v[0];
+    e[2 * j] = (uint32_t)pe;
+    e[2 * j + 1] = (uint32_t)(pe >> 32);
+    o[2 * j] = (uint32_t)po;
+    o[2 * j + 1] = (uint32_t)(po >> 32);
+  }
+  e[8] = K;
+#pragma unroll
+  for (int i = 1; i < 8; i++) {
+    // odd rows put their even-limb products on odd columns
+    uint32_t* x = i & 1 ? o : e;
+    uint32_t* y = i & 1 ? e : o;
+    const int xb = i & 1 ? i - 1 : i, yb = i & 1 ? i + 1 : i;
+    wchain4c(x + xb, a.v[0], a.v[2], a.v[4], a.v[6], b.v[i], x[xb + 8], i == 4 ? 17u : i == 6 ? 17u * K : 0u);
+    y[yb + 7] = i == 5 ? 0x08000000u : i == 7 ? K << 27 : 0u;
+    wchain4(y + yb, a.v[1], a.v[3], a.v[5], a.v[7], b.v[i]);
+  }
+  T[0] = e[0];
+  add_columns(T, e, o);
+}
+
+// T = a^2 + 2·(p·2^64 + p)·2^192, a < 2^255. Cross products once, doubled,
+// then the squares in one chain.
+__device__ __forceinline__ void sqr_wide8(const Felt& a, uint32_t T[16]) {
+  uint32_t e[16], o[16], c[16];
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const uint64_t po = (uint64_t)a.v[0] * a.v[2 * j + 1];
+    o[2 * j] = (uint32_t)po;
+    o[2 * j + 1] = (uint32_t)(po >> 32);
+  }
+#pragma unroll
+  for (int j = 1; j < 4; j++) {
+    const uint64_t pe = (uint64_t)a.v[0] * a.v[2 * j] + (j == 3 ? 1u : 0u);  // column 6: + 1
+    e[2 * j] = (uint32_t)pe;
+    e[2 * j + 1] = (uint32_t)(pe >> 32);
+  }
+  e[0] = e[1] = 0;
+  e[8] = 1;
+  e[9] = 0;
+  wchain3c(o + 2, a.v[2], a.v[4], a.v[6], a.v[1], o[8], 0);
+  wchain3(e + 4, a.v[3], a.v[5], a.v[7], a.v[1]);
+  o[9] = 0;
+  wchain3(o + 4, a.v[3], a.v[5], a.v[7], a.v[2]);
+  wchain2c(e + 6, a.v[4], a.v[6], a.v[2], e[10], 0);
+  wchain2c(o + 6, a.v[4], a.v[6], a.v[3], o[10], 0);
+  e[11] = 0;
+  wchain2(e + 8, a.v[5], a.v[7], a.v[3]);
+  o[11] = 0;
+  wchain2(o + 8, a.v[5], a.v[7], a.v[4]);
+  wchain1c(e + 10, a.v[6], a.v[4], e[12], 17u);
+  wchain1c(o + 10, a.v[6], a.v[5], o[12], 0);
+  e[13] = 0x08000000u;
+  wchain1(e + 12, a.v[7], a.v[5]);
+  o[13] = 0;
+  wchain1(o + 12, a.v[7], a.v[6]);
+  o[14] = 0;
+  e[14] = 17u;
+  e[15] = 0x08000000u;
+  c[0] = 0;
+  add_columns(c, e, o);
+  T[0] = 0;
+#pragma unroll
+  for (int j = 15; j >= 1; j--) T[j] = __funnelshift_l(c[j - 1], c[j], 1);
+  sqchain8(T, a);
+}
+
+// (T / 2^256) mod p for T = product + k·p·2^256 + p·2^192, in two steps of 192
+// and 64 bits: T - x·p with x the low bits, x·(2^59 + 17) from shifts.
+__device__ __forceinline__ Felt redc(const uint32_t T[16]) {
+  uint32_t s[8], z[8], r[10];
+  s[0] = T[0] << 4;
+  z[0] = T[0] << 27;
+#pragma unroll
+  for (int j = 1; j < 6; j++) {
+    s[j] = __funnelshift_l(T[j - 1], T[j], 4);
+    z[j] = __funnelshift_l(T[j - 1], T[j], 27);
+  }
+  s[6] = T[5] >> 28;
+  z[6] = T[5] >> 5;
+  // s = 16 x + x, then + x·2^59 (limbs 1..7)
+  asm("add.cc.u32 %0, %0, %7;\n\t"
+      "addc.cc.u32 %1, %1, %8;\n\t"
+      "addc.cc.u32 %2, %2, %9;\n\t"
+      "addc.cc.u32 %3, %3, %10;\n\t"
+      "addc.cc.u32 %4, %4, %11;\n\t"
+      "addc.cc.u32 %5, %5, %12;\n\t"
+      "addc.u32 %6, %6, 0;"
+      : "+r"(s[0]), "+r"(s[1]), "+r"(s[2]), "+r"(s[3]), "+r"(s[4]), "+r"(s[5]), "+r"(s[6])
+      : "r"(T[0]), "r"(T[1]), "r"(T[2]), "r"(T[3]), "r"(T[4]), "r"(T[5]));
+  asm("add.cc.u32 %0, %0, %7;\n\t"
+      "addc.cc.u32 %1, %1, %8;\n\t"
+      "addc.cc.u32 %2, %2, %9;\n\t"
+      "addc.cc.u32 %3, %3, %10;\n\t"
+      "addc.cc.u32 %4, %4, %11;\n\t"
+      "addc.cc.u32 %5, %5, %12;\n\t"
+      "addc.u32 %6, %13, 0;"
+      : "+r"(s[1]), "+r"(s[2]), "+r"(s[3]), "+r"(s[4]), "+r"(s[5]), "+r"(s[6]), "=r"(s[7])
+      : "r"(z[0]), "r"(z[1]), "r"(z[2]), "r"(z[3]), "r"(z[4]), "r"(z[5]), "r"(z[6]));
+  asm("sub.cc.u32 %0, %10, %20;\n\t"
+      "subc.cc.u32 %1, %11, %21;\n\t"
+      "subc.cc.u32 %2, %12, %22;\n\t"
+      "subc.cc.u32 %3, %13, %23;\n\t"
+      "subc.cc.u32 %4, %14, %24;\n\t"
+      "subc.cc.u32 %5, %15, %25;\n\t"
+      "subc.cc.u32 %6, %16, %26;\n\t"
+      "subc.cc.u32 %7, %17, %27;\n\t"
+      "subc.cc.u32 %8, %18, 0;\n\t"
+      "subc.u32 %9, %19, 0;"
+      : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]),
+        "=&r"(r[8]), "=&r"(r[9])
+      : "r"(T[6]), "r"(T[7]), "r"(T[8]), "r"(T[9]), "r"(T[10]), "r"(T[11]), "r"(T[12]), "r"(T[13]), "r"(T[14]),
+        "r"(T[15]), "r"(s[0]), "r"(s[1]), "r"(s[2]), "r"(s[3]), "r"(s[4]), "r"(s[5]), "r"(s[6]), "r"(s[7]));
+  // 64 bits more: y = r[0..1], y·q lands on limbs 6..9
+  uint32_t w0 = r[0] << 4, w1 = __funnelshift_l(r[0], r[1], 4), w2 = r[1] >> 28, w3;
+  asm("add.cc.u32 %0, %0, %3;\n\t"
+      "addc.cc.u32 %1, %1, %4;\n\t"
+      "addc.u32 %2, %2, 0;"
+      : "+r"(w0), "+r"(w1), "+r"(w2)
+      : "r"(r[0]), "r"(r[1]));
+  asm("add.cc.u32 %0, %0, %3;\n\t"
+      "addc.cc.u32 %1, %1, %4;\n\t"
+      "addc.u32 %2, %5, 0;"
+      : "+r"(w1), "+r"(w2), "=r"(w3)
+      : "r"(r[0] << 27), "r"(__funnelshift_l(r[0], r[1], 27)), "r"(r[1] >> 5));
+  Felt f;
+#pragma unroll
+  for (int j = 0; j < 4; j++) f.v[j] = r[2 + j];
+  asm("sub.cc.u32 %0, %4, %8;\n\t"
+      "subc.cc.u32 %1, %5, %9;\n\t"
+      "subc.cc.u32 %2, %6, %10;\n\t"
+      "subc.u32 %3, %7, %11;"
+      : "=&r"(f.v[4]), "=&r"(f.v[5]), "=&r"(f.v[6]), "=&r"(f.v[7])
+      : "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(w0), "r"(w1), "r"(w2), "r"(w3));
+  return f;
+}
+
+// a·b / 2^256 mod p: at least (K - 1)·p, below a·b / 2^256 + (K + 1/1000)·p.
+// The top limb of a stays below 2^31.
+template <uint32_t K>
+__device__ __forceinline__ Felt fmul_k(const Felt& a, const Felt& b) {
+  uint32_t T[16];
+  mul_wide8<K>(a, b, T);
+  return redc(T);
+}
+// Below p, for a·b < 0.9·2^256·p (the product is then below 2p).
+__device__ __forceinline__ Felt fmul(const Felt& a, const Felt& b) {
+  Felt r = fmul_k<1>(a, b);
+  reduce_once(r.v);
+  return r;
+}
+// x^3: at least (K - 1)·p. For x <= 11p (below 2^254.5) the square is below
+// (121/32 + 2 + 1/1000)·p < 5.8p and the cube below (5.8·11/32 + K)·p < (K + 2)·p.
+template <uint32_t K>
+__device__ __forceinline__ Felt fcube(const Felt& x) {
+  uint32_t T[16];
+  sqr_wide8(x, T);
+  return fmul_k<K>(x, redc(T));
+}
+
 
 // a + b without reduction (callers keep the sum below 2^256)
 __device__ __forceinline__ Felt ladd(const Felt& a, const Felt& b) {
@@ -200,88 +445,47 @@ __device__ __forceinline__ Felt fadd(const Felt& a, const Felt& b) {
   return r;
 }
 
-__device__ __forceinline__ Felt fsub(const Felt& a, const Felt& b) {
-  uint32_t t[8], bw;
-  asm("sub.cc.u32 %0, %9, %17;\n\t"
-      "subc.cc.u32 %1, %10, %18;\n\t"
-      "subc.cc.u32 %2, %11, %19;\n\t"
-      "subc.cc.u32 %3, %12, %20;\n\t"
-      "subc.cc.u32 %4, %13, %21;\n\t"
-      "subc.cc.u32 %5, %14, %22;\n\t"
-      "subc.cc.u32 %6, %15, %23;\n\t"
-      "subc.cc.u32 %7, %16, %24;\n\t"
-      "subc.u32 %8, 0, 0;"
-      : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7]), "=r"(bw)
-      : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]),
-        "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]), "r"(b.v[6]), "r"(b.v[7]));
-  // a borrow (a < b): add p back
-  asm("add.cc.u32 %0, %0, %8;\n\t"
-      "addc.cc.u32 %1, %1, 0;\n\t"
-      "addc.cc.u32 %2, %2, 0;\n\t"
-      "addc.cc.u32 %3, %3, 0;\n\t"
-      "addc.cc.u32 %4, %4, 0;\n\t"
-      "addc.cc.u32 %5, %5, 0;\n\t"
-      "addc.cc.u32 %6, %6, %9;\n\t"
-      "addc.u32 %7, %7, %10;"
-      : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7])
-      : "r"(bw & 1u), "r"(bw & 17u), "r"(bw & 0x08000000u));
-  Felt r;
-#pragma unroll
-  for (int j = 0; j < 8; j++) r.v[j] = t[j];
-  return r;
-}
-
-__device__ __forceinline__ Felt fcube(const Felt& x) { return fmul_l(fmul_l(x, x), x); }
-
-// 4p and 6p as plain integers (limbs 0, 6, 7 nonzero)
-__device__ __forceinline__ Felt p_times(uint32_t k) {
-  Felt r{};
-  r.v[0] = k;
-  r.v[6] = 17u * k;
-  r.v[7] = k << 27;
-  return r;
-}
-
-// MDS [[3, 1, 1], [1, -1, 1], [1, 1, -2]] on inputs below 2p:
-// t = s0 + s1 + s2 < 6p; (t + 2 s0, t + 4p - 2 s1, t + 6p - 3 s2), each
-// non-negative and below 12p, brought back below 2p.
-__device__ __forceinline__ void mds(Felt s[3]) {
-  const Felt t = ladd(ladd(s[0], s[1]), s[2]);
-  const Felt s1x2 = ladd(s[1], s[1]);
-  const Felt s2x3 = ladd(ladd(s[2], s[2]), s[2]);
-  const Felt a0 = ladd(t, ladd(s[0], s[0]));
-  const Felt a1 = lsub(ladd(t, p_times(4)), s1x2);
-  const Felt a2 = lsub(ladd(t, p_times(6)), s2x3);
+// MDS [[3, 1, 1], [1, -1, 1], [1, 1, -2]] on s0, s1 < 2p and 2p <= s2 < 5p (a
+// cube with K = 3): s0 + s2 - s1 is non-negative as it stands, and
+// s0 + s1 - 2 s2 is with the 10p that `c` carries besides the next round's
+// constant for s2. s0 and s1 come back below 2p; s2 is left at most
+// 2p + 2p + 11p - 4p = 11p, which the next cube accepts.
+__device__ __forceinline__ void mds(Felt s[3], const Felt& c) {
+  const Felt u = ladd(s[0], s[2]), w = ladd(s[0], s[1]);
+  const Felt a0 = ladd(ladd(u, w), s[0]);
+  const Felt a1 = lsub(u, s[1]);
+  const Felt a2 = lsub(lsub(ladd(w, c), s[2]), s[2]);
   s[0] = lreduce(a0);
   s[1] = lreduce(a1);
-  s[2] = lreduce(a2);
+  s[2] = a2;
 }
 
 // The permutation with compressed partial rounds (one constant each, added
 // to s2; the folded remainder sits in the first of the last 4 full rounds'
 // constants): the same permutation, two constant additions fewer per
-// partial round (poseidon252_constants.py derives and checks the form).
-// Bounds: each round starts below 2p (below 3.5p right after absorbing a
-// block), adding a constant keeps every product input below 4.5p, products
-// return below 2p, and the MDS output is brought back below 2p.
+// partial round (poseidon252_constants.py derives and checks the form). The
+// constant of s2 is added by the MDS before its round.
+// Bounds: the state comes in below 3.5p (below 2p, or after absorbing a
+// block), s0 and s1 enter every cube below 4.5p and s2 below 11p.
 __device__ __forceinline__ void hades(Felt s[3]) {
+  s[2] = ladd(s[2], P252_FULL_RC[2]);
 #pragma unroll 1
-  for (int r = 0; r < 4; r++) {
+  for (int half = 0; half < 2; half++) {
+#pragma unroll 1
+    for (int r = 0; r < 4; r++) {
 #pragma unroll
-    for (int j = 0; j < 3; j++) s[j] = fcube(ladd(s[j], P252_FULL_RC[3 * r + j]));
-    mds(s);
-  }
+      for (int j = 0; j < 2; j++) s[j] = fcube<1>(ladd(s[j], P252_FULL_RC[3 * (4 * half + r) + j]));
+      s[2] = fcube<3>(s[2]);
+      mds(s, P252_S2_NEXT[half ? 87 + r : r]);
+    }
+    if (half == 0)
 #pragma unroll 1
-  for (int k = 0; k < 83; k++) {
-    s[2] = fcube(ladd(s[2], P252_PARTIAL_RC[k]));
-    mds(s);
+      for (int k = 0; k < 83; k++) {
+        s[2] = fcube<3>(s[2]);
+        mds(s, P252_S2_NEXT[4 + k]);
+      }
   }
-#pragma unroll 1
-  for (int r = 4; r < 8; r++) {
-#pragma unroll
-    for (int j = 0; j < 3; j++) s[j] = fcube(ladd(s[j], P252_FULL_RC[3 * r + j]));
-    mds(s);
-  }
+  s[2] = lreduce(s[2]);
 }
 
 // 32 big-endian bytes (as 8 little-endian-stored words) <-> canonical limbs
@@ -295,7 +499,8 @@ __device__ __forceinline__ void to_be_words(const Felt& x, uint32_t w[8]) {
 #pragma unroll
   for (int k = 0; k < 8; k++) w[k] = __byte_perm(x.v[7 - k], 0, 0x0123);
 }
-__device__ __forceinline__ Felt to_mont(const Felt& x) { return fmul_l(x, P252_R2); }  // below 2p
+// any 256-bit x, to below 2p (below 1.1p for x < p)
+__device__ __forceinline__ Felt to_mont(const Felt& x) { return fmul_k<1>(P252_R2, x); }
 __device__ __forceinline__ Felt from_mont(const Felt& x) {
   Felt one{};
   one.v[0] = 1;

@@ -95,6 +95,8 @@ def main():
     for seed in range(4):  # the two forms are the same permutation
         st = [(seed * 1000003 + 7 * j + 1) ** 5 % P for j in range(3)]
         assert permute_plain(st, rcs) == permute_compressed(st, full, part)
+    s2 = [row[2] for row in full[:4]] + part + [row[2] for row in full[4:]]  # s2's constant, by round
+    s2_next = s2[1:] + [0]
     lines = [
         "// Generated by poseidon252_constants.py (do not edit): Starknet Poseidon",
         "// constants, Montgomery form (R = 2^256), 8 little-endian 32-bit limbs.",
@@ -105,9 +107,9 @@ def main():
         "__constant__ Felt P252_FULL_RC[24] = {",
         ",\n".join(felt_line(mont(c)) for row in full for c in row),
         "};",
-        "// one constant per partial round, added to s2",
-        "__constant__ Felt P252_PARTIAL_RC[83] = {",
-        ",\n".join(felt_line(mont(c)) for c in part),
+        "// what the MDS of round r adds to s2: the next round's constant plus 10p (10p alone after the last)",
+        "__constant__ Felt P252_S2_NEXT[91] = {",
+        ",\n".join(felt_line(mont(c) + 10 * P) for c in s2_next),
         "};",
         "",
     ]

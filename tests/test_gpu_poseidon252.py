@@ -46,6 +46,26 @@ def test_permutation_matches_oracle(B):
         assert got[3 * k:3 * k + 3] == PS.permute(s), k
 
 
+# values at which the products' columns, the 192- and 64-bit reduction steps
+# and the final subtraction carry or borrow; the last two are not reduced
+EDGES = [1, (1 << 64) - 1, 1 << 64, (1 << 192) - 1, 1 << 192, (1 << 251) - 1, 1 << 251, PS.P - 1, PS.P - (1 << 192),
+         (PS.P - 1) // 2, PS.P + 1, (1 << 256) - 1]
+
+
+@pytest.mark.parametrize("shift", range(3))
+def test_permutation_edge_states(B, shift):
+    """Edge values in every position, then the outputs permuted again 20 times."""
+    n = len(EDGES)
+    states = [[EDGES[i], EDGES[(i + 1 + shift) % n], EDGES[(i + 4 * shift) % n]] for i in range(n)]
+    raw = b"".join(v.to_bytes(32, "big") for s in states for v in s)
+    dev = torch.tensor(np.frombuffer(raw, dtype=np.uint8).copy(), device="cuda")
+    want = [[v % PS.P for v in s] for s in states]
+    for step in range(20):
+        dev = B.poseidon252_permute(dev)
+        want = [PS.permute(s) for s in want]
+        assert dev_to_felts(dev) == [v for s in want for v in s], step
+
+
 def test_hash_node_known_answers(B):
     a, b = GOLDEN["poseidon252_hash_node"]
     # hash_node(None, [0, 1]): one node, two columns of one row

@@ -210,12 +210,16 @@ int gs_commit_on_layer(gs_ctx* ctx, uint32_t log_size, const uint32_t* prev_laye
                        const uint32_t* const* cols, uint32_t* out) {
   CTX_REQUIRED(ctx);
   const void* const* d = nullptr;
+  bool aligned = true;
   if (n_cols) {
     GS_REQUIRE(cols != nullptr, "null column list");
-    for (uint32_t i = 0; i < n_cols; i++) GS_REQUIRE(cols[i] != nullptr, "null column");
+    for (uint32_t i = 0; i < n_cols; i++) {
+      GS_REQUIRE(cols[i] != nullptr, "null column");
+      aligned = aligned && ((uintptr_t)cols[i] & 15) == 0;
+    }
     GS_TRY(ctx->c.stage_ptrs((const void* const*)cols, n_cols, &d));
   }
-  return commit_on_layer(ctx->c.stream, log_size, prev_layer, (const uint32_t* const*)d, n_cols, out);
+  return commit_on_layer(ctx->c.stream, log_size, prev_layer, (const uint32_t* const*)d, n_cols, out, aligned);
 }
 
 int gs_merkle_worklist(gs_ctx* ctx, const gs_merkle_item* items, uint32_t n_items) {

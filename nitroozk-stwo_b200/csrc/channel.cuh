@@ -16,48 +16,60 @@
 
 namespace gs {
 
-__device__ __forceinline__ void channel_mix_root_draw_dev(uint32_t* state, const uint32_t* root, uint32_t* root_copy,
-                                                          uint32_t* felt_out) {
-  uint32_t m[16], d[8];
+// The step is two compressions whose messages lie in shared memory, so that a
+// kernel runs them through the same compression its tree levels use (one copy
+// of the unrolled rounds stays in the instruction cache; a lone warp that runs
+// into another copy waits for its instructions).
+struct ChannelWords {
+  uint4 mix[4];   // digest, root
+  uint4 draw[4];  // digest, draws so far, zeros
+};
+constexpr uint32_t CHANNEL_MIX_BYTES = 64, CHANNEL_DRAW_BYTES = 37;
+
+__device__ __forceinline__ void channel_begin(ChannelWords& w, const uint32_t* state) {  // one thread
+  w.mix[0] = make_uint4(state[0], state[1], state[2], state[3]);
+  w.mix[1] = make_uint4(state[4], state[5], state[6], state[7]);
+  w.draw[3] = make_uint4(0, 0, 0, 0);
+}
+__device__ __forceinline__ void channel_root(ChannelWords& w, const uint32_t h[8]) {  // one thread
+  w.mix[2] = make_uint4(h[0], h[1], h[2], h[3]);
+  w.mix[3] = make_uint4(h[4], h[5], h[6], h[7]);
+}
+// h: the hash of the mix message, the new digest (one thread).
+__device__ __forceinline__ void channel_mixed(ChannelWords& w, const uint32_t h[8], uint32_t* state) {
+  w.mix[0] = w.draw[0] = make_uint4(h[0], h[1], h[2], h[3]);
+  w.mix[1] = w.draw[1] = make_uint4(h[4], h[5], h[6], h[7]);
+  w.draw[2] = make_uint4(0, 0, 0, 0);
 #pragma unroll
-  for (int j = 0; j < 8; j++) {
-    m[j] = state[j];
-    m[8 + j] = root[j];
+  for (int j = 0; j < 8; j++) state[j] = h[j];
+}
+// h: the hash of the draw message after `draws` earlier ones. The same answer
+// in every thread that holds h: true when the draw is done (the felt taken, or
+// given up), false when it goes on with draws + 1; `one_thread` stores. A draw
+// is rejected with probability < 2^-27; 64 rejections in a row do not happen
+// for a hash, and running out is reported, never looped on.
+__device__ __forceinline__ bool channel_drawn(ChannelWords& w, const uint32_t h[8], uint32_t draws, bool one_thread,
+                                              uint32_t* state, uint32_t* felt_out, qm31& a) {
+  bool ok = true;
+#pragma unroll
+  for (int j = 0; j < 8; j++) ok = ok && h[j] < 2u * P;
+  if (!ok && draws + 1 < 64) {
+    if (one_thread) w.draw[2].x = draws + 1;
+    return false;
   }
-  blake2s_init(d);
-  blake2s_compress(d, m, 64, true);
-  if (root_copy)
-    for (int j = 0; j < 8; j++) root_copy[j] = root[j];
-  uint32_t n_draws = 0;
-  // A draw is rejected with probability < 2^-27; 64 rejections in a row do
-  // not happen for a hash, and running out is reported, never looped on.
-  for (int attempt = 0; attempt < 64; attempt++) {
-    uint32_t h[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) m[j] = d[j];
-    m[8] = n_draws;
-#pragma unroll
-    for (int j = 9; j < 16; j++) m[j] = 0;
-    blake2s_init(h);
-    blake2s_compress(h, m, 37, true);
-    n_draws++;
-    bool ok = true;
-#pragma unroll
-    for (int j = 0; j < 8; j++) ok = ok && h[j] < 2u * P;
-    if (ok) {
-      qm31 a = qm_make(h[0] >= P ? h[0] - P : h[0], h[1] >= P ? h[1] - P : h[1], h[2] >= P ? h[2] - P : h[2],
-                       h[3] >= P ? h[3] - P : h[3]);
-      qm31 a2 = qm_mul(a, a);
+  a = qm_make(h[0] >= P ? h[0] - P : h[0], h[1] >= P ? h[1] - P : h[1], h[2] >= P ? h[2] - P : h[2],
+              h[3] >= P ? h[3] - P : h[3]);
+  if (one_thread) {
+    if (ok) {  // the challenge, then its square
+      const qm31 a2 = qm_mul(a, a);
       felt_out[0] = a.x.a; felt_out[1] = a.x.b; felt_out[2] = a.y.a; felt_out[3] = a.y.b;
       felt_out[4] = a2.x.a; felt_out[5] = a2.x.b; felt_out[6] = a2.y.a; felt_out[7] = a2.y.b;
-      for (int j = 0; j < 8; j++) state[j] = d[j];
-      state[8] = n_draws;
-      return;
+    } else {
+      state[9] = 1;
     }
+    state[8] = draws + 1;
   }
-  for (int j = 0; j < 8; j++) state[j] = d[j];
-  state[8] = n_draws;
-  state[9] = 1;
+  return true;
 }
 
 }  // namespace gs

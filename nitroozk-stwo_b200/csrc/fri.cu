@@ -21,13 +21,11 @@
 
 namespace gs {
 
-__device__ __forceinline__ void leaf_hash4(uint32_t* leaf_out, size_t i, qm31 v) {
+__device__ __forceinline__ void leaf_hash4(uint32_t* leaf_out, size_t i, qm31 v, uint32_t one) {
   uint32_t h[8], m[16];
   blake2s_init(h);
   m[0] = v.x.a; m[1] = v.x.b; m[2] = v.y.a; m[3] = v.y.b;
-#pragma unroll
-  for (int j = 4; j < 16; j++) m[j] = 0;
-  blake2s_compress(h, m, 16, true);
+  blake2s_compress_f<4>(h, m, 16, true, one);
   uint4* o = reinterpret_cast<uint4*>(leaf_out + 8 * i);
   o[0] = make_uint4(h[0], h[1], h[2], h[3]);
   o[1] = make_uint4(h[4], h[5], h[6], h[7]);
@@ -51,7 +49,7 @@ __device__ __forceinline__ void load_pair(CPlanes s, size_t i, qm31& a, qm31& b)
 // d_alpha (optional): the challenge in device memory (4 words, then alpha^2),
 // written by the device channel; overrides `alpha`.
 __global__ void fold_line_kernel(CPlanes src, uint32_t log_n, qm31 alpha, Planes dst, const uint32_t* __restrict__ itw,
-                                 uint32_t tw_len, uint32_t* leaf_out, const uint32_t* __restrict__ d_alpha) {
+                                 uint32_t tw_len, uint32_t* leaf_out, const uint32_t* __restrict__ d_alpha, uint32_t one) {
   const size_t half = (size_t)1 << (log_n - 1);
   if (d_alpha) alpha = qm_make(d_alpha[0], d_alpha[1], d_alpha[2], d_alpha[3]);
   const uint32_t* lvl = itw + (tw_len - (1u << log_n));
@@ -63,7 +61,7 @@ __global__ void fold_line_kernel(CPlanes src, uint32_t log_n, qm31 alpha, Planes
     qm31 f1 = qm_mul_m31(qm_sub(fx, fnx), xinv);
     qm31 r = qm_add(f0, qm_mul(alpha, f1));
     dst.p[0][i] = r.x.a; dst.p[1][i] = r.x.b; dst.p[2][i] = r.y.a; dst.p[3][i] = r.y.b;
-    if (leaf_out) leaf_hash4(leaf_out, i, r);
+    if (leaf_out) leaf_hash4(leaf_out, i, r, one);
   }
 }
 
@@ -71,7 +69,7 @@ struct SmallInvY { uint32_t v[2]; };
 
 __global__ void fold_circle_kernel(CPlanes src, uint32_t log_n, qm31 alpha, qm31 alpha_sq, Planes dst,
                                    const uint32_t* __restrict__ itw, uint32_t tw_len, SmallInvY small,
-                                   uint32_t* leaf_out, const uint32_t* __restrict__ d_alpha) {
+                                   uint32_t* leaf_out, const uint32_t* __restrict__ d_alpha, uint32_t one) {
   const size_t half = (size_t)1 << (log_n - 1);
   if (d_alpha) {
     alpha = qm_make(d_alpha[0], d_alpha[1], d_alpha[2], d_alpha[3]);
@@ -95,7 +93,7 @@ __global__ void fold_circle_kernel(CPlanes src, uint32_t log_n, qm31 alpha, qm31
     qm31 d = qm_make(dst.p[0][i], dst.p[1][i], dst.p[2][i], dst.p[3][i]);
     qm31 r = qm_add(qm_mul(d, alpha_sq), fprime);
     dst.p[0][i] = r.x.a; dst.p[1][i] = r.x.b; dst.p[2][i] = r.y.a; dst.p[3][i] = r.y.b;
-    if (leaf_out) leaf_hash4(leaf_out, i, r);
+    if (leaf_out) leaf_hash4(leaf_out, i, r, one);
   }
 }
 
@@ -110,7 +108,7 @@ static int fold_line_launch(cudaStream_t st, CPlanes src, uint32_t log_n, qm31 a
   GS_REQUIRE(log_n >= 1 && log_n <= tw_log, "fold_line: line domain must fit the twiddle tree");
   size_t half = (size_t)1 << (log_n - 1);
   fold_line_kernel<<<grid_for(half, 256), 256, 0, st>>>(src, log_n, alpha, dst, d_itw, 1u << tw_log, leaf_out,
-                                                        d_alpha);
+                                                        d_alpha, 1u);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;
@@ -150,7 +148,7 @@ static int fold_circle_launch(cudaStream_t st, CPlanes src, uint32_t log_n, qm31
   qm31 alpha_sq = qm_mul(alpha, alpha);
   size_t half = (size_t)1 << (log_n - 1);
   fold_circle_kernel<<<grid_for(half, 256), 256, 0, st>>>(src, log_n, alpha, alpha_sq, dst, d_itw, 1u << tw_log, small,
-                                                          leaf_out, d_alpha);
+                                                          leaf_out, d_alpha, 1u);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;
@@ -179,84 +177,99 @@ int fold_circle_into_line_dev_alpha(cudaStream_t st, CPlanes src, uint32_t log_n
 // QM31 each): 128 KiB.
 constexpr uint32_t TAIL_CTA_SMEM = 8192 * 16;
 __global__ void __launch_bounds__(1024) fri_tail_cta_kernel(FriTail a, uint32_t* state,
-                                                            const uint32_t* __restrict__ itw, uint32_t tw_len) {
+                                                            const uint32_t* __restrict__ itw, uint32_t tw_len,
+                                                            uint32_t one) {
   extern __shared__ uint4 tsm[];
-  __shared__ uint32_t alpha_s[4];
-  uint4* nb[2] = {tsm, tsm + 2048};
-  uint4* leaves = tsm + 4096;
-  uint4* vals[2] = {tsm + 6144, tsm + 7168};
+  __shared__ ChannelWords ch;
+  __shared__ uint4 alpha_s;
+  uint4* const leaves = tsm + 4096;
+  auto nb = [&](int i) { return tsm + 2048 * i; };              // two node-hash buffers
+  auto vals = [&](uint32_t i) { return tsm + 6144 + 1024 * i; };  // this layer's and the next one's values
   const uint32_t tid = threadIdx.x;
+  if (tid == 0) channel_begin(ch, state);  // read by warp 0 after a root
   for (uint32_t k = 0; k < a.n; k++) {
-    const uint32_t log = a.log0 - k;
+    const uint32_t log = a.log0 - k, half = 1u << (log - 1);
     uint32_t* const* tree = a.tree[k];
     int cur = 0;
-    for (int L = (int)log - 1; L >= 0; L--) {
-      if (tid < (1u << L)) {
+    uint32_t draws = 0;
+    // s >= 0: the 2^s nodes of level s, one per thread; -1, -2: the channel's
+    // mix and draw; -3: the fold and the next layer's leaves. One compression
+    // serves all of them. Levels of at most 32 nodes and the channel are warp
+    // 0's alone, without block barriers; its lanes past the level's nodes
+    // hash words nobody uses.
+    for (int s = (int)log - 1; s >= -3;) {
+      const bool lone = s <= 5 && s > -3;
+      const uint32_t n = s >= 0 ? 1u << s : s == -3 ? half : 1u;
+      if (lone ? tid < 32 : tid < n) {
         uint4 c[4];
-        if (L == (int)log - 1) {
-          if (k == 0) {  // leaves hashed by the previous kernel
-            const uint4* src = reinterpret_cast<const uint4*>(tree[log]) + 4 * (size_t)tid;
-#pragma unroll
-            for (int q = 0; q < 4; q++) c[q] = __ldg(src + q);
+        if (s == -3) {
+          qm31 fx, fnx;
+          if (k == 0) {  // layer 0's values come from the previous kernel
+            uint32_t* const* sp = a.planes[0];
+            fx = qm_make(__ldg(sp[0] + 2 * tid), __ldg(sp[1] + 2 * tid), __ldg(sp[2] + 2 * tid),
+                         __ldg(sp[3] + 2 * tid));
+            fnx = qm_make(__ldg(sp[0] + 2 * tid + 1), __ldg(sp[1] + 2 * tid + 1), __ldg(sp[2] + 2 * tid + 1),
+                          __ldg(sp[3] + 2 * tid + 1));
           } else {
-#pragma unroll
-            for (int q = 0; q < 4; q++) c[q] = leaves[4 * tid + q];
+            const uint4 u = vals(k & 1)[2 * tid], v = vals(k & 1)[2 * tid + 1];
+            fx = qm_make(u.x, u.y, u.z, u.w);
+            fnx = qm_make(v.x, v.y, v.z, v.w);
           }
+          const qm31 alpha = qm_make(alpha_s.x, alpha_s.y, alpha_s.z, alpha_s.w);
+          const uint32_t xinv = __ldg(itw + (tw_len - (1u << log)) + tid);
+          const qm31 f0 = qm_add(fx, fnx);
+          const qm31 f1 = qm_mul_m31(qm_sub(fx, fnx), xinv);
+          const qm31 r = qm_add(f0, qm_mul(alpha, f1));
+          uint32_t* const* dp = a.planes[k + 1];
+          dp[0][tid] = r.x.a; dp[1][tid] = r.x.b; dp[2][tid] = r.y.a; dp[3][tid] = r.y.b;
+          c[0] = make_uint4(r.x.a, r.x.b, r.y.a, r.y.b);
+          c[1] = c[2] = c[3] = make_uint4(0, 0, 0, 0);
+          vals((k + 1) & 1)[tid] = c[0];
+        } else if (s == (int)log - 1 && k == 0) {  // leaves hashed by the previous kernel
+          const uint4* src = reinterpret_cast<const uint4*>(tree[log]) + 4 * (size_t)(tid < n ? tid : 0);
+#pragma unroll
+          for (int q = 0; q < 4; q++) c[q] = __ldg(src + q);
         } else {
+          const uint4* src = s >= 0 ? (s == (int)log - 1 ? leaves : nb(cur ^ 1)) + 4 * tid : s == -1 ? ch.mix : ch.draw;
 #pragma unroll
-          for (int q = 0; q < 4; q++) c[q] = nb[cur ^ 1][4 * tid + q];
+          for (int q = 0; q < 4; q++) c[q] = src[q];
         }
-        uint32_t h[8];
-        hash_children16(c, h);
-        tail_store_hash(tree[L], tid, h);
-        nb[cur][2 * tid] = make_uint4(h[0], h[1], h[2], h[3]);
-        nb[cur][2 * tid + 1] = make_uint4(h[4], h[5], h[6], h[7]);
-      }
-      __syncthreads();
-      cur ^= 1;
-    }
-    if (tid == 0) {  // the root sits in the buffer of the last level
-      const uint32_t* f = a.felts + 8 * k;
-      channel_mix_root_draw_dev(state, reinterpret_cast<const uint32_t*>(nb[cur ^ 1]), a.roots + 8 * k,
-                                a.felts + 8 * k);
+        if (s > -3 || k + 1 < a.n) {  // (the last layer has no leaves)
+          uint32_t h[8];
+          hash_block16(c, s == -2 ? CHANNEL_DRAW_BYTES : s == -3 ? 16u : 64u, h, one);
+          if ((s >= 0 || s == -3) && tid < n) {
+            tail_store_hash(s >= 0 ? tree[s] : a.tree[k + 1][log - 1], tid, h);
+            uint4* to = s >= 0 ? nb(cur) : leaves;
+            to[2 * tid] = make_uint4(h[0], h[1], h[2], h[3]);
+            to[2 * tid + 1] = make_uint4(h[4], h[5], h[6], h[7]);
+          }
+          if (s <= 0 && s > -3) {
+            if (s == 0 && tid == 0) {
 #pragma unroll
-      for (int j = 0; j < 4; j++) alpha_s[j] = f[j];
-    }
-    __syncthreads();
-    const qm31 alpha = qm_make(alpha_s[0], alpha_s[1], alpha_s[2], alpha_s[3]);
-    const uint32_t half = 1u << (log - 1);
-    if (tid < half) {
-      qm31 fx, fnx;
-      if (k == 0) {  // layer 0's values come from the previous kernel
-        uint32_t* const* sp = a.planes[0];
-        fx = qm_make(__ldg(sp[0] + 2 * tid), __ldg(sp[1] + 2 * tid), __ldg(sp[2] + 2 * tid), __ldg(sp[3] + 2 * tid));
-        fnx = qm_make(__ldg(sp[0] + 2 * tid + 1), __ldg(sp[1] + 2 * tid + 1), __ldg(sp[2] + 2 * tid + 1),
-                      __ldg(sp[3] + 2 * tid + 1));
+              for (int j = 0; j < 8; j++) a.roots[8 * k + j] = h[j];
+              channel_root(ch, h);
+            }
+            if (s == -1 && tid == 0) channel_mixed(ch, h, state);
+            if (s == -2) {
+              qm31 felt;
+              if (!channel_drawn(ch, h, draws, tid == 0, state, a.felts + 8 * k, felt)) {
+                draws++;
+                __syncwarp();
+                continue;
+              }
+              if (tid == 0) alpha_s = make_uint4(felt.x.a, felt.x.b, felt.y.a, felt.y.b);
+            }
+          }
+        }
+      }
+      if (lone && s != -2) {  // warp 0 goes on; the others wait for the challenge
+        if (tid < 32) __syncwarp();
       } else {
-        const uint4 u = vals[k & 1][2 * tid], v = vals[k & 1][2 * tid + 1];
-        fx = qm_make(u.x, u.y, u.z, u.w);
-        fnx = qm_make(v.x, v.y, v.z, v.w);
+        __syncthreads();
       }
-      const uint32_t xinv = __ldg(itw + (tw_len - (1u << log)) + tid);
-      const qm31 f0 = qm_add(fx, fnx);
-      const qm31 f1 = qm_mul_m31(qm_sub(fx, fnx), xinv);
-      const qm31 r = qm_add(f0, qm_mul(alpha, f1));
-      uint32_t* const* dp = a.planes[k + 1];
-      dp[0][tid] = r.x.a; dp[1][tid] = r.x.b; dp[2][tid] = r.y.a; dp[3][tid] = r.y.b;
-      vals[(k + 1) & 1][tid] = make_uint4(r.x.a, r.x.b, r.y.a, r.y.b);
-      if (k + 1 < a.n) {  // the next layer's leaf
-        uint32_t h[8], m[16];
-        blake2s_init(h);
-        m[0] = r.x.a; m[1] = r.x.b; m[2] = r.y.a; m[3] = r.y.b;
-#pragma unroll
-        for (int j = 4; j < 16; j++) m[j] = 0;
-        blake2s_compress(h, m, 16, true);
-        tail_store_hash(a.tree[k + 1][log - 1], tid, h);
-        leaves[2 * tid] = make_uint4(h[0], h[1], h[2], h[3]);
-        leaves[2 * tid + 1] = make_uint4(h[4], h[5], h[6], h[7]);
-      }
+      cur ^= 1;
+      s--;
     }
-    __syncthreads();
   }
 }
 
@@ -267,7 +280,7 @@ int fri_tail(cudaStream_t st, const FriTail& a, uint32_t* d_state, const uint32_
   static const cudaError_t attr =
       cudaFuncSetAttribute(fri_tail_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_CTA_SMEM);
   GS_CUDA_TRY(attr);
-  fri_tail_cta_kernel<<<1, 1024, TAIL_CTA_SMEM, st>>>(a, d_state, d_itw, 1u << tw_log);
+  fri_tail_cta_kernel<<<1, 1024, TAIL_CTA_SMEM, st>>>(a, d_state, d_itw, 1u << tw_log, 1u);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;

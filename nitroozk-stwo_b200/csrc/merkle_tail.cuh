@@ -15,14 +15,15 @@ __device__ __forceinline__ void tail_store_hash(uint32_t* out, size_t i, const u
   o[1] = make_uint4(h[4], h[5], h[6], h[7]);
 }
 
-__device__ __forceinline__ void hash_children16(const uint4* c, uint32_t h[8]) {
+// Blake2s of one message block (two child hashes: 64 bytes).
+__device__ __forceinline__ void hash_block16(const uint4* c, uint32_t bytes, uint32_t h[8], uint32_t one) {
   uint32_t m[16];
 #pragma unroll
   for (int q = 0; q < 4; q++) {
     m[4 * q] = c[q].x; m[4 * q + 1] = c[q].y; m[4 * q + 2] = c[q].z; m[4 * q + 3] = c[q].w;
   }
   blake2s_init(h);
-  blake2s_compress(h, m, 64, true);
+  blake2s_compress_f(h, m, bytes, true, one);
 }
 
 // The subtree part for a tree with `top` <= 11, run by every CTA of the
@@ -30,7 +31,7 @@ __device__ __forceinline__ void hash_children16(const uint4* c, uint32_t h[8]) {
 // the top layer was written earlier in the same kernel by other CTAs (read
 // at L2, not through the non-coherent path).
 __device__ __forceinline__ void cluster_tree_levels(uint32_t top, uint32_t* const* layer, bool fresh_top, uint4 (*buf)[256],
-                                    cg::cluster_group& cluster) {
+                                    cg::cluster_group& cluster, uint32_t one) {
   const uint32_t rank = cluster.block_rank();
   const uint32_t tid = threadIdx.x;
   const int split = top >= 4 ? 3 : (int)top;
@@ -49,7 +50,7 @@ __device__ __forceinline__ void cluster_tree_levels(uint32_t top, uint32_t* cons
         for (int q = 0; q < 4; q++) c[q] = buf[cur ^ 1][4 * j + q];
       }
       uint32_t h[8];
-      hash_children16(c, h);
+      hash_block16(c, 64, h, one);
       tail_store_hash(layer[L], base + j, h);
       buf[cur][2 * j] = make_uint4(h[0], h[1], h[2], h[3]);
       buf[cur][2 * j + 1] = make_uint4(h[4], h[5], h[6], h[7]);
@@ -66,7 +67,7 @@ __device__ __forceinline__ void cluster_tree_levels(uint32_t top, uint32_t* cons
 #pragma unroll
         for (int q = 0; q < 4; q++) c[q] = __ldcg(src + q);
         uint32_t h[8];
-        hash_children16(c, h);
+        hash_block16(c, 64, h, one);
         tail_store_hash(layer[L], i, h);
       }
       __syncthreads();

@@ -78,7 +78,7 @@ int CommitPlan::enqueue(bool inputs_aligned) {
     const uint32_t* prev = L == max_eval ? nullptr : layers[L + 1];
     if (inj || L == max_eval) {
       GS_TRY(commit_on_layer(st, L, prev, inj ? (const uint32_t* const*)inj->d_evals : nullptr,
-                             inj ? (uint32_t)inj->cols.size() : 0, layers[L]));
+                             inj ? (uint32_t)inj->cols.size() : 0, layers[L], true));  // carved at 256 bytes
       if (L == 0) break;
       L--;
       continue;
@@ -90,7 +90,7 @@ int CommitPlan::enqueue(bool inputs_aligned) {
       break;
     }
     while (L > stop) {
-      GS_TRY(commit_on_layer(st, L, layers[L + 1], nullptr, 0, layers[L]));
+      GS_TRY(commit_on_layer(st, L, layers[L + 1], nullptr, 0, layers[L], true));
       L--;
     }
   }

@@ -158,7 +158,7 @@ int fri_commit(Prover& pv, uint32_t* quot[4], uint32_t lifting, FriLayerDev& fir
     std::vector<const uint32_t*> cols = {quot[0], quot[1], quot[2], quot[3]};
     const uint32_t* const* tab = nullptr;
     GS_TRY(pv.table(cols, &tab));
-    GS_TRY(commit_on_layer(st, lifting, nullptr, tab, 4, first.layers[lifting]));
+    GS_TRY(commit_on_layer(st, lifting, nullptr, tab, 4, first.layers[lifting], true));
   }
   GS_TRY(commit_node_layers_ch(st, first.log, first.layers.data(), pv.ctx.tree_counters, ctl, d_roots, d_felts));
   // fold the circle evaluation into the first line layer (zero-initialised)

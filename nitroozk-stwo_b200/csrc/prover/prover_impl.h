@@ -127,7 +127,7 @@ struct Prover {
         GS_TRY(poseidon252_commit_on_layer(st, (uint32_t)L, (const uint8_t*)t.layers[L + 1], nullptr, 0,
                                            (uint8_t*)t.layers[L]));
     } else {
-      GS_TRY(commit_on_layer(st, t.eval_log, nullptr, tab, t.n_cols, t.layers[t.eval_log]));
+      GS_TRY(commit_on_layer(st, t.eval_log, nullptr, tab, t.n_cols, t.layers[t.eval_log], true));
       if (ctx.d_mail) {  // the tree kernel writes the root into mailbox slot 0 itself
         GS_TRY(commit_node_layers_to(st, t.eval_log, t.layers.data(), ctx.tree_counters, (uint32_t*)ctx.d_mail));
         return ctx.mail_record(0);

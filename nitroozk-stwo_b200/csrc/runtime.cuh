@@ -230,8 +230,9 @@ int fft_autotune(cudaStream_t st, uint32_t lo, uint32_t hi, uint32_t max_ext, co
                  uint32_t tw_log, uint32_t* out_tile, uint32_t* out_coalesce);
 
 // merkle.cu
+// cols_aligned: every column pointer of the table is 16-byte aligned.
 int commit_on_layer(cudaStream_t st, uint32_t log_size, const uint32_t* d_prev, const uint32_t* const* d_cols,
-                    uint32_t n_cols, uint32_t* d_out);
+                    uint32_t n_cols, uint32_t* d_out, bool cols_aligned = false);
 // All node-only layers below `top_log` (layers[L] has 2^L hashes, layers[top_log] given),
 // in one launch up to TREE_MAX_LOG. d_counters: TREE_COUNTERS zeroed words
 // owned by the calling stream (left zeroed); no two launches that share them

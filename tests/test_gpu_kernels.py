@@ -103,6 +103,21 @@ def test_commit_on_layer(B, n_cols, with_prev):
     assert np.array_equal(host(out).view(np.uint8).reshape(-1, 32), expect)
 
 
+# the staged-column layer kernel at its smallest size (one warp of 32 rows),
+# below it, at partial blocks of warps, with warps that walk a second tile
+# (2^18), full and partial message blocks; off = 1 word: misaligned columns
+@pytest.mark.parametrize("log_size,n_cols,with_prev,off", [
+    (4, 17, True, 0), (5, 1, False, 0), (5, 16, True, 0), (6, 17, False, 0), (7, 32, True, 0), (8, 33, False, 0),
+    (5, 17, False, 1), (9, 31, True, 1), (18, 17, False, 0), (18, 5, True, 0)])
+def test_commit_on_layer_staged_columns(B, log_size, n_cols, with_prev, off):
+    rng = np.random.default_rng(log_size * 64 + n_cols)
+    cols = [rand_m31(rng, 1 << log_size) for _ in range(n_cols)]
+    prev = rng.integers(0, 256, (1 << (log_size + 1)) * 32, dtype=np.uint8) if with_prev else None
+    dcols = [dev(np.concatenate([np.zeros(off, np.uint32), c]))[off:] for c in cols]
+    out = B.commit_on_layer(log_size, dev(prev.view(np.uint32)) if with_prev else None, dcols)
+    assert np.array_equal(host(out).view(np.uint8).reshape(-1, 32), O.commit_on_layer(log_size, prev, cols))
+
+
 def test_merkle_root_of_mixed_sizes(B):
     """Full commit with columns injected at their own layer (prover/vcs/prover.rs:22-48)."""
     rng = np.random.default_rng(9)

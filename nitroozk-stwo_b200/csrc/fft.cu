@@ -102,6 +102,20 @@ __device__ __forceinline__ void bfly(uint32_t& a, uint32_t& b, uint32_t w) {
   }
 }
 
+// The same with the twiddle already doubled.
+template <bool INV>
+__device__ __forceinline__ void bfly_b2(uint32_t& a, uint32_t& b, uint32_t w2) {
+  if (INV) {
+    uint32_t t0 = a;
+    a = add(t0, b);
+    b = mul_b2(sub(t0, b), w2);
+  } else {
+    uint32_t t0 = mul_b2(b, w2);
+    b = sub(a, t0);
+    a = add(a, t0);
+  }
+}
+
 // XOR swizzle over the block's shared-memory index (tile offset included, so
 // blocks holding several small tiles stay conflict free as well).
 __device__ __forceinline__ uint32_t swz(uint32_t e) { return e ^ ((e >> 5) & 31u); }
@@ -215,32 +229,15 @@ __global__ void __launch_bounds__(256) fft_pass_kernel(const uint32_t* const* __
 //    for disjoint bit fields the padding is additive, so the offset of
 //    element q folds into the load/store's immediate and each access costs
 //    no address arithmetic — and every access pattern of the pass stays
-//    bank-conflict free (bank = lane);
-//  * the first add of every field add/sub is an IMAD with a runtime 1 / -1
-//    (the integer ALU pipe is the bottleneck of the butterfly; IMAD runs on
-//    the FMA pipe), leaving one add-then-min (VIADDMNMX) per add/sub on the
-//    ALU pipe.
+//    bank-conflict free (bank = lane).
+// (The adds' pipes: m31.cuh.)
 // ---------------------------------------------------------------------------
-// (imad_u32, add_f, sub_f: m31.cuh)
-template <bool INV>
-__device__ __forceinline__ void bfly_f(uint32_t& a, uint32_t& b, uint32_t w, uint32_t one, uint32_t neg1) {
-  if (INV) {
-    uint32_t t0 = a;
-    a = add_f(t0, b, one);
-    b = mul(sub_f(t0, b, neg1), w);
-  } else {
-    uint32_t t0 = mul(b, w);
-    b = sub_f(a, t0, neg1);
-    a = add_f(a, t0, one);
-  }
-}
 __host__ __device__ constexpr uint32_t padw(uint32_t e) { return e + (e >> 5); }
 
 template <bool INV, int L, int C>
 __global__ void __launch_bounds__(256) fft_tile_kernel(const uint32_t* const* __restrict__ src_tab,
                                                        uint32_t* const* __restrict__ dst_tab,
-                                                       const uint32_t* __restrict__ tw, FftPass a, uint32_t one,
-                                                       uint32_t neg1) {
+                                                       const uint32_t* __restrict__ tw, FftPass a) {
   extern __shared__ uint32_t sm[];
   constexpr int R = 5, NQ = 32;
   constexpr int T = L + C;
@@ -316,7 +313,7 @@ __global__ void __launch_bounds__(256) fft_tile_kernel(const uint32_t* const* __
 #pragma unroll
       for (int q = 0; q < NQ; q++) {
         if (q & (1 << j)) continue;
-        bfly_f<INV>(x[q], x[q | (1 << j)], w[q >> (j + 1)], one, neg1);
+        bfly<INV>(x[q], x[q | (1 << j)], w[q >> (j + 1)]);
       }
     }
     if (k + 1 < K) {
@@ -336,6 +333,256 @@ __global__ void __launch_bounds__(256) fft_tile_kernel(const uint32_t* const* __
         const uint32_t stride = 1u << (s0 - C + a.lo);
 #pragma unroll
         for (int q = 0; q < NQ; q++) p0[(size_t)((uint32_t)q * stride)] = x[q];
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Streaming pass: the passes of large aligned columns. A pass is bound by the
+// instructions around its butterflies as much as by the butterflies (7 of
+// 11.2 per butterfly in fft_tile_kernel, which reloads, doubles and negates
+// its twiddles and forms an address per element for every tile), and its
+// warps wait for the tile's loads. So a block fixes the part of the index
+// that selects twiddles and walks the columns (and, in a strided pass, the
+// tiles) that share it:
+//  * the twiddles, already doubled for mul_b2, sit in shared memory, built once
+//    per block: layer section of size s at [s, 2s), so a thread's 2^k
+//    consecutive twiddles are 16-byte shared loads at offsets computed once;
+//  * the next tile arrives by 16-byte cp.async while the current one is in its
+//    last stage: the buffer is free again once that stage has read it. An
+//    evaluation's contiguous pass, which also stores through shared memory
+//    (whole lines per warp; its threads end with 32 consecutive words each),
+//    has a second buffer for the exchanges and that store, and takes the next
+//    tile from the first stage on.
+// 2^TB words per tile, 32 per thread (radix 2^5 stages as above). C > 0: a
+// strided pass, layers [lo, lo + L) on 2^L rows of 2^C contiguous words, TB =
+// L + C. C = 0: layers [0, L) of 2^TB contiguous words (2^(TB - L) transforms).
+// Padding, free of bank conflicts in the accesses it serves: e + 4 (e / 128)
+// for 16-byte copies and strided stages; e + 4 (e / 32) + 8 (e / 256) where
+// threads read and write 32 consecutive words as 16-byte vectors; e + e / 32
+// in the second buffer.
+// Extension of 158 columns, 2^18 coefficients to 2^20 points: 740 us in 9 + 9
+// layers through fft_tile_kernel, 593 us in 8 + 10 here (8.9 against 11.2
+// instructions per butterfly); interpolation 198 -> 167 us. The extension's
+// memory traffic alone, without a butterfly, takes 400 of the 593.
+// ---------------------------------------------------------------------------
+template <bool INV, int C>
+__device__ __host__ constexpr uint32_t in_pad(uint32_t e) {
+  return INV && C == 0 ? e + 4 * (e >> 5) + 8 * (e >> 8) : e + 4 * (e >> 7);
+}
+template <bool INV, int L, int C, int TB>
+struct StreamShape {
+  static constexpr uint32_t THREADS = 1u << (TB - 5);
+  static constexpr bool TWO = !INV && C == 0;  // two buffers
+  static constexpr uint32_t IN_WORDS = in_pad<INV, C>(1u << TB);
+  static constexpr uint32_t X_WORDS = TWO ? (1u << TB) / 8 * 9 : 0;
+  static constexpr uint32_t TW_WORDS = C > 0 ? 1u << L : 1u << (TB - 1);
+  static constexpr size_t SMEM = 4 * (size_t)(IN_WORDS + X_WORDS + TW_WORDS);
+  // resident blocks: shared memory, and 64 registers per thread with one buffer
+  static constexpr int BY_SMEM = (int)((227u << 10) / (SMEM + 1024)), BY_REGS = TWO ? 5 : 1024 / THREADS;
+  static constexpr int PER_SM = BY_SMEM < BY_REGS ? BY_SMEM : BY_REGS;
+};
+
+// 2^set_log twiddle sets; the `units` tiles of a set (columns x the middle
+// index) are walked by `group` blocks. Neighbouring blocks take either the
+// sets of one tile position (sets_first: contiguous passes, and an
+// extension's first pass, whose replicas then read the coefficients from L2)
+// or the tiles of one set (other strided passes: neighbouring rows of memory).
+struct StreamGrid {
+  uint32_t units, group, set_log, sets_first;
+};
+
+template <bool INV, int L, int C, int TB>
+__global__ void __launch_bounds__(1 << (TB - 5), (StreamShape<INV, L, C, TB>::PER_SM))
+    fft_stream_kernel(const uint32_t* const* __restrict__ src_tab, uint32_t* const* __restrict__ dst_tab,
+                      const uint32_t* __restrict__ tw, FftPass a, StreamGrid g) {
+  using Shape = StreamShape<INV, L, C, TB>;
+  constexpr int R = 5, NQ = 32, T = C > 0 ? TB : L;  // T: tile bits of one transform
+  constexpr int K = (L + R - 1) / R;
+  constexpr uint32_t THREADS = Shape::THREADS, CMASK = (1u << C) - 1u;
+  extern __shared__ uint4 stream_sm[];
+  uint32_t* const in = reinterpret_cast<uint32_t*>(stream_sm);
+  uint32_t* const ex = Shape::TWO ? in + Shape::IN_WORDS : in;
+  uint32_t* const tab = in + Shape::IN_WORDS + Shape::X_WORDS;
+  const uint32_t tid = threadIdx.x;
+  // C > 0: the high index; C = 0: the chunk of 2^TB words
+  const uint32_t set = g.sets_first ? blockIdx.x & ((1u << g.set_log) - 1u) : blockIdx.x / g.group;
+  uint32_t unit = g.sets_first ? blockIdx.x >> g.set_log : blockIdx.x - set * g.group;
+
+  // Words of a tile relative to its column; cp.async in 16-byte chunks.
+  const uint32_t mid_bits = C > 0 ? a.lo - C : 0;
+  auto tile_base = [&](uint32_t u) -> uint32_t {
+    return C > 0 ? (set << (a.lo + L)) | ((u & ((1u << mid_bits) - 1u)) << C) : set << TB;
+  };
+  auto issue = [&](uint32_t u, const uint32_t* src) {
+    const uint32_t base = tile_base(u);
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const uint32_t e = 4 * tid + 4 * THREADS * q;
+      const uint32_t v = base | (C > 0 ? ((e >> C) << a.lo) | (e & CMASK) : e);
+      const uint32_t d = (uint32_t)__cvta_generic_to_shared(in + in_pad<INV, C>(4 * tid) + in_pad<INV, C>(4 * THREADS * q));
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + (v & a.src_mask)) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  issue(unit, src_tab[unit >> mid_bits]);
+  // the next tile's column, one tile ahead of its copies
+  const uint32_t* next_src = unit + g.group < g.units ? src_tab[(unit + g.group) >> mid_bits] : nullptr;
+
+  // the block's twiddles, doubled
+  if (C > 0) {
+    for (uint32_t i = tid; i < (1u << L); i += THREADS) {
+      if (i == 0) continue;
+      const uint32_t lg = 31 - __clz(i);  // section of 2^lg twiddles: layer lo + L - 1 - lg
+      tab[i] = __ldg(tw + (a.tw_len - (1u << (a.n - a.lo - (L - 1) + lg))) + (set << lg) + (i - (1u << lg))) << 1;
+    }
+  } else {
+    // layers 1 .. L - 1; the circle layer 0 takes its twiddles from layer 1's
+    for (uint32_t i = tid; i < (1u << (TB - 1)); i += THREADS) {
+      if (i < (1u << (TB - L))) continue;
+      const uint32_t lg = 31 - __clz(i);  // layer TB - 1 - lg
+      tab[i] = __ldg(tw + (a.tw_len - (1u << (a.n - (TB - 1) + lg))) + (set << lg) + (i - (1u << lg))) << 1;
+    }
+  }
+
+  for (; unit < g.units; unit += g.group) {
+    uint32_t* const dst = dst_tab[unit >> mid_bits];
+    // the buffer is free: the next tile may arrive
+    auto refill = [&] {
+      __syncthreads();
+      const uint32_t next = unit + g.group;
+      if (next < g.units) {
+        issue(next, next_src);
+        if (next + g.group < g.units) next_src = src_tab[(next + g.group) >> mid_bits];
+      }
+    };
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();  // the tile has landed (and, the first time, the twiddles)
+    uint32_t x[NQ];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      // stage windows, as in fft_tile_kernel
+      const int s0 = INV ? ((k + 1 < K) ? C + k * R : T - R) : ((k + 1 < K) ? T - (k + 1) * R : C);
+      const int ja = INV ? ((k + 1 < K) ? 0 : C + k * R - s0) : 0;
+      const int jb = INV ? R : ((k + 1 < K) ? R : T - k * R - C);
+      const uint32_t ebase = ((tid >> s0) << (s0 + R)) | (tid & ((1u << s0) - 1u));
+      if (k == 0) {
+        if (INV && C == 0) {
+          const uint4* p = reinterpret_cast<const uint4*>(in + in_pad<INV, C>(ebase));
+#pragma unroll
+          for (int q = 0; q < NQ / 4; q++) {
+            const uint4 v = p[q];
+            x[4 * q] = v.x; x[4 * q + 1] = v.y; x[4 * q + 2] = v.z; x[4 * q + 3] = v.w;
+          }
+        } else {
+          const uint32_t* p = in + in_pad<INV, C>(ebase);  // the padding adds over disjoint bit fields
+#pragma unroll
+          for (int q = 0; q < NQ; q++) x[q] = p[in_pad<INV, C>((uint32_t)q << s0)];
+        }
+        if (Shape::TWO || K == 1) refill();
+      } else {
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < NQ; q++)
+          x[q] = Shape::TWO ? ex[padw(ebase) + padw((uint32_t)q << s0)]
+                            : in[in_pad<INV, C>(ebase) + in_pad<INV, C>((uint32_t)q << s0)];
+        if (!Shape::TWO && k + 1 == K) refill();
+      }
+      // twiddle group of this thread's window: its row index above the window
+      const uint32_t grp = tid >> s0;
+      uint32_t w1[8];  // layer 1's twiddles of this thread, kept for layer 0
+#pragma unroll
+      for (int jj = 0; jj < R; jj++) {
+        const int j = INV ? jj : (R - 1 - jj);
+        if (j < ja || j >= jb) continue;
+        const int layer = s0 + j - C;           // within the pass
+        const int cnt = 1 << (R - 1 - j);       // twiddles per thread
+        uint32_t w[NQ / 2];
+        if (C == 0 && layer == 0) {
+          // s0 = 0: this thread's 16 circle twiddles from its 8 of layer 1
+          if (INV || jb == 1) {  // layer 1 comes after, or was in the stage before
+            const uint4* p = reinterpret_cast<const uint4*>(tab + (1u << (TB - 2)) + 8 * grp);
+            const uint4 u = p[0], v = p[1];
+            w1[0] = u.x; w1[1] = u.y; w1[2] = u.z; w1[3] = u.w;
+            w1[4] = v.x; w1[5] = v.y; w1[6] = v.z; w1[7] = v.w;
+          }
+#pragma unroll
+          for (int q = 0; q < 4; q++) {  // [y, -y, -x, x], doubled: 2 (p - w) = 2p - 2w
+            w[4 * q] = w1[2 * q + 1];
+            w[4 * q + 1] = 2u * P - w1[2 * q + 1];
+            w[4 * q + 2] = 2u * P - w1[2 * q];
+            w[4 * q + 3] = w1[2 * q];
+          }
+        } else if (C == 0 && layer == 1 && INV) {
+#pragma unroll
+          for (int q = 0; q < 8; q++) w[q] = w1[q];
+        } else {
+          // section size: 2^(L - 1 - layer) rows' worth, 2^(TB - 1 - layer) in a contiguous pass
+          const uint32_t sec = 1u << ((C > 0 ? L : TB) - 1 - layer);
+          const uint32_t* p = tab + sec + (grp << (R - 1 - j));
+          if (cnt >= 4) {
+#pragma unroll
+            for (int q = 0; q < cnt / 4; q++) {
+              const uint4 v = reinterpret_cast<const uint4*>(p)[q];
+              w[4 * q] = v.x; w[4 * q + 1] = v.y; w[4 * q + 2] = v.z; w[4 * q + 3] = v.w;
+            }
+          } else if (cnt == 2) {
+            const uint2 v = *reinterpret_cast<const uint2*>(p);
+            w[0] = v.x; w[1] = v.y;
+          } else {
+            w[0] = *p;
+          }
+          if (C == 0 && layer == 1 && s0 == 0)
+#pragma unroll
+            for (int q = 0; q < 8; q++) w1[q] = w[q];
+        }
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+          if (q & (1 << j)) continue;
+          bfly_b2<INV>(x[q], x[q | (1 << j)], w[q >> (j + 1)]);
+        }
+      }
+      if (k + 1 < K) {
+        if (INV && C == 0 && k == 0) {
+          uint4* p = reinterpret_cast<uint4*>(in + in_pad<INV, C>(ebase));
+#pragma unroll
+          for (int q = 0; q < NQ / 4; q++) p[q] = make_uint4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+        } else {
+#pragma unroll
+          for (int q = 0; q < NQ; q++) {
+            if (Shape::TWO) ex[padw(ebase) + padw((uint32_t)q << s0)] = x[q];
+            else in[in_pad<INV, C>(ebase) + in_pad<INV, C>((uint32_t)q << s0)] = x[q];
+          }
+        }
+        continue;
+      }
+      if (INV && a.has_scale) {
+        // 1/2^n = 2^(31 - n mod 31): a rotation of the 31-bit word, canonical as it is
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+          const uint64_t p = (uint64_t)x[q] * (a.scale << 1);
+          x[q] = (uint32_t)(p >> 32) + ((uint32_t)p >> 1);
+        }
+      }
+      if (!INV && C == 0) {
+        __syncthreads();  // every thread has read its exchange words
+        uint4* o = reinterpret_cast<uint4*>(ex + 36 * tid);  // s0 = 0: row tid of 32 words, 4 of padding
+#pragma unroll
+        for (int q = 0; q < NQ / 4; q++) o[q] = make_uint4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+        __syncthreads();
+        uint4* d = reinterpret_cast<uint4*>(dst + (set << TB));
+#pragma unroll
+        for (int q = 0; q < NQ / 4; q++) {
+          const uint32_t e = 4 * tid + 4 * THREADS * q;
+          d[tid + THREADS * q] = *reinterpret_cast<const uint4*>(ex + e + 4 * (e >> 5));
+        }
+      } else {
+        const uint32_t v = tile_base(unit) | (C > 0 ? ((ebase >> C) << a.lo) | (ebase & CMASK) : ebase);
+        uint32_t* p0 = dst + v;
+        const uint32_t stride = C > 0 ? 1u << (s0 - C + a.lo) : 1u << s0;
+#pragma unroll
+        for (int q = 0; q < NQ; q++) p0[(size_t)q * stride] = x[q];
       }
     }
   }
@@ -435,15 +682,48 @@ static int launch_small(cudaStream_t st, const uint32_t* const* src, uint32_t* c
 }
 
 struct FftTuning {
-  uint32_t tile_log = 13;      // log2 of the shared-memory tile (elements), <= 13
-  uint32_t coalesce_bits = 4;  // contiguous low bits per strided tile row
+  uint32_t tile_log;       // log2 of the shared-memory tile (elements), <= 13
+  uint32_t coalesce_bits;  // contiguous low bits per strided tile row
 };
 // Per number of computed layers (an FFT of 2^n, or an LDE from 2^n
 // coefficients, computes n layers) and extension (domain log size minus
 // layers: 0 for an FFT, the blowup for an LDE; capped at FFT_MAX_EXT). Written
 // at set-up (set_fft_tuning, fft_autotune), read by every launch.
 constexpr uint32_t FFT_MAX_EXT = 3;
-static FftTuning g_fft_tuning[32][FFT_MAX_EXT + 1];
+static void split_layers(uint32_t layers, FftTuning tn, std::vector<std::pair<uint32_t, uint32_t>>& parts);
+
+// The default split of each size: fewest passes, then fewest register stages
+// (of up to 5 layers), then the wider rows of 12/5 (whole 128-byte lines).
+// 13/4, whose strided passes hold 9 layers in tiles of 2^13, only where it
+// saves a pass: 9 + 9 layers measured 345 + 193 us (extension by 2 and
+// interpolation of 158 columns of 2^18: 638 + 194), 10 + 8 (12/4) 328 + 177
+// (600 + 176); 2^19, 12 + 7 (12/5) 280 + 155 against 290 + 162 for 10 + 9;
+// 2^22, 13 + 9 345 + 178 against three passes' 387 + 256.
+static FftTuning default_tuning(uint32_t layers) {
+  FftTuning best{13, 4};
+  size_t best_passes = 99, best_stages = 0;
+  for (FftTuning tn : {FftTuning{12, 5}, FftTuning{12, 4}, FftTuning{13, 4}}) {
+    std::vector<std::pair<uint32_t, uint32_t>> parts;
+    split_layers(layers, tn, parts);
+    size_t stages = 0;
+    for (auto& p : parts) stages += (p.second + 4) / 5;
+    if (parts.size() < best_passes || (parts.size() == best_passes && tn.tile_log == 12 && stages < best_stages)) {
+      best = tn;
+      best_passes = parts.size();
+      best_stages = stages;
+    }
+  }
+  return best;
+}
+struct FftTunings {
+  FftTuning at[32][FFT_MAX_EXT + 1];
+  FftTunings() {
+    for (uint32_t l = 0; l < 32; l++)
+      for (uint32_t e = 0; e <= FFT_MAX_EXT; e++) at[l][e] = default_tuning(l);
+  }
+  FftTuning* operator[](uint32_t l) { return at[l]; }
+};
+static FftTunings g_fft_tuning;
 static uint32_t ext_slot(uint32_t layers, uint32_t n) {
   return n - layers < FFT_MAX_EXT ? n - layers : FFT_MAX_EXT;
 }
@@ -453,8 +733,7 @@ static FftTuning tuning_for(uint32_t layers, uint32_t n) {
 
 // Splits layers [0, layers) into balanced passes (lo, L): the first pass has
 // the whole tile for layers, later ones reserve `coalesce_bits` of it.
-static void fft_partition(uint32_t layers, uint32_t n, std::vector<std::pair<uint32_t, uint32_t>>& parts) {
-  const FftTuning tn = tuning_for(layers, n);
+static void split_layers(uint32_t layers, FftTuning tn, std::vector<std::pair<uint32_t, uint32_t>>& parts) {
   const uint32_t T = tn.tile_log, C = tn.coalesce_bits;
   if (layers <= T) {
     parts.push_back({0, layers});
@@ -471,6 +750,10 @@ static void fft_partition(uint32_t layers, uint32_t n, std::vector<std::pair<uin
   }
 }
 
+static void fft_partition(uint32_t layers, uint32_t n, std::vector<std::pair<uint32_t, uint32_t>>& parts) {
+  split_layers(layers, tuning_for(layers, n), parts);
+}
+
 template <bool INV, int R>
 static void launch_pass(cudaStream_t st, dim3 grid, uint32_t threads, size_t smem, const uint32_t* const* s,
                         uint32_t* const* d, const uint32_t* tw, const FftPass& a) {
@@ -483,22 +766,83 @@ static void launch_tile(cudaStream_t st, dim3 grid, uint32_t threads, const uint
                         const uint32_t* tw, const FftPass& a) {
   const uint32_t words = 1u << (a.t + a.tile_shift);
   const size_t smem = (size_t)4 * (words + (words >> 5));
-  fft_tile_kernel<INV, L, C><<<grid, threads, smem, st>>>(s, d, tw, a, 1u, 0xffffffffu);
+  fft_tile_kernel<INV, L, C><<<grid, threads, smem, st>>>(s, d, tw, a);
   note_launch();
 }
 
-// The specialised kernel covers first passes (C = 0, 5..13 layers) and later
-// passes with 16 or 32 contiguous words per tile row (C = 4 with 5..9 layers,
-// C = 5 with 5..8); anything else runs the generic pass. GS_FFT_GENERIC=1 forces the generic
-// pass (for comparisons).
-template <bool INV>
-static bool launch_tile_any(cudaStream_t st, dim3 grid, uint32_t threads, const uint32_t* const* s,
-                            uint32_t* const* d, const uint32_t* tw, const FftPass& a) {
+// GS_FFT_GENERIC=1 forces the generic pass (for comparisons).
+static bool fft_generic() {
   static const bool generic = [] {
     const char* e = getenv("GS_FFT_GENERIC");
     return e && e[0] == '1';
   }();
-  if (generic) return false;
+  return generic;
+}
+
+// Tiles per block: the chip's share of all tiles in whole waves of equal
+// blocks, each of 8 tiles or a few more (one wave below 16; 4 tiles against 5
+// in a wave and a bit took 35 us against 26 on 100 columns of 2^17), at most
+// a set's.
+static uint32_t stream_tiles(uint32_t set_log, uint32_t units, uint32_t per_sm) {
+  const uint64_t resident = (uint64_t)num_sms() * per_sm, total = (uint64_t)units << set_log;
+  const uint64_t waves = std::max<uint64_t>(1, total / (8 * resident));
+  return (uint32_t)std::min<uint64_t>(units, (total + waves * resident - 1) / (waves * resident));
+}
+
+template <bool INV, int L, int C, int TB>
+static int launch_stream(cudaStream_t st, uint32_t n_cols, const uint32_t* const* s, uint32_t* const* d,
+                         const uint32_t* tw, const FftPass& a) {
+  using Shape = StreamShape<INV, L, C, TB>;
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      fft_stream_kernel<INV, L, C, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape::SMEM);
+  GS_CUDA_TRY(attr);
+  StreamGrid g;
+  g.set_log = C > 0 ? a.n - a.lo - L : a.n - TB;
+  g.units = C > 0 ? n_cols << (a.lo - C) : n_cols;
+  g.sets_first = C == 0 || a.src_mask != 0xffffffffu;
+  const uint32_t per = stream_tiles(g.set_log, g.units, Shape::PER_SM);
+  g.group = (g.units + per - 1) / per;
+  fft_stream_kernel<INV, L, C, TB><<<g.group << g.set_log, Shape::THREADS, Shape::SMEM, st>>>(s, d, tw, a, g);
+  note_launch();
+  GS_CUDA_TRY(cudaGetLastError());
+  return OK;
+}
+
+// Passes the streaming kernel takes: aligned columns of at least one tile,
+// contiguous passes of 5..13 layers, strided ones of 5..9 whose rows of
+// 2^(TB - L) words start a layer range high enough. *taken says whether it ran.
+// A contiguous pass builds a table of half a tile's words per block, which
+// takes 4 tiles to pay (one column of 2^24, a tile per block: 46 -> 77 us).
+constexpr uint32_t STREAM_MIN_TILES = 4;
+template <bool INV>
+static int launch_stream_any(cudaStream_t st, uint32_t n_cols, const uint32_t* const* s, uint32_t* const* d,
+                             const uint32_t* tw, const FftPass& a, bool* taken) {
+  *taken = false;
+  if (fft_generic() || !a.vec_ok || (uint64_t)n_cols << a.n >= 1ull << 40) return OK;
+#define GS_STREAM(LL, CC, TB)                                                   \
+  case LL:                                                                      \
+    if (a.n < TB || (CC > 0 && a.lo < CC)) return OK;                           \
+    if (CC == 0 && stream_tiles(a.n - TB, n_cols, StreamShape<INV, LL, CC, TB>::PER_SM) < STREAM_MIN_TILES) \
+      return OK;                                                                \
+    *taken = true;                                                              \
+    return launch_stream<INV, LL, CC, TB>(st, n_cols, s, d, tw, a);
+  if (a.lo == 0) {
+    switch (a.L) { GS_STREAM(5, 0, 12) GS_STREAM(6, 0, 12) GS_STREAM(7, 0, 12) GS_STREAM(8, 0, 12) GS_STREAM(9, 0, 12)
+                   GS_STREAM(10, 0, 12) GS_STREAM(11, 0, 12) GS_STREAM(12, 0, 12) GS_STREAM(13, 0, 13)
+                   default: return OK; }
+  }
+  switch (a.L) { GS_STREAM(5, 7, 12) GS_STREAM(6, 6, 12) GS_STREAM(7, 5, 12) GS_STREAM(8, 4, 12) GS_STREAM(9, 4, 13)
+                 default: return OK; }
+#undef GS_STREAM
+}
+
+// The specialised kernel covers first passes (C = 0, 5..13 layers) and later
+// passes with 16 or 32 contiguous words per tile row (C = 4 with 5..9 layers,
+// C = 5 with 5..8); anything else runs the generic pass.
+template <bool INV>
+static bool launch_tile_any(cudaStream_t st, dim3 grid, uint32_t threads, const uint32_t* const* s,
+                            uint32_t* const* d, const uint32_t* tw, const FftPass& a) {
+  if (fft_generic()) return false;
 #define GS_TILE(LL, CC) \
   case LL: launch_tile<INV, LL, CC>(st, grid, threads, s, d, tw, a); return true;
   if (a.c == 0) {
@@ -549,6 +893,9 @@ static int run_passes(cudaStream_t st, const uint32_t* const* src, uint32_t* con
     const size_t smem = (size_t)4 << (a.t + tile_shift);
     dim3 grid(1u << (tiles_log - tile_shift), n_cols);
     const uint32_t* const* s = (p == 0) ? src : (const uint32_t* const*)dst;
+    bool taken = false;
+    GS_TRY(launch_stream_any<INV>(st, n_cols, s, dst, tw, a, &taken));
+    if (taken) continue;
     if (R == 5 && launch_tile_any<INV>(st, grid, threads, s, dst, tw, a)) {
       GS_CUDA_TRY(cudaGetLastError());
       continue;

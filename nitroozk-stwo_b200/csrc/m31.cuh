@@ -24,13 +24,17 @@ constexpr uint32_t P = 0x7fffffffu;
 
 GS_HD uint32_t umin32(uint32_t a, uint32_t b) { return a < b ? a : b; }
 
-// a + b for a, b < p: with s = a + b - p (mod 2^32), the result is
-// min(s + p, s) (s wraps above s + p exactly when a + b < p). On the device
-// that is one three-input add and one add-then-min (VIADDMNMX).
+// a + b for a, b < p: with s = a + b, the result is min(s, s - p) mod 2^32 (s -
+// p wraps above s exactly when s < p). On the device that is one two-input
+// add, which issues in one cycle beside the integer ALU pipe (a three-input
+// add takes two on that pipe, an IMAD two on the FMA pipe: measured), and one
+// add-then-min (VIADDMNMX). Against the three-input form: Poseidon2
+// constraints 354 -> 348 us per 2^20 rows; against IMAD forms of the adds:
+// the Poseidon2 trace's extension 743 -> 722 us.
 GS_HD uint32_t add(uint32_t a, uint32_t b) {
 #ifdef __CUDA_ARCH__
-  uint32_t s = a + b - P;
-  return __viaddmin_u32(s, P, s);
+  uint32_t s = a + b;
+  return __viaddmin_u32(s, 0u - P, s);
 #else
   uint32_t r = a + b;
   return umin32(r, r - P);
@@ -60,29 +64,6 @@ __device__ __forceinline__ uint32_t mul_b2(uint32_t a, uint32_t b2) {
   uint64_t p = (uint64_t)a * b2;
   uint32_t r = (uint32_t)(p >> 32) + ((uint32_t)p >> 1);
   return __viaddmin_u32(r, 0u - P, r);
-}
-// FMA-pipe forms. The integer ALU pipe bounds the FFT, Blake2s and
-// constraint kernels while the FMA pipe idles; an add issued as an IMAD
-// against a runtime 1 (or -1), which the compiler cannot fold, runs there
-// instead, leaving one add-then-min per field add/sub on the ALU pipe.
-__device__ __forceinline__ uint32_t imad_u32(uint32_t a, uint32_t b, uint32_t c) {
-  uint32_t r;
-  asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
-  return r;
-}
-// a + b (one = 1 at run time)
-__device__ __forceinline__ uint32_t add_f(uint32_t a, uint32_t b, uint32_t one) {
-  uint32_t s = imad_u32(a, one, b);
-  return __viaddmin_u32(s, 0u - P, s);
-}
-// a - b (neg1 = 2^32 - 1 at run time)
-__device__ __forceinline__ uint32_t sub_f(uint32_t a, uint32_t b, uint32_t neg1) {
-  uint32_t d = imad_u32(b, neg1, a);
-  return __viaddmin_u32(d, P, d);
-}
-// a * b with the doubling of b on the FMA pipe
-__device__ __forceinline__ uint32_t mul_f(uint32_t a, uint32_t b, uint32_t one) {
-  return mul_b2(a, imad_u32(b, one, b));
 }
 GS_HD uint32_t mul(uint32_t a, uint32_t b) {
 #ifdef __CUDA_ARCH__

@@ -75,6 +75,43 @@ def qm31(v):
     return L.QM31(*v)
 
 
+def qm31_array(values, n=None):
+    """QM31 values (4 ints each) as a host array of n gs_qm31, zeros after the
+    last: (address, array to keep alive)."""
+    values = list(values)
+    n = len(values) if n is None else n
+    if len(values) > max(n, 1):
+        raise ValueError(f"{len(values)} values for {n} places")
+    out = np.zeros((max(n, 1), 4), np.uint32)
+    if values:
+        try:  # one conversion for the whole list; words wrap mod 2^32, as in a ctypes field
+            a = np.array(values, dtype=np.int64)
+        except (OverflowError, TypeError, ValueError):
+            a = None
+        if a is not None and a.shape == (len(values), 4):
+            out[:len(values)] = a.astype(np.uint32)
+        else:
+            arr = (L.QM31 * len(values))(*[qm31(v) for v in values])
+            out[:len(values)] = np.frombuffer(arr, np.uint32).reshape(-1, 4)
+    return out.ctypes.data, out
+
+
+# gs_fft_item and gs_merkle_item (include/gpustark.h)
+_FFT_ITEM = np.dtype([("src", "u8"), ("dst", "u8"), ("log_size", "u4"), ("coeffs_log_size", "u4"), ("inverse", "u4"),
+                      ("reserved", "u4")])
+_MERKLE_ITEM = np.dtype([("cols", "u8"), ("n_cols", "u4"), ("log_size", "u4"), ("layers", "u8")])
+# A small tree's layers are one allocation; a larger tree's are separate, so
+# that a caller who keeps only its root keeps only the root's memory.
+_ONE_BUFFER_TREE_LOG = 10
+
+
+def _tree_layers(log):
+    if log > _ONE_BUFFER_TREE_LOG:
+        return [torch.empty(8 << lg, dtype=torch.int32, device="cuda") for lg in range(log + 1)]
+    sizes = [8 << lg for lg in range(log + 1)]
+    return list(torch.empty(sum(sizes), dtype=torch.int32, device="cuda").split(sizes))
+
+
 @dataclass
 class TwiddleTree:
     """PolyOps::Twiddles for the coset half_odds(root_log) (prover/poly/twiddles.rs:9-14)."""
@@ -140,15 +177,17 @@ class GpuBackend:
         (src is dst: in place) or ("evaluate", coeffs, dst) with dst of
         2^log words; returns the dst tensors."""
         ctx = ctx or default_context()
-        arr = (L.FftItem * max(len(items), 1))()
-        for k, (kind, src, dst) in enumerate(items):
+        for kind, _, _ in items:
             if kind not in ("interpolate", "evaluate"):
                 raise ValueError(f"unknown work-list item kind {kind!r}")
-            arr[k].src, arr[k].dst = src.data_ptr(), dst.data_ptr()
-            arr[k].log_size = dst.numel().bit_length() - 1
-            arr[k].coeffs_log_size = src.numel().bit_length() - 1
-            arr[k].inverse = 1 if kind == "interpolate" else 0
-        L.check(L.lib().gs_fft_worklist(ctx.handle, arr, len(items), _p(twiddles.twiddles), _p(twiddles.itwiddles),
+        arr = np.zeros(max(len(items), 1), _FFT_ITEM)
+        if items:
+            arr["src"] = [src.data_ptr() for _, src, _ in items]
+            arr["dst"] = [dst.data_ptr() for _, _, dst in items]
+            arr["log_size"] = [dst.numel().bit_length() - 1 for _, _, dst in items]
+            arr["coeffs_log_size"] = [src.numel().bit_length() - 1 for _, src, _ in items]
+            arr["inverse"] = [kind == "interpolate" for kind, _, _ in items]
+        L.check(L.lib().gs_fft_worklist(ctx.handle, arr.ctypes.data, len(items), _p(twiddles.twiddles), _p(twiddles.itwiddles),
                                         twiddles.root_log), "fft_worklist")
         return [dst for _, _, dst in items]
 
@@ -218,17 +257,21 @@ class GpuBackend:
         trees: lists of columns (tensors of 2^log words each, at least one per
         tree); returns per tree its layers, layers[L] of 2^L x 8 words."""
         ctx = ctx or default_context()
-        arr = (L.MerkleItem * max(len(trees), 1))()
-        keep, out = [], []
-        for k, cols in enumerate(trees):
-            log = cols[0].numel().bit_length() - 1
-            layers = [torch.empty((1 << lg) * 8, dtype=torch.int32, device="cuda") for lg in range(log + 1)]
-            cp, kc = L.ptr_array([c.data_ptr() for c in cols])
-            lp, kl = L.ptr_array([t.data_ptr() for t in layers])
-            keep += [kc, kl]
-            arr[k].cols, arr[k].n_cols, arr[k].log_size, arr[k].layers = cp, len(cols), log, lp
-            out.append(layers)
-        L.check(L.lib().gs_merkle_worklist(ctx.handle, arr, len(trees)), "merkle_worklist")
+        logs = [cols[0].numel().bit_length() - 1 for cols in trees]
+        out = [_tree_layers(log) for log in logs]
+        ptrs, at = [], []  # every tree's column and layer pointers in one array; where they start
+        for cols, layers in zip(trees, out):
+            at.append((len(ptrs), len(ptrs) + len(cols)))
+            ptrs += [c.data_ptr() for c in cols]
+            ptrs += [t.data_ptr() for t in layers]
+        base, keep = L.ptr_array(ptrs)
+        arr = np.zeros(max(len(trees), 1), _MERKLE_ITEM)
+        if trees:
+            arr["cols"] = [base + 8 * c for c, _ in at]
+            arr["n_cols"] = [len(cols) for cols in trees]
+            arr["log_size"] = logs
+            arr["layers"] = [base + 8 * l for _, l in at]
+        L.check(L.lib().gs_merkle_worklist(ctx.handle, arr.ctypes.data, len(trees)), "merkle_worklist")
         return out
 
     @staticmethod
@@ -297,11 +340,12 @@ class GpuBackend:
         out = [torch.empty(1 << log_size, dtype=torch.int32, device="cuda") for _ in range(4)]
         cp, k1 = L.ptr_array([c.data_ptr() for c in columns])
         n = len(column_indices)
-        idx = (C.c_uint32 * max(n, 1))(*[int(i) for i in column_indices])
-        bs = (L.QM31 * max(n, 1))(*[qm31(b) for b in line_coeffs_b])
-        cs = (L.QM31 * max(n, 1))(*[qm31(c) for c in line_coeffs_c])
+        idx = np.array([int(i) for i in column_indices] or [0], dtype=np.int64).astype(np.uint32)
+        bs, kb = qm31_array(line_coeffs_b, n)
+        cs, kc = qm31_array(line_coeffs_c, n)
         op, k2 = L.ptr_array([t.data_ptr() for t in out])
-        L.check(L.lib().gs_accumulate_numerators(ctx.handle, log_size, cp, len(columns), idx, bs, cs, n, op),
+        L.check(L.lib().gs_accumulate_numerators(ctx.handle, log_size, cp, len(columns),
+                                                 idx.ctypes.data_as(L.U32P), bs, cs, n, op),
                 "accumulate_numerators")
         return out
 
@@ -354,7 +398,7 @@ class GpuBackend:
         out = (L.QM31 * len(polys))()
         pt = L.PointQM31(qm31(point[:4]), qm31(point[4:]))
         L.check(L.lib().gs_batch_eval_at_point(ctx.handle, pp, len(polys), log_size, pt, out), "batch_eval_at_point")
-        return [[o.a, o.b, o.c, o.d] for o in out]
+        return np.frombuffer(out, np.uint32).reshape(-1, 4).tolist()
 
     @staticmethod
     def batch_eval_at_point_noalloc(polys, point, log_size=None, stream=None):
@@ -448,7 +492,7 @@ class GpuBackend:
         t0, k1 = L.ptr_array([t.data_ptr() for t in trace0])
         t1, k2 = L.ptr_array([t.data_ptr() for t in trace1])
         t2, k3 = L.ptr_array([t.data_ptr() for t in trace2])
-        pw = (L.QM31 * max(len(random_coeff_powers), 1))(*[qm31(p) for p in random_coeff_powers])
+        pw, kp = qm31_array(random_coeff_powers)
         dn = np.ascontiguousarray(denominator_inverses, dtype=np.uint32)
         eb = (C.c_uint8 * len(eval_bytes)).from_buffer_copy(eval_bytes)
         L.check(L.lib().gs_evaluate_constraint_quotients_on_domain(

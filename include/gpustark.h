@@ -131,7 +131,8 @@ int gs_fft_worklist(gs_ctx* ctx, const gs_fft_item* items, uint32_t n_items, con
  * set-up calls: no other FFT may be in flight. gs_fft_set_tuning installs one
  * split (log_size 0: every size; extension > 3: every extension; tile_log in
  * [6, 13], coalesce_bits <= min(5, tile_log - 5)); gs_fft_get_tuning reads
- * it. Default: by size (12 / 5, 12 / 4 or 13 / 4). */
+ * it. The default, 13 / 4, takes the split measured best for the size within
+ * tiles of 2^13 (12 / 5, 12 / 4 or 13 / 4). */
 int gs_fft_autotune(gs_ctx* ctx, uint32_t min_log, uint32_t max_log, uint32_t max_extension, uint32_t* tile_logs,
                     uint32_t* coalesce_bits);
 int gs_fft_set_tuning(uint32_t log_size, uint32_t extension, uint32_t tile_log, uint32_t coalesce_bits);

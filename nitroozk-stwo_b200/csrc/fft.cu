@@ -692,7 +692,8 @@ struct FftTuning {
 constexpr uint32_t FFT_MAX_EXT = 3;
 static void split_layers(uint32_t layers, FftTuning tn, std::vector<std::pair<uint32_t, uint32_t>>& parts);
 
-// The default split of each size: fewest passes, then fewest register stages
+// What the default, 13/4, stands for: within tiles of 2^13, the split measured
+// best for each size. Fewest passes, then fewest register stages
 // (of up to 5 layers), then the wider rows of 12/5 (whole 128-byte lines).
 // 13/4, whose strided passes hold 9 layers in tiles of 2^13, only where it
 // saves a pass: 9 + 9 layers measured 345 + 193 us (extension by 2 and
@@ -716,10 +717,13 @@ static FftTuning default_tuning(uint32_t layers) {
   return best;
 }
 struct FftTunings {
-  FftTuning at[32][FFT_MAX_EXT + 1];
+  FftTuning by_size[32];
+  FftTuning at[32][FFT_MAX_EXT + 1];  // as installed
   FftTunings() {
-    for (uint32_t l = 0; l < 32; l++)
-      for (uint32_t e = 0; e <= FFT_MAX_EXT; e++) at[l][e] = default_tuning(l);
+    for (uint32_t l = 0; l < 32; l++) {
+      by_size[l] = default_tuning(l);
+      for (uint32_t e = 0; e <= FFT_MAX_EXT; e++) at[l][e] = {13, 4};
+    }
   }
   FftTuning* operator[](uint32_t l) { return at[l]; }
 };
@@ -728,7 +732,9 @@ static uint32_t ext_slot(uint32_t layers, uint32_t n) {
   return n - layers < FFT_MAX_EXT ? n - layers : FFT_MAX_EXT;
 }
 static FftTuning tuning_for(uint32_t layers, uint32_t n) {
-  return g_fft_tuning[layers < 32 ? layers : 31][ext_slot(layers, n)];
+  const uint32_t l = layers < 32 ? layers : 31;
+  const FftTuning t = g_fft_tuning[l][ext_slot(layers, n)];
+  return t.tile_log == 13 && t.coalesce_bits == 4 ? g_fft_tuning.by_size[l] : t;
 }
 
 // Splits layers [0, layers) into balanced passes (lo, L): the first pass has
@@ -1156,7 +1162,8 @@ int fft_autotune(cudaStream_t st, uint32_t lo, uint32_t hi, uint32_t max_ext, co
         g_fft_tuning[n][e] = c;
         std::vector<std::pair<uint32_t, uint32_t>> parts;
         fft_partition(n, dn, parts);
-        for (auto& pr : parts) pr.first = std::min(c.coalesce_bits, pr.first) | (pr.first << 8);
+        const uint32_t cb = tuning_for(n, dn).coalesce_bits;
+        for (auto& pr : parts) pr.first = std::min(cb, pr.first) | (pr.first << 8);
         if (std::find(seen.begin(), seen.end(), parts) != seen.end()) continue;
         seen.push_back(parts);
         float ms = 1e30f;

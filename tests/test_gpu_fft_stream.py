@@ -32,7 +32,7 @@ SHAPES = [(12, 0, 3333, 13, 4), (13, 0, 1601, 13, 4), (13, 1, 801, 13, 4), (12, 
           (10, 2, 3001, 13, 4), (9, 3, 3003, 13, 4), (8, 4, 3001, 13, 4), (7, 5, 3001, 13, 4), (6, 6, 3001, 13, 4),
           (5, 7, 3001, 13, 4), (14, 0, 777, 12, 4), (16, 1, 95, 13, 4), (18, 0, 49, 13, 4), (18, 2, 13, 13, 4),
           (18, 1, 25, 12, 4), (18, 0, 47, 12, 5), (18, 1, 25, 11, 5), (18, 0, 47, 10, 5), (20, 1, 7, 13, 4),
-          (20, 0, 1, 12, 4), (23, 0, 3, 13, 4), (24, 0, 1, 12, 5)]
+          (20, 0, 1, 12, 4), (21, 0, 5, 13, 4), (22, 1, 3, 13, 4), (23, 0, 3, 13, 4), (24, 0, 1, 12, 5)]
 
 
 @pytest.mark.parametrize("log,ext,n_cols,tile,coalesce", SHAPES)

@@ -139,9 +139,9 @@ int gs_interpolate_columns(gs_ctx* ctx, uint32_t* const* cols, uint32_t n_cols, 
   bool aligned = true;
   for (uint32_t i = 0; i < n_cols; i++) aligned = aligned && (((uintptr_t)cols[i] & 15) == 0);
   fft_set_columns_aligned(aligned);
-  const void* const* d = nullptr;
-  GS_TRY(ctx->c.stage_ptrs((const void* const*)cols, n_cols, &d));
-  return interpolate_columns(ctx->c.stream, (uint32_t* const*)d, n_cols, log_size, itwiddles, twiddles_log_size);
+  MutCols c;
+  GS_TRY(ctx->c.columns(cols, n_cols, &c));
+  return interpolate_columns(ctx->c.stream, c, n_cols, log_size, itwiddles, twiddles_log_size);
 }
 
 int gs_fft_worklist(gs_ctx* ctx, const gs_fft_item* items, uint32_t n_items, const uint32_t* twiddles,
@@ -175,12 +175,11 @@ int gs_evaluate_columns(gs_ctx* ctx, const uint32_t* const* coeffs, uint32_t coe
   for (uint32_t i = 0; i < n_cols; i++)
     aligned = aligned && (((uintptr_t)coeffs[i] & 15) == 0) && (((uintptr_t)evals[i] & 15) == 0);
   fft_set_columns_aligned(aligned);
-  const void* const* ds = nullptr;
-  const void* const* dd = nullptr;
-  GS_TRY(ctx->c.stage_ptrs((const void* const*)coeffs, n_cols, &ds));
-  GS_TRY(ctx->c.stage_ptrs((const void* const*)evals, n_cols, &dd));
-  return evaluate_columns(ctx->c.stream, (const uint32_t* const*)ds, coeffs_log_size, (uint32_t* const*)dd, n_cols,
-                          log_size, twiddles, twiddles_log_size);
+  Cols src;
+  MutCols dst;
+  GS_TRY(ctx->c.columns(coeffs, n_cols, &src));
+  GS_TRY(ctx->c.columns(evals, n_cols, &dst));
+  return evaluate_columns(ctx->c.stream, src, coeffs_log_size, dst, n_cols, log_size, twiddles, twiddles_log_size);
 }
 
 int gs_fft_autotune(gs_ctx* ctx, uint32_t min_log, uint32_t max_log, uint32_t max_extension, uint32_t* tile_logs,
@@ -209,7 +208,7 @@ int gs_fft_get_tuning(uint32_t log_size, uint32_t extension, uint32_t* tile_log,
 int gs_commit_on_layer(gs_ctx* ctx, uint32_t log_size, const uint32_t* prev_layer, uint32_t n_cols,
                        const uint32_t* const* cols, uint32_t* out) {
   CTX_REQUIRED(ctx);
-  const void* const* d = nullptr;
+  Cols c;
   bool aligned = true;
   if (n_cols) {
     GS_REQUIRE(cols != nullptr, "null column list");
@@ -217,9 +216,9 @@ int gs_commit_on_layer(gs_ctx* ctx, uint32_t log_size, const uint32_t* prev_laye
       GS_REQUIRE(cols[i] != nullptr, "null column");
       aligned = aligned && ((uintptr_t)cols[i] & 15) == 0;
     }
-    GS_TRY(ctx->c.stage_ptrs((const void* const*)cols, n_cols, &d));
+    GS_TRY(ctx->c.columns(cols, n_cols, &c));
   }
-  return commit_on_layer(ctx->c.stream, log_size, prev_layer, (const uint32_t* const*)d, n_cols, out, aligned);
+  return commit_on_layer(ctx->c.stream, log_size, prev_layer, c, n_cols, out, aligned);
 }
 
 int gs_merkle_worklist(gs_ctx* ctx, const gs_merkle_item* items, uint32_t n_items) {
@@ -242,13 +241,13 @@ int gs_commit_node_layers(gs_ctx* ctx, uint32_t top_log, uint32_t* const* layers
 int gs_poseidon252_commit_on_layer(gs_ctx* ctx, uint32_t log_size, const uint8_t* prev_layer, uint32_t n_cols,
                                    const uint32_t* const* cols, uint8_t* out) {
   CTX_REQUIRED(ctx);
-  const void* const* d = nullptr;
+  Cols c;
   if (n_cols) {
     GS_REQUIRE(cols != nullptr, "null column list");
     for (uint32_t i = 0; i < n_cols; i++) GS_REQUIRE(cols[i] != nullptr, "null column");
-    GS_TRY(ctx->c.stage_ptrs((const void* const*)cols, n_cols, &d));
+    GS_TRY(ctx->c.columns(cols, n_cols, &c));
   }
-  return poseidon252_commit_on_layer(ctx->c.stream, log_size, prev_layer, (const uint32_t* const*)d, n_cols, out);
+  return poseidon252_commit_on_layer(ctx->c.stream, log_size, prev_layer, c, n_cols, out);
 }
 
 int gs_poseidon252_grind(gs_ctx* ctx, const uint8_t digest[32], uint32_t pow_bits, uint64_t* nonce) {
@@ -399,13 +398,13 @@ int gs_batch_eval_at_point(gs_ctx* ctx, const uint32_t* const* polys, uint32_t n
   size_t need = eval_at_point_scratch_bytes(n_polys, log_size) + 16 * (size_t)n_polys;
   void* scratch = nullptr;
   GS_TRY(ctx->c.get_scratch(need, &scratch));
-  const void* const* d = nullptr;
-  GS_TRY(ctx->c.stage_ptrs((const void* const*)polys, n_polys, &d));
+  Cols c;
+  GS_TRY(ctx->c.columns(polys, n_polys, &c));
   uint32_t* d_out = (uint32_t*)((uint8_t*)scratch + eval_at_point_scratch_bytes(n_polys, log_size));
   ptq p = {to_qm(point.x), to_qm(point.y)};
   bool vec = true;
   for (uint32_t i = 0; i < n_polys; i++) vec = vec && ((uintptr_t)polys[i] & 15) == 0;
-  GS_TRY(batch_eval_at_point(ctx->c.stream, (const uint32_t* const*)d, n_polys, log_size, p, d_out, (uint32_t*)scratch,
+  GS_TRY(batch_eval_at_point(ctx->c.stream, c, n_polys, log_size, p, d_out, (uint32_t*)scratch,
                              12, vec));
   GS_CUDA_TRY(cudaMemcpyAsync(out, d_out, 16 * (size_t)n_polys, cudaMemcpyDeviceToHost, ctx->c.stream));
   GS_CUDA_TRY(cudaStreamSynchronize(ctx->c.stream));

@@ -31,7 +31,7 @@ __global__ void eap_weights_kernel(Factors fs, uint32_t s, uint32_t* w /* [j][4]
 // coefficients of one poly, 2^(s-8) per thread: products of M31 by the QM31
 // weights accumulate in 64 bits, folded every third term (a folded value is
 // below 2^34, a product below 2^62).
-__global__ void __launch_bounds__(256) eap_chunk_kernel(const uint32_t* const* __restrict__ polys, uint32_t log_n,
+__global__ void __launch_bounds__(256) eap_chunk_kernel(Cols polys, uint32_t log_n,
                                                         uint32_t s, const uint32_t* __restrict__ w, Factors fs,
                                                         uint32_t* partials, bool vec) {
   __shared__ uint32_t red[4][256 / 32];
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(256) eap_chunk_kernel(const uint32_t* const* _
 // coefficient: three products of < 2^62 on a folded value < 2^34 fit 64 bits).
 constexpr uint32_t EAP_MULTI_LOG = 12;
 template <int K>
-__global__ void __launch_bounds__(256) eap_chunk_multi_kernel(const uint32_t* const* __restrict__ polys,
+__global__ void __launch_bounds__(256) eap_chunk_multi_kernel(Cols polys,
                                                               uint32_t n_polys, uint32_t log_n,
                                                               const uint32_t* __restrict__ w, Factors fs,
                                                               uint32_t* partials) {
@@ -223,7 +223,7 @@ size_t eval_at_point_scratch_bytes(uint32_t n_polys, uint32_t log_n, uint32_t ch
 
 // out: 4 words per polynomial (device). scratch: eval_at_point_scratch_bytes()
 // for the same chunk_log (coefficients per block, log 2).
-int batch_eval_at_point(cudaStream_t st, const uint32_t* const* d_polys, uint32_t n_polys, uint32_t log_n, ptq point,
+int batch_eval_at_point(cudaStream_t st, Cols polys, uint32_t n_polys, uint32_t log_n, ptq point,
                         uint32_t* d_out, uint32_t* d_scratch, uint32_t chunk_log, bool vec) {
   GS_REQUIRE(log_n <= 30, "log size out of range");
   GS_REQUIRE(chunk_log >= 8 && chunk_log <= 14, "chunk log size out of range");
@@ -233,7 +233,8 @@ int batch_eval_at_point(cudaStream_t st, const uint32_t* const* d_polys, uint32_
   uint32_t chunks = 1u << (log_n - s);
   GS_REQUIRE(chunks <= 65535 * 32768u, "too many chunks");
   uint32_t* w = d_scratch;
-  uint32_t* partials = d_scratch + 4 * (1u << s);
+  // one chunk per polynomial: its sum is the value
+  uint32_t* partials = chunks == 1 ? d_out : d_scratch + 4 * (1u << s);
   eap_weights_kernel<<<((1u << s) + 255) / 256, 256, 0, st>>>(fs, s, w);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
@@ -241,13 +242,14 @@ int batch_eval_at_point(cudaStream_t st, const uint32_t* const* d_polys, uint32_
     // four polynomials per block (two: L1-bound again, 84 µs on the Poseidon2
     // 2^18 trace; eight: register-bound, 75 µs; four: 54 µs)
     dim3 grid(chunks, (n_polys + 3) / 4);
-    eap_chunk_multi_kernel<4><<<grid, 256, 0, st>>>(d_polys, n_polys, log_n, w, fs, partials);
+    eap_chunk_multi_kernel<4><<<grid, 256, 0, st>>>(polys, n_polys, log_n, w, fs, partials);
   } else {
     dim3 grid(chunks, n_polys);
-    eap_chunk_kernel<<<grid, 256, 0, st>>>(d_polys, log_n, s, w, fs, partials, vec);
+    eap_chunk_kernel<<<grid, 256, 0, st>>>(polys, log_n, s, w, fs, partials, vec);
   }
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
+  if (chunks == 1) return OK;
   eap_finalize_kernel<<<n_polys, 128, 0, st>>>(partials, chunks, n_polys, d_out);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());

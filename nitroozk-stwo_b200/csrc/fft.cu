@@ -121,8 +121,7 @@ __device__ __forceinline__ void bfly_b2(uint32_t& a, uint32_t& b, uint32_t w2) {
 __device__ __forceinline__ uint32_t swz(uint32_t e) { return e ^ ((e >> 5) & 31u); }
 
 template <bool INV, int R>
-__global__ void __launch_bounds__(256) fft_pass_kernel(const uint32_t* const* __restrict__ src_tab,
-                                                       uint32_t* const* __restrict__ dst_tab,
+__global__ void __launch_bounds__(256) fft_pass_kernel(Cols src_tab, MutCols dst_tab,
                                                        const uint32_t* __restrict__ tw, FftPass a) {
   extern __shared__ uint32_t sm[];
   constexpr int NQ = 1 << R;
@@ -235,8 +234,7 @@ __global__ void __launch_bounds__(256) fft_pass_kernel(const uint32_t* const* __
 __host__ __device__ constexpr uint32_t padw(uint32_t e) { return e + (e >> 5); }
 
 template <bool INV, int L, int C>
-__global__ void __launch_bounds__(256) fft_tile_kernel(const uint32_t* const* __restrict__ src_tab,
-                                                       uint32_t* const* __restrict__ dst_tab,
+__global__ void __launch_bounds__(256) fft_tile_kernel(Cols src_tab, MutCols dst_tab,
                                                        const uint32_t* __restrict__ tw, FftPass a) {
   extern __shared__ uint32_t sm[];
   constexpr int R = 5, NQ = 32;
@@ -395,8 +393,7 @@ struct StreamGrid {
 
 template <bool INV, int L, int C, int TB>
 __global__ void __launch_bounds__(1 << (TB - 5), (StreamShape<INV, L, C, TB>::PER_SM))
-    fft_stream_kernel(const uint32_t* const* __restrict__ src_tab, uint32_t* const* __restrict__ dst_tab,
-                      const uint32_t* __restrict__ tw, FftPass a, StreamGrid g) {
+    fft_stream_kernel(Cols src_tab, MutCols dst_tab, const uint32_t* __restrict__ tw, FftPass a, StreamGrid g) {
   using Shape = StreamShape<INV, L, C, TB>;
   constexpr int R = 5, NQ = 32, T = C > 0 ? TB : L;  // T: tile bits of one transform
   constexpr int K = (L + R - 1) / R;
@@ -596,7 +593,7 @@ struct SmallFft {
   uint32_t k[4];
   uint32_t src_mask;
 };
-__global__ void fft_small_kernel(const uint32_t* const* src_tab, uint32_t* const* dst_tab, SmallFft a, uint32_t n_cols) {
+__global__ void fft_small_kernel(Cols src_tab, MutCols dst_tab, SmallFft a, uint32_t n_cols) {
   uint32_t col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= n_cols) return;
   const uint32_t* s = src_tab[col];
@@ -648,7 +645,7 @@ static pt31 host_index_to_point(uint32_t k) {
 // Initial point of the half coset of CanonicCoset(n): index 2^(31 - (n + 1)).
 static pt31 canonic_half_coset_initial(uint32_t n) { return host_index_to_point(1u << (31 - (n + 1))); }
 
-static int launch_small(cudaStream_t st, const uint32_t* const* src, uint32_t* const* dst, uint32_t n_cols, uint32_t n,
+static int launch_small(cudaStream_t st, Cols src, MutCols dst, uint32_t n_cols, uint32_t n,
                         bool inverse, uint32_t src_mask) {
   pt31 p = canonic_half_coset_initial(n);
   SmallFft a{};
@@ -761,14 +758,14 @@ static void fft_partition(uint32_t layers, uint32_t n, std::vector<std::pair<uin
 }
 
 template <bool INV, int R>
-static void launch_pass(cudaStream_t st, dim3 grid, uint32_t threads, size_t smem, const uint32_t* const* s,
-                        uint32_t* const* d, const uint32_t* tw, const FftPass& a) {
+static void launch_pass(cudaStream_t st, dim3 grid, uint32_t threads, size_t smem, Cols s,
+                        MutCols d, const uint32_t* tw, const FftPass& a) {
   fft_pass_kernel<INV, R><<<grid, threads, smem, st>>>(s, d, tw, a);
   note_launch();
 }
 
 template <bool INV, int L, int C>
-static void launch_tile(cudaStream_t st, dim3 grid, uint32_t threads, const uint32_t* const* s, uint32_t* const* d,
+static void launch_tile(cudaStream_t st, dim3 grid, uint32_t threads, Cols s, MutCols d,
                         const uint32_t* tw, const FftPass& a) {
   const uint32_t words = 1u << (a.t + a.tile_shift);
   const size_t smem = (size_t)4 * (words + (words >> 5));
@@ -796,7 +793,7 @@ static uint32_t stream_tiles(uint32_t set_log, uint32_t units, uint32_t per_sm) 
 }
 
 template <bool INV, int L, int C, int TB>
-static int launch_stream(cudaStream_t st, uint32_t n_cols, const uint32_t* const* s, uint32_t* const* d,
+static int launch_stream(cudaStream_t st, uint32_t n_cols, Cols s, MutCols d,
                          const uint32_t* tw, const FftPass& a) {
   using Shape = StreamShape<INV, L, C, TB>;
   static const cudaError_t attr = cudaFuncSetAttribute(
@@ -821,7 +818,7 @@ static int launch_stream(cudaStream_t st, uint32_t n_cols, const uint32_t* const
 // takes 4 tiles to pay (one column of 2^24, a tile per block: 46 -> 77 us).
 constexpr uint32_t STREAM_MIN_TILES = 4;
 template <bool INV>
-static int launch_stream_any(cudaStream_t st, uint32_t n_cols, const uint32_t* const* s, uint32_t* const* d,
+static int launch_stream_any(cudaStream_t st, uint32_t n_cols, Cols s, MutCols d,
                              const uint32_t* tw, const FftPass& a, bool* taken) {
   *taken = false;
   if (fft_generic() || !a.vec_ok || (uint64_t)n_cols << a.n >= 1ull << 40) return OK;
@@ -846,8 +843,8 @@ static int launch_stream_any(cudaStream_t st, uint32_t n_cols, const uint32_t* c
 // passes with 16 or 32 contiguous words per tile row (C = 4 with 5..9 layers,
 // C = 5 with 5..8); anything else runs the generic pass.
 template <bool INV>
-static bool launch_tile_any(cudaStream_t st, dim3 grid, uint32_t threads, const uint32_t* const* s,
-                            uint32_t* const* d, const uint32_t* tw, const FftPass& a) {
+static bool launch_tile_any(cudaStream_t st, dim3 grid, uint32_t threads, Cols s,
+                            MutCols d, const uint32_t* tw, const FftPass& a) {
   if (fft_generic()) return false;
 #define GS_TILE(LL, CC) \
   case LL: launch_tile<INV, LL, CC>(st, grid, threads, s, d, tw, a); return true;
@@ -866,12 +863,12 @@ static bool launch_tile_any(cudaStream_t st, dim3 grid, uint32_t threads, const 
 }
 
 // Column pointers of the current call are 16-byte aligned (checked by the
-// callers that know them on the host; the device tables are opaque here).
+// callers that know them on the host; a device table is opaque here).
 static thread_local bool g_cols_aligned = true;
 void fft_set_columns_aligned(bool aligned) { g_cols_aligned = aligned; }
 
 template <bool INV>
-static int run_passes(cudaStream_t st, const uint32_t* const* src, uint32_t* const* dst, uint32_t n_cols, uint32_t n,
+static int run_passes(cudaStream_t st, Cols src, MutCols dst, uint32_t n_cols, uint32_t n,
                       uint32_t layers, uint32_t src_mask, const uint32_t* tw, uint32_t tw_len) {
   std::vector<std::pair<uint32_t, uint32_t>> parts;
   fft_partition(layers, n, parts);
@@ -898,7 +895,7 @@ static int run_passes(cudaStream_t st, const uint32_t* const* src, uint32_t* con
     const uint32_t threads = 1u << (tpt_log + tile_shift);
     const size_t smem = (size_t)4 << (a.t + tile_shift);
     dim3 grid(1u << (tiles_log - tile_shift), n_cols);
-    const uint32_t* const* s = (p == 0) ? src : (const uint32_t* const*)dst;
+    Cols s = (p == 0) ? src : Cols(dst);
     bool taken = false;
     GS_TRY(launch_stream_any<INV>(st, n_cols, s, dst, tw, a, &taken));
     if (taken) continue;
@@ -918,19 +915,19 @@ static int run_passes(cudaStream_t st, const uint32_t* const* src, uint32_t* con
   return OK;
 }
 
-int interpolate_columns(cudaStream_t st, uint32_t* const* d_cols, uint32_t n_cols, uint32_t log_n,
+int interpolate_columns(cudaStream_t st, MutCols d_cols, uint32_t n_cols, uint32_t log_n,
                         const uint32_t* d_itwiddles, uint32_t tw_log) {
   if (n_cols == 0) return OK;
   GS_REQUIRE(log_n >= 1 && log_n <= 30, "log_n out of range");
   GS_REQUIRE(n_cols <= 65535, "too many columns in one call");
-  if (log_n <= 2) return launch_small(st, (const uint32_t* const*)d_cols, d_cols, n_cols, log_n, true, 0xffffffffu);
+  if (log_n <= 2) return launch_small(st, d_cols, d_cols, n_cols, log_n, true, 0xffffffffu);
   GS_REQUIRE(tw_log + 1 >= log_n, "twiddle tree too small for the domain");
-  return run_passes<true>(st, (const uint32_t* const*)d_cols, d_cols, n_cols, log_n, log_n, 0xffffffffu, d_itwiddles,
+  return run_passes<true>(st, d_cols, d_cols, n_cols, log_n, log_n, 0xffffffffu, d_itwiddles,
                           1u << tw_log);
 }
 
 // Out-of-place interpolation (src and dst tables may differ).
-int interpolate_columns_to(cudaStream_t st, const uint32_t* const* d_src, uint32_t* const* d_dst, uint32_t n_cols,
+int interpolate_columns_to(cudaStream_t st, Cols d_src, MutCols d_dst, uint32_t n_cols,
                            uint32_t log_n, const uint32_t* d_itwiddles, uint32_t tw_log) {
   if (n_cols == 0) return OK;
   GS_REQUIRE(log_n >= 1 && log_n <= 30, "log_n out of range");
@@ -940,7 +937,7 @@ int interpolate_columns_to(cudaStream_t st, const uint32_t* const* d_src, uint32
   return run_passes<true>(st, d_src, d_dst, n_cols, log_n, log_n, 0xffffffffu, d_itwiddles, 1u << tw_log);
 }
 
-int evaluate_columns(cudaStream_t st, const uint32_t* const* d_src, uint32_t coeff_log, uint32_t* const* d_dst,
+int evaluate_columns(cudaStream_t st, Cols d_src, uint32_t coeff_log, MutCols d_dst,
                      uint32_t n_cols, uint32_t log_n, const uint32_t* d_twiddles, uint32_t tw_log) {
   if (n_cols == 0) return OK;
   GS_REQUIRE(log_n >= 1 && log_n <= 30, "log_n out of range");
@@ -1041,16 +1038,10 @@ int fft_worklist(Context& ctx, const FftItem* items, uint32_t n_items, const uin
   for (uint32_t k = 0; k < n_items; k++) {
     const FftItem& x = items[k];
     if (x.log >= FFT_WL_MIN_LOG && x.log <= FFT_WL_MAX_LOG) continue;
-    const void* const* ts = nullptr;
-    const void* const* td = nullptr;
-    GS_TRY(ctx.stage_ptrs((const void* const*)&x.src, 1, &ts));
-    GS_TRY(ctx.stage_ptrs((const void* const*)&x.dst, 1, &td));
     if (x.inverse)
-      GS_TRY(interpolate_columns_to(st, (const uint32_t* const*)ts, (uint32_t* const*)td, 1, x.log, d_itwiddles,
-                                    tw_log));
+      GS_TRY(interpolate_columns_to(st, Cols(x.src, 0), MutCols(x.dst, 0), 1, x.log, d_itwiddles, tw_log));
     else
-      GS_TRY(evaluate_columns(st, (const uint32_t* const*)ts, x.coeff_log, (uint32_t* const*)td, 1, x.log,
-                              d_twiddles, tw_log));
+      GS_TRY(evaluate_columns(st, Cols(x.src, 0), x.coeff_log, MutCols(x.dst, 0), 1, x.log, d_twiddles, tw_log));
   }
   if (wl.empty()) return OK;
   const void* d = nullptr;

@@ -69,7 +69,8 @@ struct SmallInvY { uint32_t v[2]; };
 
 __global__ void fold_circle_kernel(CPlanes src, uint32_t log_n, qm31 alpha, qm31 alpha_sq, Planes dst,
                                    const uint32_t* __restrict__ itw, uint32_t tw_len, SmallInvY small,
-                                   uint32_t* leaf_out, const uint32_t* __restrict__ d_alpha, uint32_t one) {
+                                   uint32_t* leaf_out, const uint32_t* __restrict__ d_alpha, uint32_t one,
+                                   uint32_t fresh) {
   const size_t half = (size_t)1 << (log_n - 1);
   if (d_alpha) {
     alpha = qm_make(d_alpha[0], d_alpha[1], d_alpha[2], d_alpha[3]);
@@ -90,8 +91,11 @@ __global__ void fold_circle_kernel(CPlanes src, uint32_t log_n, qm31 alpha, qm31
     qm31 f0 = qm_add(fp, fnp);
     qm31 f1 = qm_mul_m31(qm_sub(fp, fnp), yinv);
     qm31 fprime = qm_add(qm_mul(alpha, f1), f0);
-    qm31 d = qm_make(dst.p[0][i], dst.p[1][i], dst.p[2][i], dst.p[3][i]);
-    qm31 r = qm_add(qm_mul(d, alpha_sq), fprime);
+    qm31 r = fprime;
+    if (!fresh) {  // (a fresh dst counts as zero and is not read)
+      qm31 d = qm_make(dst.p[0][i], dst.p[1][i], dst.p[2][i], dst.p[3][i]);
+      r = qm_add(qm_mul(d, alpha_sq), fprime);
+    }
     dst.p[0][i] = r.x.a; dst.p[1][i] = r.x.b; dst.p[2][i] = r.y.a; dst.p[3][i] = r.y.b;
     if (leaf_out) leaf_hash4(leaf_out, i, r, one);
   }
@@ -133,7 +137,8 @@ int fold_line_dev_alpha(cudaStream_t st, CPlanes src, uint32_t log_n, const uint
 }
 
 static int fold_circle_launch(cudaStream_t st, CPlanes src, uint32_t log_n, qm31 alpha, Planes dst,
-                              const uint32_t* d_itw, uint32_t tw_log, uint32_t* leaf_out, const uint32_t* d_alpha) {
+                              const uint32_t* d_itw, uint32_t tw_log, uint32_t* leaf_out, const uint32_t* d_alpha,
+                              bool fresh = false) {
   GS_REQUIRE(log_n >= 1 && log_n <= tw_log + 1, "fold_circle_into_line: domain must fit the twiddle tree");
   SmallInvY small{{0, 0}};
   if (log_n < 3) {
@@ -148,7 +153,7 @@ static int fold_circle_launch(cudaStream_t st, CPlanes src, uint32_t log_n, qm31
   qm31 alpha_sq = qm_mul(alpha, alpha);
   size_t half = (size_t)1 << (log_n - 1);
   fold_circle_kernel<<<grid_for(half, 256), 256, 0, st>>>(src, log_n, alpha, alpha_sq, dst, d_itw, 1u << tw_log, small,
-                                                          leaf_out, d_alpha, 1u);
+                                                          leaf_out, d_alpha, 1u, fresh ? 1u : 0u);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;
@@ -157,9 +162,14 @@ int fold_circle_into_line_fused(cudaStream_t st, CPlanes src, uint32_t log_n, qm
                                 const uint32_t* d_itw, uint32_t tw_log, uint32_t* leaf_out) {
   return fold_circle_launch(st, src, log_n, alpha, dst, d_itw, tw_log, leaf_out, nullptr);
 }
-int fold_circle_into_line_dev_alpha(cudaStream_t st, CPlanes src, uint32_t log_n, const uint32_t* d_alpha, Planes dst,
-                                    const uint32_t* d_itw, uint32_t tw_log, uint32_t* leaf_out) {
-  return fold_circle_launch(st, src, log_n, qm_zero(), dst, d_itw, tw_log, leaf_out, d_alpha);
+// The same into planes that hold nothing yet (dst counts as zero).
+int fold_circle_fresh(cudaStream_t st, CPlanes src, uint32_t log_n, qm31 alpha, Planes dst, const uint32_t* d_itw,
+                      uint32_t tw_log) {
+  return fold_circle_launch(st, src, log_n, alpha, dst, d_itw, tw_log, nullptr, nullptr, true);
+}
+int fold_circle_fresh_dev_alpha(cudaStream_t st, CPlanes src, uint32_t log_n, const uint32_t* d_alpha, Planes dst,
+                                const uint32_t* d_itw, uint32_t tw_log, uint32_t* leaf_out) {
+  return fold_circle_launch(st, src, log_n, qm_zero(), dst, d_itw, tw_log, leaf_out, d_alpha, true);
 }
 
 // Fused tail of the FRI commit phase: every layer of log size <= 11 in one

@@ -30,8 +30,8 @@ __device__ __forceinline__ void store_hash(uint32_t* out, size_t i, const uint32
 // FMA: adds of the compression on the FMA pipe (blake2s_compress_f).
 template <bool FMA>
 __global__ void __launch_bounds__(256) merkle_layer_kernel(uint32_t log_size, const uint32_t* __restrict__ prev,
-                                                           const uint32_t* const* __restrict__ cols, uint32_t n_cols,
-                                                           uint32_t* __restrict__ out, uint32_t one) {
+                                                           Cols cols, uint32_t n_cols, uint32_t* __restrict__ out,
+                                                           uint32_t one) {
   const size_t n = (size_t)1 << log_size;
   const uint32_t prev_words = prev ? 16u : 0u;
   const uint32_t total_words = prev_words + n_cols;
@@ -86,8 +86,7 @@ constexpr int COL_WARPS = 4;
 template <bool PREV>
 __global__ void __launch_bounds__(32 * COL_WARPS, 8)
     merkle_columns_kernel(uint32_t log_size, const uint32_t* __restrict__ prev,
-                          const uint32_t* const* __restrict__ cols, uint32_t n_cols, uint32_t* __restrict__ out,
-                          uint32_t one) {
+                          Cols cols, uint32_t n_cols, uint32_t* __restrict__ out, uint32_t one) {
   __shared__ uint4 stage[COL_WARPS][2][16 * 8];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t n_tiles = 1u << (log_size - 5), n_warps = gridDim.x * COL_WARPS;
@@ -189,11 +188,10 @@ int lifted_leaves(cudaStream_t st, uint32_t lift, const uint32_t* const* d_cols,
   return OK;
 }
 
-int commit_on_layer(cudaStream_t st, uint32_t log_size, const uint32_t* d_prev, const uint32_t* const* d_cols,
-                    uint32_t n_cols, uint32_t* d_out, bool cols_aligned) {
+int commit_on_layer(cudaStream_t st, uint32_t log_size, const uint32_t* d_prev, Cols cols, uint32_t n_cols, uint32_t* d_out, bool cols_aligned) {
   GS_REQUIRE(log_size <= 30, "layer log size out of range");
   GS_REQUIRE(d_out != nullptr, "null output");
-  GS_REQUIRE(n_cols == 0 || d_cols != nullptr, "null column table");
+  GS_REQUIRE(n_cols == 0 || cols.given(), "null column table");
   GS_REQUIRE(((uintptr_t)d_out & 15) == 0 && ((uintptr_t)d_prev & 15) == 0, "hash buffers must be 16-byte aligned");
   size_t n = (size_t)1 << log_size;
   int threads = 256;
@@ -209,13 +207,13 @@ int commit_on_layer(cudaStream_t st, uint32_t log_size, const uint32_t* d_prev, 
     const size_t resident = (size_t)num_sms() * 8;  // one wave; a warp walks its tiles, copies crossing from one to the next
     const unsigned grid = (unsigned)(tiles < resident ? tiles : resident);
     if (d_prev)
-      merkle_columns_kernel<true><<<grid, 32 * COL_WARPS, 0, st>>>(log_size, d_prev, d_cols, n_cols, d_out, 1u);
+      merkle_columns_kernel<true><<<grid, 32 * COL_WARPS, 0, st>>>(log_size, d_prev, cols, n_cols, d_out, 1u);
     else
-      merkle_columns_kernel<false><<<grid, 32 * COL_WARPS, 0, st>>>(log_size, d_prev, d_cols, n_cols, d_out, 1u);
+      merkle_columns_kernel<false><<<grid, 32 * COL_WARPS, 0, st>>>(log_size, d_prev, cols, n_cols, d_out, 1u);
   } else if (alu_only)
-    merkle_layer_kernel<false><<<(unsigned)blocks, threads, 0, st>>>(log_size, d_prev, d_cols, n_cols, d_out, 1u);
+    merkle_layer_kernel<false><<<(unsigned)blocks, threads, 0, st>>>(log_size, d_prev, cols, n_cols, d_out, 1u);
   else
-    merkle_layer_kernel<true><<<(unsigned)blocks, threads, 0, st>>>(log_size, d_prev, d_cols, n_cols, d_out, 1u);
+    merkle_layer_kernel<true><<<(unsigned)blocks, threads, 0, st>>>(log_size, d_prev, cols, n_cols, d_out, 1u);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;
@@ -448,11 +446,11 @@ int merkle_worklist(Context& ctx, const MerkleItem* items, uint32_t n_items) {
   for (uint32_t k = 0; k < n_items; k++) {
     const MerkleItem& x = items[k];
     if (x.log <= MERKLE_WL_MAX_LOG) continue;
-    const void* const* d = nullptr;
-    GS_TRY(ctx.stage_ptrs((const void* const*)x.cols, x.n_cols, &d));
+    Cols cols;
+    GS_TRY(ctx.columns(x.cols, x.n_cols, &cols));
     bool aligned = true;
     for (uint32_t c = 0; c < x.n_cols; c++) aligned = aligned && ((uintptr_t)x.cols[c] & 15) == 0;
-    GS_TRY(commit_on_layer(st, x.log, nullptr, (const uint32_t* const*)d, x.n_cols, x.layers[x.log], aligned));
+    GS_TRY(commit_on_layer(st, x.log, nullptr, cols, x.n_cols, x.layers[x.log], aligned));
     GS_TRY(commit_node_layers(st, x.log, x.layers, ctx.tree_counters));
   }
   uint32_t first[MERKLE_WL_MAX_LOG + 1] = {0}, total = 0, max_log = 0;
@@ -534,7 +532,7 @@ int commit_node_layers_ch(cudaStream_t st, uint32_t top_log, uint32_t* const* la
   if (!legacy) {
     uint32_t top = top_log;
     while (top > TREE_MAX_LOG) {  // layers above 2^27 nodes: one launch each
-      GS_TRY(commit_on_layer(st, top - 1, layers[top], nullptr, 0, layers[top - 1]));
+      GS_TRY(commit_on_layer(st, top - 1, layers[top], Cols(), 0, layers[top - 1]));
       top--;
     }
     if (top == 0) {
@@ -571,7 +569,7 @@ int commit_node_layers_ch(cudaStream_t st, uint32_t top_log, uint32_t* const* la
   // one cluster launch.
   uint32_t top = top_log;
   while (top > MERKLE_TAIL_LOG) {
-    GS_TRY(commit_on_layer(st, top - 1, layers[top], nullptr, 0, layers[top - 1]));
+    GS_TRY(commit_on_layer(st, top - 1, layers[top], Cols(), 0, layers[top - 1]));
     top--;
   }
   int L = (int)top - 1;

@@ -524,7 +524,7 @@ __device__ __forceinline__ void store_hash(uint8_t* base, size_t i, const Felt& 
 // Value k of a node's input sequence: the children (when there is a previous
 // layer), then the column words of 8 values each.
 __device__ __forceinline__ Felt node_value(uint32_t k, size_t i, const uint8_t* prev,
-                                           const uint32_t* const* cols, uint32_t n_cols) {
+                                           const Cols& cols, uint32_t n_cols) {
   if (prev) {
     if (k < 2) return load_hash(prev, 2 * i + k);
     k -= 2;
@@ -549,8 +549,8 @@ __device__ __forceinline__ Felt node_value(uint32_t k, size_t i, const uint8_t* 
 // columns) is one permutation of (l, r, 2). Either way one call site of the
 // permutation, inlined with the state in registers.
 __global__ void __launch_bounds__(128) poseidon252_layer_kernel(uint32_t log_size, const uint8_t* __restrict__ prev,
-                                                                const uint32_t* const* __restrict__ cols,
-                                                                uint32_t n_cols, uint8_t* __restrict__ out) {
+                                                                Cols cols, uint32_t n_cols,
+                                                                uint8_t* __restrict__ out) {
   const size_t n = (size_t)1 << log_size;
   const bool node_only = prev && n_cols == 0;
   const uint32_t m = (prev ? 2u : 0u) + (n_cols + 7) / 8;  // values
@@ -582,16 +582,16 @@ __global__ void poseidon252_permute_kernel(const uint8_t* __restrict__ in, uint3
 }
 
 int poseidon252_commit_on_layer(cudaStream_t st, uint32_t log_size, const uint8_t* d_prev,
-                                const uint32_t* const* d_cols, uint32_t n_cols, uint8_t* d_out) {
+                                Cols cols, uint32_t n_cols, uint8_t* d_out) {
   GS_REQUIRE(log_size <= 30, "layer log size out of range");
   GS_REQUIRE(d_out != nullptr, "null output");
-  GS_REQUIRE(n_cols == 0 || d_cols != nullptr, "null column table");
+  GS_REQUIRE(n_cols == 0 || cols.given(), "null column table");
   GS_REQUIRE(((uintptr_t)d_out & 15) == 0 && ((uintptr_t)d_prev & 15) == 0, "hash buffers must be 16-byte aligned");
   const size_t n = (size_t)1 << log_size;
   size_t blocks = (n + 127) / 128;
   const size_t cap = (size_t)num_sms() * 16;
   if (blocks > cap) blocks = cap;
-  poseidon252_layer_kernel<<<(unsigned)blocks, 128, 0, st>>>(log_size, d_prev, d_cols, n_cols, d_out);
+  poseidon252_layer_kernel<<<(unsigned)blocks, 128, 0, st>>>(log_size, d_prev, cols, n_cols, d_out);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;

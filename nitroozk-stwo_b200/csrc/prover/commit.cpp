@@ -38,8 +38,7 @@ struct CommitPlan {
     uint32_t* evals = nullptr;          // contiguous, column stride `stride_e`
     size_t stride_c = 0, stride_e = 0;
     const uint32_t* const* d_src = nullptr;  // into d_src_table
-    uint32_t* const* d_coeffs = nullptr;
-    uint32_t* const* d_evals = nullptr;
+    MutCols d_coeffs, d_evals;
   };
   std::vector<Group> groups;
   std::vector<uint32_t*> layers;        // layers[L]: 2^L hashes
@@ -66,7 +65,7 @@ int CommitPlan::enqueue(bool inputs_aligned) {
     fft_set_columns_aligned(inputs_aligned);
     GS_TRY(interpolate_columns_to(st, g.d_src, g.d_coeffs, (uint32_t)g.cols.size(), g.log, itw, tw_log));
     fft_set_columns_aligned(true);
-    GS_TRY(evaluate_columns(st, (const uint32_t* const*)g.d_coeffs, g.log, g.d_evals, (uint32_t)g.cols.size(),
+    GS_TRY(evaluate_columns(st, g.d_coeffs, g.log, g.d_evals, (uint32_t)g.cols.size(),
                             g.log + blowup, tw, tw_log));
   }
   // 3. Merkle tree, from the largest layer down
@@ -77,7 +76,7 @@ int CommitPlan::enqueue(bool inputs_aligned) {
     if (inj) gi++;
     const uint32_t* prev = L == max_eval ? nullptr : layers[L + 1];
     if (inj || L == max_eval) {
-      GS_TRY(commit_on_layer(st, L, prev, inj ? (const uint32_t* const*)inj->d_evals : nullptr,
+      GS_TRY(commit_on_layer(st, L, prev, inj ? Cols(inj->d_evals) : Cols(),
                              inj ? (uint32_t)inj->cols.size() : 0, layers[L], true));  // carved at 256 bytes
       if (L == 0) break;
       L--;
@@ -90,7 +89,7 @@ int CommitPlan::enqueue(bool inputs_aligned) {
       break;
     }
     while (L > stop) {
-      GS_TRY(commit_on_layer(st, L, layers[L + 1], nullptr, 0, layers[L], true));
+      GS_TRY(commit_on_layer(st, L, layers[L + 1], Cols(), 0, layers[L], true));
       L--;
     }
   }
@@ -182,8 +181,8 @@ int plan_create(Context& ctx, const uint32_t* log_sizes, uint32_t n, uint32_t bl
     g.stride_e = up64((size_t)1 << (lg + blowup));
     p->groups.push_back(g);
   }
-  // one device block: pointer tables, coefficients, evaluations, layers
-  size_t words = 3 * up64(2 * (size_t)n);  // src / coeff / eval tables (8 bytes per pointer)
+  // one device block: pointer table, coefficients, evaluations, layers
+  size_t words = up64(2 * (size_t)n);  // the source table (8 bytes per pointer)
   for (auto& g : p->groups) words += g.cols.size() * (g.stride_c + g.stride_e);
   for (uint32_t L = 0; L <= p->max_eval; L++) words += up64((size_t)8 << L);
   words += up64(TREE_COUNTERS);  // the tree kernel's tickets, owned by the plan's stream
@@ -191,28 +190,20 @@ int plan_create(Context& ctx, const uint32_t* log_sizes, uint32_t n, uint32_t bl
   uint32_t* carve = (uint32_t*)p->block;
   auto take = [&](size_t w) { uint32_t* q = carve; carve += up64(w); return q; };
   uint32_t* t_src = take(2 * (size_t)n);
-  uint32_t* t_coef = take(2 * (size_t)n);
-  uint32_t* t_eval = take(2 * (size_t)n);
   p->d_src_table = (const void**)t_src;
-  std::vector<const void*> h_src, h_coef, h_eval;  // host images of the tables
+  size_t n_src = 0;
   for (auto& g : p->groups) {
     g.coeffs = take(g.cols.size() * g.stride_c);
     g.evals = take(g.cols.size() * g.stride_e);
     // the group's slice of the source table, written at each run
-    g.d_src = (const uint32_t* const*)((const void**)t_src + h_src.size());
-    g.d_coeffs = (uint32_t* const*)((const void**)t_coef + h_coef.size());
-    g.d_evals = (uint32_t* const*)((const void**)t_eval + h_eval.size());
-    for (size_t k = 0; k < g.cols.size(); k++) {
-      h_src.push_back(nullptr);
-      h_coef.push_back(g.coeffs + k * g.stride_c);
-      h_eval.push_back(g.evals + k * g.stride_e);
-    }
+    g.d_src = (const uint32_t* const*)((const void**)t_src + n_src);
+    g.d_coeffs = MutCols(g.coeffs, g.stride_c);
+    g.d_evals = MutCols(g.evals, g.stride_e);
+    n_src += g.cols.size();
   }
   p->layers.resize(p->max_eval + 1);
   for (uint32_t L = 0; L <= p->max_eval; L++) p->layers[L] = take((size_t)8 << L);
   p->counters = take(TREE_COUNTERS);
-  GS_CUDA_TRY(cudaMemcpy(t_coef, h_coef.data(), h_coef.size() * sizeof(void*), cudaMemcpyHostToDevice));
-  GS_CUDA_TRY(cudaMemcpy(t_eval, h_eval.data(), h_eval.size() * sizeof(void*), cudaMemcpyHostToDevice));
   p->tw_log = p->max_eval - 1;
   GS_TRY(ctx.twiddles(p->tw_log, &p->tw, &p->itw));
   GS_CUDA_TRY(cudaStreamSynchronize(ctx.stream));

@@ -23,19 +23,20 @@ static int fri_commit_p252(Prover& pv, uint32_t* quot[4], uint32_t lifting, FriL
   GS_REQUIRE(lifting >= last_log + 1, "FRI: lifting domain below the last layer");
   auto planes_of = [&](FriLayerDev& L, uint32_t log) -> int {
     L.log = log;
-    for (int c = 0; c < 4; c++) GS_TRY(pv.A.alloc_n((size_t)1 << log, &L.planes[c]));
+    const size_t stride = log < 6 ? 64 : (size_t)1 << log;
+    GS_TRY(pv.A.alloc_n(4 * stride, &L.planes[0]));
+    for (int c = 1; c < 4; c++) L.planes[c] = L.planes[0] + c * stride;
     return OK;
   };
   bool busy_done = false;
   auto commit_layer = [&](FriLayerDev& L) -> int {
     L.layers.assign(L.log + 1, nullptr);
     for (uint32_t k = 0; k <= L.log; k++) GS_TRY(pv.A.alloc_n((size_t)8 << k, &L.layers[k]));
-    std::vector<const uint32_t*> cols = {L.planes[0], L.planes[1], L.planes[2], L.planes[3]};
-    const uint32_t* const* tab = nullptr;
-    GS_TRY(pv.table(cols, &tab));
-    GS_TRY(poseidon252_commit_on_layer(st, L.log, nullptr, tab, 4, (uint8_t*)L.layers[L.log]));
+    Cols cols;
+    GS_TRY(pv.ctx.columns(L.planes, 4, &cols));
+    GS_TRY(poseidon252_commit_on_layer(st, L.log, nullptr, cols, 4, (uint8_t*)L.layers[L.log]));
     for (int k = (int)L.log - 1; k >= 0; k--)
-      GS_TRY(poseidon252_commit_on_layer(st, (uint32_t)k, (const uint8_t*)L.layers[k + 1], nullptr, 0,
+      GS_TRY(poseidon252_commit_on_layer(st, (uint32_t)k, (const uint8_t*)L.layers[k + 1], Cols(), 0,
                                          (uint8_t*)L.layers[k]));
     if (!busy_done && while_busy) while_busy();  // overlaps the first tree
     busy_done = true;
@@ -49,10 +50,8 @@ static int fri_commit_p252(Prover& pv, uint32_t* quot[4], uint32_t lifting, FriL
   qm31 alpha = pv.ch.draw_felt();
   FriLayerDev cur;
   GS_TRY(planes_of(cur, lifting - 1));
-  for (int c = 0; c < 4; c++) GS_CUDA_TRY(cudaMemsetAsync(cur.planes[c], 0, (size_t)4 << cur.log, st));
-  GS_TRY(fold_circle_into_line_fused(st, CPlanes{{quot[0], quot[1], quot[2], quot[3]}}, lifting, alpha,
-                                     Planes{{cur.planes[0], cur.planes[1], cur.planes[2], cur.planes[3]}}, pv.itw,
-                                     pv.tw_log, nullptr));
+  GS_TRY(fold_circle_fresh(st, CPlanes{{quot[0], quot[1], quot[2], quot[3]}}, lifting, alpha,
+                           Planes{{cur.planes[0], cur.planes[1], cur.planes[2], cur.planes[3]}}, pv.itw, pv.tw_log));
   while (cur.log > last_log) {
     GS_TRY(commit_layer(cur));
     alpha = pv.ch.draw_felt();
@@ -118,8 +117,7 @@ int fri_commit(Prover& pv, uint32_t* quot[4], uint32_t lifting, FriLayerDev& fir
   const size_t ctl_words = up(ctl_used);
   size_t words = ctl_words + tree_words(lifting);
   for (uint32_t lg = lifting - 1;; lg--) {
-    words += 4 * up((size_t)1 << lg);
-    if (lg > last_log) words += tree_words(lg);
+    if (lg > last_log) words += 4 * up((size_t)1 << lg) + tree_words(lg);
     if (lg == last_log) break;
   }
   uint32_t* block = nullptr;
@@ -133,41 +131,39 @@ int fri_commit(Prover& pv, uint32_t* quot[4], uint32_t lifting, FriLayerDev& fir
   uint32_t* ctl = take(ctl_words);  // [0,16): channel state; then roots, then challenges
   uint32_t* d_roots = ctl + 16;
   uint32_t* d_felts = d_roots + 8 * (size_t)n_roots;
+  uint32_t* d_last = d_felts + 8 * (size_t)n_roots;
   auto take_tree = [&](FriLayerDev& L) {
     L.layers.assign(L.log + 1, nullptr);
     for (uint32_t k = 0; k <= L.log; k++) L.layers[k] = take((size_t)8 << k);
   };
   auto take_layer = [&](FriLayerDev& L, uint32_t log) {
     L.log = log;
-    for (int c = 0; c < 4; c++) L.planes[c] = take((size_t)1 << log);
+    // the last layer's values go where they are read back
+    for (int c = 0; c < 4; c++) L.planes[c] = log > last_log ? take((size_t)1 << log) : d_last + ((size_t)c << log);
     if (log > last_log) take_tree(L);
   };
   {
     uint32_t h[16] = {0};
     for (int j = 0; j < 8; j++) h[j] = host::word(pv.ch.digest, j);
     h[8] = pv.ch.n_draws;
-    const void* d = nullptr;
-    GS_TRY(pv.ctx.stage_bytes(h, sizeof h, &d));
-    GS_CUDA_TRY(cudaMemcpyAsync(ctl, d, sizeof h, cudaMemcpyDeviceToDevice, st));
+    GS_TRY(pv.ctx.stage_to(ctl, h, sizeof h));
   }
   // first layer: the quotient columns themselves
   first.log = lifting;
   for (int c = 0; c < 4; c++) first.planes[c] = quot[c];
   take_tree(first);
   {
-    std::vector<const uint32_t*> cols = {quot[0], quot[1], quot[2], quot[3]};
-    const uint32_t* const* tab = nullptr;
-    GS_TRY(pv.table(cols, &tab));
-    GS_TRY(commit_on_layer(st, lifting, nullptr, tab, 4, first.layers[lifting], true));
+    Cols cols;
+    GS_TRY(pv.ctx.columns(first.planes, 4, &cols));
+    GS_TRY(commit_on_layer(st, lifting, nullptr, cols, 4, first.layers[lifting], true));
   }
   GS_TRY(commit_node_layers_ch(st, first.log, first.layers.data(), pv.ctx.tree_counters, ctl, d_roots, d_felts));
-  // fold the circle evaluation into the first line layer (zero-initialised)
+  // fold the circle evaluation into the first line layer
   FriLayerDev cur;
   take_layer(cur, lifting - 1);
-  for (int c = 0; c < 4; c++) GS_CUDA_TRY(cudaMemsetAsync(cur.planes[c], 0, (size_t)4 << cur.log, st));
-  GS_TRY(fold_circle_into_line_dev_alpha(st, CPlanes{{quot[0], quot[1], quot[2], quot[3]}}, lifting, d_felts,
-                                         Planes{{cur.planes[0], cur.planes[1], cur.planes[2], cur.planes[3]}},
-                                         pv.itw, pv.tw_log, cur.log > last_log ? cur.layers[cur.log] : nullptr));
+  GS_TRY(fold_circle_fresh_dev_alpha(st, CPlanes{{quot[0], quot[1], quot[2], quot[3]}}, lifting, d_felts,
+                                     Planes{{cur.planes[0], cur.planes[1], cur.planes[2], cur.planes[3]}}, pv.itw,
+                                     pv.tw_log, cur.log > last_log ? cur.layers[cur.log] : nullptr));
   uint32_t k = 1;
   while (cur.log > last_log) {
     if (cur.log <= FRI_TAIL_LOG) {
@@ -203,11 +199,7 @@ int fri_commit(Prover& pv, uint32_t* quot[4], uint32_t lifting, FriLayerDev& fir
     k++;
   }
   // one read-back through pinned memory: channel state, roots, challenges
-  // and the last layer (copied next to them on the device)
-  size_t n = (size_t)1 << cur.log;
-  uint32_t* d_last = ctl + 16 + 16 * (size_t)n_roots;
-  for (int c = 0; c < 4; c++)
-    GS_CUDA_TRY(cudaMemcpyAsync(d_last + c * n, cur.planes[c], 4 * n, cudaMemcpyDeviceToDevice, st));
+  // and the last layer, which lies next to them
   if (dev_pow) GS_TRY(fri_last_layer_pow(st, d_last, cur.log, pv.cfg.log_last_layer, pv.cfg.pow_bits, ctl, ctl + pow_off));
   std::vector<uint32_t> hc(ctl_used);
   if (while_busy) while_busy();
@@ -407,10 +399,8 @@ int prove_component(Context& ctx, const ProveRequest& req, std::string* proof_by
   uint32_t* trace = nullptr;
   GS_TRY(pv.A.alloc_n((size_t)air.n_trace_cols() << T, &trace));
   if (air.kind == AirKind::WideFibonacci) {
-    if (req.input_mode == 2) {
-      GS_CUDA_TRY(cudaMemcpyAsync(trace, req.host_inputs, 4 * n, cudaMemcpyHostToDevice, st));
-      GS_CUDA_TRY(cudaMemcpyAsync(trace + n, req.host_inputs + n, 4 * n, cudaMemcpyHostToDevice, st));
-    }
+    if (req.input_mode == 2)
+      GS_CUDA_TRY(cudaMemcpyAsync(trace, req.host_inputs, 2 * 4 * n, cudaMemcpyHostToDevice, st));
     GS_TRY(wf_trace(st, trace, T, air.n_cols, req.seed, req.input_mode));
   } else {
     if (req.input_mode == 2)

@@ -243,7 +243,7 @@ int prove_tail(Prover& pv, AirHost& air, uint32_t split, std::string* proof_byte
       bool vec = true;
       for (auto* c : tr.coeff_ptrs) vec = vec && ((uintptr_t)c & 15) == 0;
       const bool side = split_streams && i == big;
-      GS_TRY(batch_eval_at_point(side ? pv.ctx.side : st, tr.coeff_tab, tr.n_cols, tr.coeff_log,
+      GS_TRY(batch_eval_at_point(side ? pv.ctx.side : st, tr.coeffs, tr.n_cols, tr.coeff_log,
                                  host::ptq_rep_double(r.p, lifting - tr.eval_log), d_vals + 4 * r.slot,
                                  (uint32_t*)(side ? eval_scratch_big : eval_scratch), 12, vec));
     }
@@ -326,7 +326,8 @@ int prove_tail(Prover& pv, AirHost& air, uint32_t split, std::string* proof_byte
                                  Planes{{pa.res, pa.res + nn, pa.res + 2 * nn, pa.res + 3 * nn}}));
     }
   uint32_t* quot[4];
-  for (int c = 0; c < 4; c++) GS_TRY(pv.A.alloc_n((size_t)1 << lifting, &quot[c]));
+  GS_TRY(pv.A.alloc_n((size_t)4 << lifting, &quot[0]));
+  for (int c = 1; c < 4; c++) quot[c] = quot[0] + ((size_t)c << lifting);
   {
     DomainTables dt;
     GS_TRY(pv.ctx.domain_tables(lifting, &dt));

@@ -108,7 +108,7 @@ struct Arena {
 struct Tree {
   uint32_t n_cols = 0;
   uint32_t coeff_log = 0, eval_log = 0;
-  const uint32_t* const* coeff_tab = nullptr;  // device pointer tables
+  Cols coeffs;
   uint32_t* evals = nullptr;
   std::vector<const uint32_t*> coeff_ptrs;    // host copies of the column pointers
   std::vector<uint32_t*> layers;              // layers[L]: 2^L hashes; empty tree: none
@@ -119,6 +119,7 @@ struct Tree {
   uint32_t ext_log = 0;
   uint32_t ext_done = 0;  // columns [0, ext_done) extended
   uint32_t max_log() const { return layers.empty() ? 0 : (uint32_t)layers.size() - 1; }
+  MutCols eval_cols() const { return MutCols(evals, (size_t)1 << eval_log); }
   const uint32_t* eval_col(uint32_t c) const { return evals + ((size_t)c << eval_log); }
 };
 

@@ -16,9 +16,11 @@ int fold_circle_into_line_fused(cudaStream_t st, CPlanes src, uint32_t log_n, qm
                                 const uint32_t* d_itw, uint32_t tw_log, uint32_t* leaf_out);
 int fold_line_dev_alpha(cudaStream_t st, CPlanes src, uint32_t log_n, const uint32_t* d_alpha, Planes dst,
                         const uint32_t* d_itw, uint32_t tw_log, uint32_t* leaf_out);
-int fold_circle_into_line_dev_alpha(cudaStream_t st, CPlanes src, uint32_t log_n, const uint32_t* d_alpha, Planes dst,
-                                    const uint32_t* d_itw, uint32_t tw_log, uint32_t* leaf_out);
-int interpolate_columns_to(cudaStream_t st, const uint32_t* const* d_src, uint32_t* const* d_dst, uint32_t n_cols,
+int fold_circle_fresh(cudaStream_t st, CPlanes src, uint32_t log_n, qm31 alpha, Planes dst, const uint32_t* d_itw,
+                      uint32_t tw_log);
+int fold_circle_fresh_dev_alpha(cudaStream_t st, CPlanes src, uint32_t log_n, const uint32_t* d_alpha, Planes dst,
+                                const uint32_t* d_itw, uint32_t tw_log, uint32_t* leaf_out);
+int interpolate_columns_to(cudaStream_t st, Cols d_src, MutCols d_dst, uint32_t n_cols,
                            uint32_t log_n, const uint32_t* d_itwiddles, uint32_t tw_log);
 
 namespace prover {
@@ -107,24 +109,14 @@ struct Prover {
     return OK;
   }
 
-  int table(const std::vector<const uint32_t*>& ptrs, const uint32_t* const** out) {
-    const void* const* d = nullptr;
-    GS_TRY(ctx.stage_ptrs((const void* const*)ptrs.data(), ptrs.size(), &d));
-    *out = (const uint32_t* const*)d;
-    return OK;
-  }
-
   int merkle(Tree& t) {
     t.layers.assign(t.eval_log + 1, nullptr);
     for (uint32_t L = 0; L <= t.eval_log; L++) GS_TRY(A.alloc_n((size_t)8 << L, &t.layers[L]));
-    std::vector<const uint32_t*> cols;
-    for (uint32_t c = 0; c < t.n_cols; c++) cols.push_back(t.eval_col(c));
-    const uint32_t* const* tab = nullptr;
-    GS_TRY(table(cols, &tab));
+    const Cols tab = t.eval_cols();
     if (ch.p252) {  // Poseidon252MerkleHasher: one launch per layer
       GS_TRY(poseidon252_commit_on_layer(st, t.eval_log, nullptr, tab, t.n_cols, (uint8_t*)t.layers[t.eval_log]));
       for (int L = (int)t.eval_log - 1; L >= 0; L--)
-        GS_TRY(poseidon252_commit_on_layer(st, (uint32_t)L, (const uint8_t*)t.layers[L + 1], nullptr, 0,
+        GS_TRY(poseidon252_commit_on_layer(st, (uint32_t)L, (const uint8_t*)t.layers[L + 1], Cols(), 0,
                                            (uint8_t*)t.layers[L]));
     } else {
       GS_TRY(commit_on_layer(st, t.eval_log, nullptr, tab, t.n_cols, t.layers[t.eval_log], true));
@@ -150,18 +142,15 @@ struct Prover {
       t.ext_log = E;
     }
     std::vector<const uint32_t*> src(t.coeff_ptrs.begin() + t.ext_done, t.coeff_ptrs.begin() + c_end);
-    std::vector<const uint32_t*> dst;
-    for (uint32_t c = t.ext_done; c < c_end; c++) dst.push_back(t.ext + ((size_t)c << E));
-    const uint32_t* const* stab = nullptr;
-    const uint32_t* const* dtab = nullptr;
-    GS_TRY(table(src, &stab));
-    GS_TRY(table(dst, &dtab));
+    Cols scols;
+    GS_TRY(ctx.columns(src.data(), src.size(), &scols));
+    const MutCols dcols(t.ext + ((size_t)t.ext_done << E), (size_t)1 << E);
     cudaStream_t s = st;
     if (on_side && ctx.side) {
       GS_TRY(ctx.fork_side());
       s = ctx.side;
     }
-    GS_TRY(evaluate_columns(s, stab, t.coeff_log, (uint32_t* const*)dtab, c_end - t.ext_done, E, tw, tw_log));
+    GS_TRY(evaluate_columns(s, scols, t.coeff_log, dcols, c_end - t.ext_done, E, tw, tw_log));
     t.ext_done = c_end;
     return OK;
   }
@@ -181,13 +170,9 @@ struct Prover {
     t.eval_log = coeff_log + cfg.log_blowup;
     t.coeff_ptrs = coeffs;
     if (early) GS_TRY(early(t));
-    GS_TRY(table(coeffs, &t.coeff_tab));
+    GS_TRY(ctx.columns(coeffs.data(), coeffs.size(), &t.coeffs));
     GS_TRY(A.alloc_n((size_t)t.n_cols << t.eval_log, &t.evals));
-    std::vector<const uint32_t*> dst;
-    for (uint32_t c = 0; c < t.n_cols; c++) dst.push_back(t.eval_col(c));
-    const uint32_t* const* dtab = nullptr;
-    GS_TRY(table(dst, &dtab));
-    GS_TRY(evaluate_columns(st, t.coeff_tab, coeff_log, (uint32_t* const*)dtab, t.n_cols, t.eval_log, tw, tw_log));
+    GS_TRY(evaluate_columns(st, t.coeffs, coeff_log, t.eval_cols(), t.n_cols, t.eval_log, tw, tw_log));
     GS_TRY(merkle(t));
     if (overlap) GS_TRY(overlap(t));
     const void* h = nullptr;
@@ -205,16 +190,10 @@ struct Prover {
                    const std::function<int(Tree&)>& early = nullptr) {
     uint32_t* coeffs = nullptr;
     GS_TRY(A.alloc_n((size_t)n_cols << log, &coeffs));
-    std::vector<const uint32_t*> src, dst;
-    for (uint32_t c = 0; c < n_cols; c++) {
-      src.push_back(evals + ((size_t)c << log));
-      dst.push_back(coeffs + ((size_t)c << log));
-    }
-    const uint32_t* const* stab = nullptr;
-    const uint32_t* const* dtab = nullptr;
-    GS_TRY(table(src, &stab));
-    GS_TRY(table(dst, &dtab));
-    GS_TRY(interpolate_columns_to(st, stab, (uint32_t* const*)dtab, n_cols, log, itw, tw_log));
+    std::vector<const uint32_t*> dst;
+    for (uint32_t c = 0; c < n_cols; c++) dst.push_back(coeffs + ((size_t)c << log));
+    const size_t n = (size_t)1 << log;
+    GS_TRY(interpolate_columns_to(st, Cols(evals, n), MutCols(coeffs, n), n_cols, log, itw, tw_log));
     return commit_coeffs(dst, log, overlap, early);
   }
 
@@ -228,14 +207,13 @@ struct Prover {
   }
 
   // What the composition needs before its random coefficient is drawn: the
-  // constraint denominators, the output planes and their pointer table.
+  // constraint denominators and the output planes.
   // Called while the last trace root is read back; composition() calls it
   // itself when nothing did.
   struct CompositionPrep {
     bool ready = false;
     ConstraintParams prm;
     uint32_t* comp[4] = {nullptr, nullptr, nullptr, nullptr};
-    const uint32_t* const* ctab = nullptr;
   } cprep;
   int prepare_composition(const AirHost& air) {
     if (cprep.ready) return OK;
@@ -253,9 +231,8 @@ struct Prover {
       dn[i] = inv(host::canonic_vanishing_m31(T, host::index_point(idx)));
     }
     for (uint32_t i = 0; i < dn.size(); i++) prm.denom_inv[host::bitrev(i, log_expand)] = dn[i];
-    for (int c = 0; c < 4; c++) GS_TRY(A.alloc_n((size_t)1 << E, &cprep.comp[c]));
-    std::vector<const uint32_t*> cp = {cprep.comp[0], cprep.comp[1], cprep.comp[2], cprep.comp[3]};
-    GS_TRY(table(cp, &cprep.ctab));
+    GS_TRY(A.alloc_n((size_t)4 << E, &cprep.comp[0]));
+    for (int c = 1; c < 4; c++) cprep.comp[c] = cprep.comp[0] + ((size_t)c << E);
     cprep.ready = true;
     return OK;
   }
@@ -291,8 +268,7 @@ struct Prover {
       GS_TRY(poseidon_constraints(st, on_domain[1], on_domain[2], E, T, prm, air.lookup, shift, out));
     }
     // finalize: interpolate the 4 coordinates on CanonicCoset(E)
-    const uint32_t* const* ctab = cprep.ctab;
-    GS_TRY(interpolate_columns(st, (uint32_t* const*)ctab, 4, E, itw, tw_log));
+    GS_TRY(interpolate_columns(st, MutCols(comp[0], (size_t)1 << E), 4, E, itw, tw_log));
     return OK;
   }
 };

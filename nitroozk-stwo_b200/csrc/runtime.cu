@@ -214,7 +214,8 @@ int Context::join_side() {
   return OK;
 }
 
-int Context::stage_bytes(const void* host, size_t len, const void** out) {
+// A slot of the ring, its host side filled.
+int Context::ring_slot(const void* host, size_t len, size_t* off) {
   size_t bytes = (len + 255) & ~(size_t)255;
   GS_REQUIRE(bytes <= ring_cap, "staged argument block too large");
   if (ring_off + bytes > ring_cap) {
@@ -226,9 +227,23 @@ int Context::stage_bytes(const void* host, size_t len, const void** out) {
     ring_off = 0;
   }
   memcpy(h_ring + ring_off, host, len);
-  GS_CUDA_TRY(cudaMemcpyAsync(d_ring + ring_off, h_ring + ring_off, len, cudaMemcpyHostToDevice, stream));
-  *out = (const void*)(d_ring + ring_off);
+  *off = ring_off;
   ring_off += bytes;
+  return OK;
+}
+
+int Context::stage_bytes(const void* host, size_t len, const void** out) {
+  size_t off = 0;
+  GS_TRY(ring_slot(host, len, &off));
+  GS_CUDA_TRY(cudaMemcpyAsync(d_ring + off, h_ring + off, len, cudaMemcpyHostToDevice, stream));
+  *out = (const void*)(d_ring + off);
+  return OK;
+}
+
+int Context::stage_to(void* dst, const void* host, size_t len) {
+  size_t off = 0;
+  GS_TRY(ring_slot(host, len, &off));
+  GS_CUDA_TRY(cudaMemcpyAsync(dst, h_ring + off, len, cudaMemcpyHostToDevice, stream));
   return OK;
 }
 
@@ -236,6 +251,29 @@ int Context::stage_ptrs(const void* const* host_ptrs, size_t n, const void* cons
   const void* d = nullptr;
   GS_TRY(stage_bytes(host_ptrs, n * sizeof(void*), &d));
   *out = (const void* const*)d;
+  return OK;
+}
+
+int Context::columns(const uint32_t* const* host_ptrs, size_t n, Cols* out) {
+  const uintptr_t step = n > 1 ? (uintptr_t)host_ptrs[1] - (uintptr_t)host_ptrs[0] : 0;  // mod 2^64: may go down
+  bool even = n > 0 && step % 4 == 0;
+  for (size_t i = 2; i < n && even; i++) even = (uintptr_t)host_ptrs[i] - (uintptr_t)host_ptrs[i - 1] == step;
+  if (even) {
+    *out = Cols(host_ptrs[0], (size_t)((intptr_t)step / 4));
+    return OK;
+  }
+  const void* const* d = nullptr;
+  GS_TRY(stage_ptrs((const void* const*)host_ptrs, n, &d));
+  *out = Cols((const uint32_t* const*)d);
+  return OK;
+}
+
+int Context::columns(uint32_t* const* host_ptrs, size_t n, MutCols* out) {
+  Cols c;
+  GS_TRY(columns((const uint32_t* const*)host_ptrs, n, &c));
+  out->tab = (uint32_t* const*)c.tab;
+  out->base = const_cast<uint32_t*>(c.base);
+  out->stride = c.stride;
   return OK;
 }
 

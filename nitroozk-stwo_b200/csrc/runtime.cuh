@@ -44,6 +44,40 @@ const char* last_error();
     if (_s != ::gs::OK) return _s;        \
   } while (0)
 
+// The columns of a call as a kernel sees them: evenly spaced from a base, by
+// value, or through a device table of pointers. Spaced columns (a tree's, a
+// matrix's rows) need no table: an upload costs the host a copy call and the
+// stream one to three microseconds before the kernel, and each block a
+// dependent load.
+struct Cols {
+  const uint32_t* const* tab = nullptr;
+  const uint32_t* base = nullptr;
+  size_t stride = 0;  // words
+  Cols() = default;
+  Cols(const uint32_t* const* t) : tab(t) {}
+  Cols(const uint32_t* b, size_t words) : base(b), stride(words) {}
+  __device__ __forceinline__ const uint32_t* operator[](uint32_t c) const {
+    return tab ? tab[c] : base + c * stride;
+  }
+  bool given() const { return tab || base; }
+};
+struct MutCols {
+  uint32_t* const* tab = nullptr;
+  uint32_t* base = nullptr;
+  size_t stride = 0;
+  MutCols() = default;
+  MutCols(uint32_t* const* t) : tab(t) {}
+  MutCols(uint32_t* b, size_t words) : base(b), stride(words) {}
+  operator Cols() const {
+    Cols c;
+    c.tab = (const uint32_t* const*)tab;
+    c.base = base;
+    c.stride = stride;
+    return c;
+  }
+  __device__ __forceinline__ uint32_t* operator[](uint32_t c) const { return tab ? tab[c] : base + c * stride; }
+};
+
 // A QM31 column as 4 coordinate planes, passed by value to kernels.
 struct Planes { uint32_t* p[4]; };
 struct CPlanes { const uint32_t* p[4]; };
@@ -178,6 +212,7 @@ struct Context {
   DomainTables dom[31];
 
   int init(void* user_stream);
+  int ring_slot(const void* host, size_t len, size_t* off);
   int stage_bytes(const void* host, size_t bytes, const void** out);
   int get_scratch(size_t bytes, void** out);
   int domain_tables(uint32_t lift, DomainTables* out);
@@ -186,6 +221,11 @@ struct Context {
   uint32_t* itw_buf[31] = {nullptr};
   int twiddles(uint32_t root_log, const uint32_t** tw, const uint32_t** itw);
   void destroy();
+  // The columns of a host list: spaced evenly, or staged as a table.
+  int columns(const uint32_t* const* host_ptrs, size_t n, Cols* out);
+  int columns(uint32_t* const* host_ptrs, size_t n, MutCols* out);
+  // One host-to-device copy, through the staging ring, to a place of the caller's.
+  int stage_to(void* dst, const void* host, size_t len);
   // Copies `n` host pointers into device memory usable by kernels launched on
   // `stream` after this call; returns the device address.
   int stage_ptrs(const void* const* host_ptrs, size_t n, const void* const** out);
@@ -201,7 +241,7 @@ int precompute_twiddles(cudaStream_t st, uint32_t initial_index, uint32_t step_i
 int batch_inverse(cudaStream_t st, const uint32_t* d_in, uint32_t* d_out, size_t n);
 
 // fft.cu (columns given by a device table of pointers)
-int interpolate_columns(cudaStream_t st, uint32_t* const* d_cols, uint32_t n_cols, uint32_t log_n,
+int interpolate_columns(cudaStream_t st, MutCols cols, uint32_t n_cols, uint32_t log_n,
                         const uint32_t* d_itwiddles, uint32_t tw_log);
 // One FFT of a work-list: interpolate (inverse != 0) 2^log evaluations, or
 // evaluate 2^coeff_log coefficients on the domain of 2^log; src and dst are
@@ -219,7 +259,7 @@ constexpr uint32_t FFT_WL_MIN_LOG = 3, FFT_WL_MAX_LOG = 13;
 // those (tw_log + 1 >= every log).
 int fft_worklist(Context& ctx, const FftItem* items, uint32_t n_items, const uint32_t* d_twiddles,
                  const uint32_t* d_itwiddles, uint32_t tw_log);
-int evaluate_columns(cudaStream_t st, const uint32_t* const* d_src, uint32_t coeff_log, uint32_t* const* d_dst,
+int evaluate_columns(cudaStream_t st, Cols src, uint32_t coeff_log, MutCols dst,
                      uint32_t n_cols, uint32_t log_n, const uint32_t* d_twiddles, uint32_t tw_log);
 int bit_reverse(cudaStream_t st, uint32_t* d, uint32_t log_n);
 // Pass-split tuning per number of computed layers and extension (domain log
@@ -230,8 +270,8 @@ int fft_autotune(cudaStream_t st, uint32_t lo, uint32_t hi, uint32_t max_ext, co
                  uint32_t tw_log, uint32_t* out_tile, uint32_t* out_coalesce);
 
 // merkle.cu
-// cols_aligned: every column pointer of the table is 16-byte aligned.
-int commit_on_layer(cudaStream_t st, uint32_t log_size, const uint32_t* d_prev, const uint32_t* const* d_cols,
+// cols_aligned: every column is 16-byte aligned.
+int commit_on_layer(cudaStream_t st, uint32_t log_size, const uint32_t* d_prev, Cols cols,
                     uint32_t n_cols, uint32_t* d_out, bool cols_aligned = false);
 // All node-only layers below `top_log` (layers[L] has 2^L hashes, layers[top_log] given),
 // in one launch up to TREE_MAX_LOG. d_counters: TREE_COUNTERS zeroed words
@@ -271,7 +311,7 @@ int lifted_leaves(cudaStream_t st, uint32_t lift, const uint32_t* const* d_cols,
 // poseidon252.cu: Poseidon252 Merkle layers and permutations; hashes are
 // felt252 values as 32 big-endian bytes.
 int poseidon252_commit_on_layer(cudaStream_t st, uint32_t log_size, const uint8_t* d_prev,
-                                const uint32_t* const* d_cols, uint32_t n_cols, uint8_t* d_out);
+                                Cols cols, uint32_t n_cols, uint8_t* d_out);
 int poseidon252_permute(cudaStream_t st, const uint8_t* d_in, uint32_t n, uint8_t* d_out);
 // d_scratch: 48 bytes of device memory; h_word: 8 bytes of pinned host memory.
 // digest_is_prefixed: d_digest already holds poseidon_hash_many([POW_PREFIX,
@@ -343,7 +383,7 @@ int quot_line_coeffs(cudaStream_t st, const LineTerm* d_terms, uint32_t n_terms,
 
 // eval_at_point.cu
 size_t eval_at_point_scratch_bytes(uint32_t n_polys, uint32_t log_n, uint32_t chunk_log = 12);
-int batch_eval_at_point(cudaStream_t st, const uint32_t* const* d_polys, uint32_t n_polys, uint32_t log_n, ptq point,
+int batch_eval_at_point(cudaStream_t st, Cols polys, uint32_t n_polys, uint32_t log_n, ptq point,
                         uint32_t* d_out, uint32_t* d_scratch, uint32_t chunk_log = 12, bool vec = false);
 
 // barycentric weights on CanonicCoset(dt.lift) (4 planes) and evaluation

@@ -1,7 +1,7 @@
 // Device-side Fiat-Shamir step of the Blake2s channel (Blake2sChannel::
 // mix_root followed by draw_secure_felt, crates/stwo/src/core/channel/
 // blake2s.rs), shared by the stand-alone channel kernel and the fused FRI
-// tail kernel. Run by one thread.
+// tail kernel. Run by one warp, four lanes per compression.
 //
 //   mix_root:    digest <- Blake2s(digest || root), n_draws <- 0
 //   draw_u32s:   Blake2s(digest || n_draws (LE u32) || 0x00), n_draws += 1
@@ -16,58 +16,59 @@
 
 namespace gs {
 
-// The step is two compressions whose messages lie in shared memory, so that a
-// kernel runs them through the same compression its tree levels use (one copy
-// of the unrolled rounds stays in the instruction cache; a lone warp that runs
-// into another copy waits for its instructions).
+// One warp runs the step with four lanes per compression (blake2s_quad); its
+// messages lie in shared memory.
 struct ChannelWords {
   uint4 mix[4];   // digest, root
   uint4 draw[4];  // digest, draws so far, zeros
+  uint4 felt;     // the challenge
 };
 constexpr uint32_t CHANNEL_MIX_BYTES = 64, CHANNEL_DRAW_BYTES = 37;
 
-__device__ __forceinline__ void channel_begin(ChannelWords& w, const uint32_t* state) {  // one thread
-  w.mix[0] = make_uint4(state[0], state[1], state[2], state[3]);
-  w.mix[1] = make_uint4(state[4], state[5], state[6], state[7]);
-  w.draw[3] = make_uint4(0, 0, 0, 0);
+// Warp 0, before the root is known.
+__device__ __forceinline__ void channel_begin(ChannelWords& w, const uint32_t* state) {
+  const uint32_t lane = threadIdx.x;
+  if (lane < 8) reinterpret_cast<uint32_t*>(w.mix)[lane] = state[lane];
+  if (lane < 8) reinterpret_cast<uint32_t*>(w.draw)[8 + lane] = 0;
 }
-__device__ __forceinline__ void channel_root(ChannelWords& w, const uint32_t h[8]) {  // one thread
-  w.mix[2] = make_uint4(h[0], h[1], h[2], h[3]);
-  w.mix[3] = make_uint4(h[4], h[5], h[6], h[7]);
+// Words j and 4 + j of the root, from lanes j < 4 of warp 0.
+__device__ __forceinline__ void channel_root(ChannelWords& w, uint32_t j, uint32_t h0, uint32_t h1) {
+  uint32_t* m = reinterpret_cast<uint32_t*>(w.mix);
+  m[8 + j] = h0;
+  m[12 + j] = h1;
 }
-// h: the hash of the mix message, the new digest (one thread).
-__device__ __forceinline__ void channel_mixed(ChannelWords& w, const uint32_t h[8], uint32_t* state) {
-  w.mix[0] = w.draw[0] = make_uint4(h[0], h[1], h[2], h[3]);
-  w.mix[1] = w.draw[1] = make_uint4(h[4], h[5], h[6], h[7]);
-  w.draw[2] = make_uint4(0, 0, 0, 0);
-#pragma unroll
-  for (int j = 0; j < 8; j++) state[j] = h[j];
+// The hash of the mix message, the new digest (lanes j < 4).
+__device__ __forceinline__ void channel_mixed(ChannelWords& w, uint32_t j, uint32_t h0, uint32_t h1, uint32_t* state) {
+  uint32_t *m = reinterpret_cast<uint32_t*>(w.mix), *d = reinterpret_cast<uint32_t*>(w.draw);
+  m[j] = d[j] = state[j] = h0;
+  m[4 + j] = d[4 + j] = state[4 + j] = h1;
+  if (j == 0) d[8] = 0;
 }
-// h: the hash of the draw message after `draws` earlier ones. The same answer
-// in every thread that holds h: true when the draw is done (the felt taken, or
-// given up), false when it goes on with draws + 1; `one_thread` stores. A draw
+// The hash of the draw message after `draws` earlier ones, in every quad of
+// warp 0: true when the draw is done (the felt taken, in w.felt and felt_out
+// with its square, or given up), false when it goes on with draws + 1. A draw
 // is rejected with probability < 2^-27; 64 rejections in a row do not happen
 // for a hash, and running out is reported, never looped on.
-__device__ __forceinline__ bool channel_drawn(ChannelWords& w, const uint32_t h[8], uint32_t draws, bool one_thread,
-                                              uint32_t* state, uint32_t* felt_out, qm31& a) {
-  bool ok = true;
-#pragma unroll
-  for (int j = 0; j < 8; j++) ok = ok && h[j] < 2u * P;
+__device__ __forceinline__ bool channel_drawn(ChannelWords& w, uint32_t h0, uint32_t h1, uint32_t draws,
+                                              uint32_t* state, uint32_t* felt_out) {
+  const uint32_t lane = threadIdx.x;
+  const bool ok = __all_sync(0xffffffffu, h0 < 2u * P && h1 < 2u * P);
   if (!ok && draws + 1 < 64) {
-    if (one_thread) w.draw[2].x = draws + 1;
+    if (lane == 0) w.draw[2].x = draws + 1;
+    __syncwarp();
     return false;
   }
-  a = qm_make(h[0] >= P ? h[0] - P : h[0], h[1] >= P ? h[1] - P : h[1], h[2] >= P ? h[2] - P : h[2],
-              h[3] >= P ? h[3] - P : h[3]);
-  if (one_thread) {
-    if (ok) {  // the challenge, then its square
-      const qm31 a2 = qm_mul(a, a);
+  if (lane < 4) reinterpret_cast<uint32_t*>(&w.felt)[lane] = h0 >= P ? h0 - P : h0;
+  __syncwarp();
+  if (lane == 0) {
+    state[8] = draws + 1;
+    if (ok) {
+      const qm31 a = qm_make(w.felt.x, w.felt.y, w.felt.z, w.felt.w), a2 = qm_mul(a, a);
       felt_out[0] = a.x.a; felt_out[1] = a.x.b; felt_out[2] = a.y.a; felt_out[3] = a.y.b;
       felt_out[4] = a2.x.a; felt_out[5] = a2.x.b; felt_out[6] = a2.y.a; felt_out[7] = a2.y.b;
     } else {
       state[9] = 1;
     }
-    state[8] = draws + 1;
   }
   return true;
 }

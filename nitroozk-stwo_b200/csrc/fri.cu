@@ -174,112 +174,130 @@ int fold_circle_fresh_dev_alpha(cudaStream_t st, CPlanes src, uint32_t log_n, co
 
 // Fused tail of the FRI commit phase: every layer of log size <= 11 in one
 // launch of one 1024-thread CTA. For layer k (log size log0 - k, leaves
-// already hashed): its Merkle node levels (at most 1024 nodes each, one per
-// thread), the channel step on its root (one thread), then fold_line into
-// layer k + 1 with that layer's leaf hashes — the steps the per-layer kernels
-// run, with the data in shared memory and `__syncthreads` between them. The
-// tail is a chain of about a hundred dependent steps, most of them one
-// Blake2s compression long; an earlier 8-CTA cluster version spent more on
-// cluster barriers and L2 re-reads than it gained in width (164 µs against
-// 132 µs for the Poseidon2 2^18 proof's tail).
-// Shared memory (uint4): two node-hash buffers of 1024 hashes, the current
-// layer's leaves (1024 hashes), the current and next layer values (1024
-// QM31 each): 128 KiB.
-constexpr uint32_t TAIL_CTA_SMEM = 8192 * 16;
+// already hashed): its Merkle node levels (at most 1024 nodes each), the
+// channel step on its root, then fold_line into layer k + 1 with that layer's
+// leaf hashes — the steps the per-layer kernels run, with the data in shared
+// memory and block barriers between them. The tail is a chain of about a
+// hundred dependent steps, most of them one Blake2s compression long, so the
+// latency of a compression bounds it: levels (and leaf layers) of at most 32
+// hashes and the channel step take four lanes per compression (blake2s_quad),
+// on warps 0..3 down to warp 0 alone; larger ones a thread each. The tail of a
+// 2^16 or larger first layer: 144 -> 124 us, of a 2^11 one 112 -> 94 us. An
+// 8-CTA cluster spent more on cluster barriers and L2 re-reads than it gained
+// in width (164 against 132 us, a thread per hash in both).
+// Shared memory (uint4): two hash buffers (2048: a layer's leaves, then its
+// levels in turn), this layer's and the next one's values (1024 QM31 each) and
+// 32 leaf messages.
+constexpr uint32_t TAIL_CTA_SMEM = (2 * 2048 + 2 * 1024 + 32 * 4) * 16;
+__device__ __forceinline__ void bar_sync_128() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 __global__ void __launch_bounds__(1024) fri_tail_cta_kernel(FriTail a, uint32_t* state,
                                                             const uint32_t* __restrict__ itw, uint32_t tw_len,
                                                             uint32_t one) {
   extern __shared__ uint4 tsm[];
   __shared__ ChannelWords ch;
-  __shared__ uint4 alpha_s;
-  uint4* const leaves = tsm + 4096;
-  auto nb = [&](int i) { return tsm + 2048 * i; };              // two node-hash buffers
-  auto vals = [&](uint32_t i) { return tsm + 6144 + 1024 * i; };  // this layer's and the next one's values
-  const uint32_t tid = threadIdx.x;
-  if (tid == 0) channel_begin(ch, state);  // read by warp 0 after a root
-  for (uint32_t k = 0; k < a.n; k++) {
-    const uint32_t log = a.log0 - k, half = 1u << (log - 1);
+  __shared__ uint32_t quad_tab[40];
+  auto hashes = [&](int i) { return tsm + 2048 * i; };
+  auto vals = [&](uint32_t i) { return tsm + 4096 + 1024 * i; };
+  uint4* const msgs = tsm + 6144;
+  const uint32_t tid = threadIdx.x, j = tid & 3u;
+  blake2s_quad_table(quad_tab);
+  if (tid < 32) {
+    channel_begin(ch, state);  // read by warp 0 after a root
+    for (int q = 0; q < 4; q++) msgs[4 * tid + q] = make_uint4(0, 0, 0, 0);
+  }
+  for (uint32_t k = 0; k <= a.n; k++) {
+    const uint32_t log = a.log0 - k;
     uint32_t* const* tree = a.tree[k];
-    int cur = 0;
-    uint32_t draws = 0;
-    // s >= 0: the 2^s nodes of level s, one per thread; -1, -2: the channel's
-    // mix and draw; -3: the fold and the next layer's leaves. One compression
-    // serves all of them. Levels of at most 32 nodes and the channel are warp
-    // 0's alone, without block barriers; its lanes past the level's nodes
-    // hash words nobody uses.
-    for (int s = (int)log - 1; s >= -3;) {
-      const bool lone = s <= 5 && s > -3;
-      const uint32_t n = s >= 0 ? 1u << s : s == -3 ? half : 1u;
-      if (lone ? tid < 32 : tid < n) {
+    uint4 v;  // this thread's value of the layer
+    if (k > 0 && tid < (1u << log)) {  // the fold of the layer before
+      qm31 fx, fnx;
+      if (k == 1) {  // layer 0's values come from the previous kernel
+        uint32_t* const* sp = a.planes[0];
+        fx = qm_make(__ldg(sp[0] + 2 * tid), __ldg(sp[1] + 2 * tid), __ldg(sp[2] + 2 * tid), __ldg(sp[3] + 2 * tid));
+        fnx = qm_make(__ldg(sp[0] + 2 * tid + 1), __ldg(sp[1] + 2 * tid + 1), __ldg(sp[2] + 2 * tid + 1),
+                      __ldg(sp[3] + 2 * tid + 1));
+      } else {
+        const uint4 p = vals((k - 1) & 1)[2 * tid], q = vals((k - 1) & 1)[2 * tid + 1];
+        fx = qm_make(p.x, p.y, p.z, p.w);
+        fnx = qm_make(q.x, q.y, q.z, q.w);
+      }
+      const qm31 alpha = qm_make(ch.felt.x, ch.felt.y, ch.felt.z, ch.felt.w);
+      const uint32_t xinv = __ldg(itw + (tw_len - (2u << log)) + tid);
+      const qm31 f0 = qm_add(fx, fnx);
+      const qm31 f1 = qm_mul_m31(qm_sub(fx, fnx), xinv);
+      const qm31 r = qm_add(f0, qm_mul(alpha, f1));
+      uint32_t* const* dp = a.planes[k];
+      dp[0][tid] = r.x.a; dp[1][tid] = r.x.b; dp[2][tid] = r.y.a; dp[3][tid] = r.y.b;
+      v = make_uint4(r.x.a, r.x.b, r.y.a, r.y.b);
+      vals(k & 1)[tid] = v;
+      if (log <= 5) msgs[4 * tid] = v;
+    }
+    if (k == a.n) return;  // the last layer is not committed
+    // s = log: the leaves (layer 0's were hashed by the previous kernel); s <
+    // log: the 2^s nodes of level s, one thread each while there are more than 32
+    int s = k == 0 ? (int)log - 1 : (int)log, cur = 0;
+    for (; s > 5; s--) {
+      if (tid < (1u << s)) {
         uint4 c[4];
-        if (s == -3) {
-          qm31 fx, fnx;
-          if (k == 0) {  // layer 0's values come from the previous kernel
-            uint32_t* const* sp = a.planes[0];
-            fx = qm_make(__ldg(sp[0] + 2 * tid), __ldg(sp[1] + 2 * tid), __ldg(sp[2] + 2 * tid),
-                         __ldg(sp[3] + 2 * tid));
-            fnx = qm_make(__ldg(sp[0] + 2 * tid + 1), __ldg(sp[1] + 2 * tid + 1), __ldg(sp[2] + 2 * tid + 1),
-                          __ldg(sp[3] + 2 * tid + 1));
-          } else {
-            const uint4 u = vals(k & 1)[2 * tid], v = vals(k & 1)[2 * tid + 1];
-            fx = qm_make(u.x, u.y, u.z, u.w);
-            fnx = qm_make(v.x, v.y, v.z, v.w);
-          }
-          const qm31 alpha = qm_make(alpha_s.x, alpha_s.y, alpha_s.z, alpha_s.w);
-          const uint32_t xinv = __ldg(itw + (tw_len - (1u << log)) + tid);
-          const qm31 f0 = qm_add(fx, fnx);
-          const qm31 f1 = qm_mul_m31(qm_sub(fx, fnx), xinv);
-          const qm31 r = qm_add(f0, qm_mul(alpha, f1));
-          uint32_t* const* dp = a.planes[k + 1];
-          dp[0][tid] = r.x.a; dp[1][tid] = r.x.b; dp[2][tid] = r.y.a; dp[3][tid] = r.y.b;
-          c[0] = make_uint4(r.x.a, r.x.b, r.y.a, r.y.b);
+        if (s == (int)log) {
+          c[0] = v;
           c[1] = c[2] = c[3] = make_uint4(0, 0, 0, 0);
-          vals((k + 1) & 1)[tid] = c[0];
-        } else if (s == (int)log - 1 && k == 0) {  // leaves hashed by the previous kernel
-          const uint4* src = reinterpret_cast<const uint4*>(tree[log]) + 4 * (size_t)(tid < n ? tid : 0);
+        } else if (s == (int)log - 1 && k == 0) {
+          const uint4* src = reinterpret_cast<const uint4*>(tree[log]) + 4 * (size_t)tid;
 #pragma unroll
           for (int q = 0; q < 4; q++) c[q] = __ldg(src + q);
         } else {
-          const uint4* src = s >= 0 ? (s == (int)log - 1 ? leaves : nb(cur ^ 1)) + 4 * tid : s == -1 ? ch.mix : ch.draw;
 #pragma unroll
-          for (int q = 0; q < 4; q++) c[q] = src[q];
+          for (int q = 0; q < 4; q++) c[q] = hashes(cur ^ 1)[4 * tid + q];
         }
-        if (s > -3 || k + 1 < a.n) {  // (the last layer has no leaves)
-          uint32_t h[8];
-          hash_block16(c, s == -2 ? CHANNEL_DRAW_BYTES : s == -3 ? 16u : 64u, h, one);
-          if ((s >= 0 || s == -3) && tid < n) {
-            tail_store_hash(s >= 0 ? tree[s] : a.tree[k + 1][log - 1], tid, h);
-            uint4* to = s >= 0 ? nb(cur) : leaves;
-            to[2 * tid] = make_uint4(h[0], h[1], h[2], h[3]);
-            to[2 * tid + 1] = make_uint4(h[4], h[5], h[6], h[7]);
-          }
-          if (s <= 0 && s > -3) {
-            if (s == 0 && tid == 0) {
-#pragma unroll
-              for (int j = 0; j < 8; j++) a.roots[8 * k + j] = h[j];
-              channel_root(ch, h);
-            }
-            if (s == -1 && tid == 0) channel_mixed(ch, h, state);
-            if (s == -2) {
-              qm31 felt;
-              if (!channel_drawn(ch, h, draws, tid == 0, state, a.felts + 8 * k, felt)) {
-                draws++;
-                __syncwarp();
-                continue;
-              }
-              if (tid == 0) alpha_s = make_uint4(felt.x.a, felt.x.b, felt.y.a, felt.y.b);
-            }
-          }
-        }
+        uint32_t h[8];
+        hash_block16(c, s == (int)log ? 16u : 64u, h, one);
+        tail_store_hash(tree[s], tid, h);
+        hashes(cur)[2 * tid] = make_uint4(h[0], h[1], h[2], h[3]);
+        hashes(cur)[2 * tid + 1] = make_uint4(h[4], h[5], h[6], h[7]);
       }
-      if (lone && s != -2) {  // warp 0 goes on; the others wait for the challenge
-        if (tid < 32) __syncwarp();
-      } else {
-        __syncthreads();
-      }
+      __syncthreads();
       cur ^= 1;
-      s--;
     }
+    if (tid < 128) {
+      if (k == 0 && log <= 6) {  // a small first layer: its leaves
+        const uint4* src = reinterpret_cast<const uint4*>(tree[log]);
+        for (uint32_t i = tid; i < (2u << log); i += 128) hashes(cur ^ 1)[i] = __ldg(src + i);
+      }
+      bar_sync_128();  // the leaves or messages of the other warps
+      uint32_t draws = 0;
+      while (s >= -2) {
+        if (s <= 3 && tid >= 32) break;
+        const uint32_t n = s >= 0 ? 1u << s : 1u, i = tid >> 2;
+        if (tid < (4 * n > 32 ? 4 * n : 32)) {
+          const bool leaf = s == (int)log;
+          uint32_t h0, h1;
+          blake2s_quad(quad_tab, s >= 0 ? (leaf ? msgs : hashes(cur ^ 1)) + 4 * i : s == -1 ? ch.mix : ch.draw,
+                       leaf ? 16u : s == -2 ? CHANNEL_DRAW_BYTES : 64u, h0, h1);
+          if (s >= 0 && i < n) {
+            uint32_t* to = tree[s] + 8 * (size_t)i;
+            uint32_t* sh = reinterpret_cast<uint32_t*>(hashes(cur) + 2 * i);
+            to[j] = sh[j] = h0;
+            to[4 + j] = sh[4 + j] = h1;
+          }
+          if (s == 0 && tid < 4) {
+            a.roots[8 * k + j] = h0;
+            a.roots[8 * k + 4 + j] = h1;
+            channel_root(ch, j, h0, h1);
+          }
+          if (s == -1 && tid < 4) channel_mixed(ch, j, h0, h1, state);
+          if (s == -2 && !channel_drawn(ch, h0, h1, draws, state, a.felts + 8 * k)) {
+            draws++;
+            continue;
+          }
+        }
+        if (s > 3) bar_sync_128();
+        else __syncwarp();
+        cur ^= 1;
+        s--;
+      }
+    }
+    __syncthreads();  // the challenge
   }
 }
 

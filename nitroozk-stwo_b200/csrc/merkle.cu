@@ -239,21 +239,26 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(1024) merkle_tail_ke
   cg::cluster_group cluster = cg::this_cluster();
   cluster_tree_levels(top, layers.p, false, buf, cluster, one);
   __shared__ ChannelWords ch;
-  if (state && cluster.block_rank() == 0 && threadIdx.x == 0) {
-    uint32_t h[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) h[j] = layers.p[0][j];
-    if (root_copy)
-#pragma unroll
-      for (int j = 0; j < 8; j++) root_copy[j] = h[j];
+  __shared__ uint32_t quad_tab[40];
+  if (state && cluster.block_rank() == 0 && threadIdx.x < 32) {
+    const uint32_t j = threadIdx.x & 3u;
+    blake2s_quad_table(quad_tab);
     channel_begin(ch, state);
-    channel_root(ch, h);
-    hash_block16(ch.mix, CHANNEL_MIX_BYTES, h, one);
-    channel_mixed(ch, h, state);
-    qm31 a;
+    uint32_t h0 = layers.p[0][j], h1 = layers.p[0][4 + j];
+    if (threadIdx.x < 4) {
+      if (root_copy) {
+        root_copy[j] = h0;
+        root_copy[4 + j] = h1;
+      }
+      channel_root(ch, j, h0, h1);
+    }
+    __syncwarp();
+    blake2s_quad(quad_tab, ch.mix, CHANNEL_MIX_BYTES, h0, h1);
+    if (threadIdx.x < 4) channel_mixed(ch, j, h0, h1, state);
+    __syncwarp();
     uint32_t draws = 0;
-    do hash_block16(ch.draw, CHANNEL_DRAW_BYTES, h, one);
-    while (!channel_drawn(ch, h, draws++, true, state, felt, a));
+    do blake2s_quad(quad_tab, ch.draw, CHANNEL_DRAW_BYTES, h0, h1);
+    while (!channel_drawn(ch, h0, h1, draws++, state, felt));
   }
 }
 
@@ -266,8 +271,10 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(1024) merkle_tail_ke
 // last from a ticket (atomicInc after __threadfence, the counter wrapping
 // back to 0 for the next launch). No block waits for another, so there is no
 // spinning and nothing to bound. The block that writes the root runs the
-// optional channel step. Critical path: one compression per level, against
-// one launch per level before.
+// optional channel step. Critical path: one compression per level, four
+// lanes to each where a level has at most 32 nodes (blake2s_quad): the trees of
+// a 2^16 Wide-Fibonacci proof 24.6 -> 22.7 us each, a 2^20-leaf tree 94 -> 76
+// us (its units are cheaper too: the upper levels of a unit leave warps idle).
 struct TreePtrs { uint32_t* p[TREE_MAX_LOG + 1]; };
 // Threads per 512-child unit: 128, each hashing two nodes of the unit's first
 // level (452 us of tree kernels per Poseidon2 2^18 proof, against 464 us
@@ -279,66 +286,83 @@ template <int U, int TH>
 __global__ void __launch_bounds__(TH, TH >= 256 ? 4 : 8)
     merkle_tree_kernel(uint32_t top, TreePtrs layers, uint32_t* counters, uint32_t* state, uint32_t* root_copy,
                        uint32_t* felt, uint32_t one) {
+  static_assert(TH >= 128, "four lanes for each of 32 nodes");
   __shared__ uint4 buf[2][1 << U];
   __shared__ ChannelWords ch;
-  __shared__ uint32_t last;
-  const uint32_t tid = threadIdx.x;
+  __shared__ uint32_t last, quad_tab[40];
+  const uint32_t tid = threadIdx.x, j = tid & 3u;
+  blake2s_quad_table(quad_tab);
   uint32_t in_log = top;
   uint32_t u = blockIdx.x;
   uint32_t cnt_off = 0;
   for (;;) {
     const int out_log = in_log > U ? (int)in_log - U : 0;
     const bool channel = out_log == 0 && state;
-    if (channel && tid == 0) channel_begin(ch, state);  // read by warp 0 after the root
-    int cur = 0;
-    uint32_t draws = 0;
-    // rel >= 0: the unit's 2^rel nodes of level out_log + rel; then the
-    // channel's mix (-1) and draw (-2). One compression serves all of them.
-    // Levels of at most 32 nodes and the channel are warp 0's alone, without
-    // block barriers; lanes past the level's nodes hash words nobody uses.
-    for (int rel = (int)in_log - 1 - out_log; rel >= (channel ? -2 : 0);) {
-      if (rel <= 5 && tid >= 32) break;
-      const uint32_t n = rel >= 0 ? 1u << rel : 1u;
-      const bool first = rel >= 0 && out_log + rel + 1 == (int)in_log;
-      uint32_t h[8];
+    if (channel && tid < 32) channel_begin(ch, state);  // read by warp 0 after the root
+    int cur = 0, rel = (int)in_log - 1 - out_log;  // the unit's 2^rel nodes of level out_log + rel
+    bool first = true;                             // its children: the input layer
+    for (; rel > 5; rel--) {
+      const uint32_t n = 1u << rel;
 #pragma unroll 1
-      for (uint32_t i = tid; i < n || (rel <= 5 && i < 32); i += TH) {
+      for (uint32_t i = tid; i < n; i += TH) {
         uint4 c[4];
         if (first) {
           // written before the launch, or by other blocks of this launch:
           // read at L2, not through the non-coherent path
-          const size_t node = ((size_t)u << rel) + (i < n ? i : 0);
-          const uint4* src = reinterpret_cast<const uint4*>(layers.p[in_log]) + 4 * node;
+          const uint4* src = reinterpret_cast<const uint4*>(layers.p[in_log]) + 4 * (((size_t)u << rel) + i);
 #pragma unroll
           for (int q = 0; q < 4; q++) c[q] = __ldcg(src + q);
         } else {
-          const uint4* src = rel >= 0 ? buf[cur ^ 1] + 4 * i : rel == -1 ? ch.mix : ch.draw;
 #pragma unroll
-          for (int q = 0; q < 4; q++) c[q] = src[q];
+          for (int q = 0; q < 4; q++) c[q] = buf[cur ^ 1][4 * i + q];
         }
-        hash_block16(c, rel == -2 ? CHANNEL_DRAW_BYTES : 64u, h, one);
-        if (rel >= 0 && i < n) {
-          tail_store_hash(layers.p[out_log + rel], ((size_t)u << rel) + i, h);
-          buf[cur][2 * i] = make_uint4(h[0], h[1], h[2], h[3]);
-          buf[cur][2 * i + 1] = make_uint4(h[4], h[5], h[6], h[7]);
-        }
+        uint32_t h[8];
+        hash_block16(c, 64, h, one);
+        tail_store_hash(layers.p[out_log + rel], ((size_t)u << rel) + i, h);
+        buf[cur][2 * i] = make_uint4(h[0], h[1], h[2], h[3]);
+        buf[cur][2 * i + 1] = make_uint4(h[4], h[5], h[6], h[7]);
       }
-      if (out_log == 0 && rel <= 0) {  // the root, then the channel: warp 0
-        if (rel == 0 && tid == 0) {
-          if (root_copy)
-#pragma unroll
-            for (int j = 0; j < 8; j++) root_copy[j] = h[j];
-          if (channel) channel_root(ch, h);
+      __syncthreads();
+      cur ^= 1;
+      first = false;
+    }
+    if (first) {  // a unit of at most 64 children
+      const uint4* src = reinterpret_cast<const uint4*>(layers.p[in_log]) + 4 * ((size_t)u << rel);
+      for (uint32_t i = tid; i < (4u << rel); i += TH) buf[cur ^ 1][i] = __ldcg(src + i);
+      __syncthreads();
+    }
+    // Levels of at most 32 nodes, then the channel's mix (-1) and draw (-2):
+    // latency alone counts, so four lanes take each compression; from 8 nodes
+    // on warp 0 goes on alone, without block barriers. Quads past the level's
+    // nodes hash words nobody uses.
+    uint32_t draws = 0;
+    while (rel >= (channel ? -2 : 0)) {
+      if (rel <= 3 && tid >= 32) break;
+      const uint32_t n = rel >= 0 ? 1u << rel : 1u, i = tid >> 2;
+      if (tid < (4 * n > 32 ? 4 * n : 32)) {
+        uint32_t h0, h1;
+        blake2s_quad(quad_tab, rel >= 0 ? buf[cur ^ 1] + 4 * i : rel == -1 ? ch.mix : ch.draw,
+                     rel == -2 ? CHANNEL_DRAW_BYTES : CHANNEL_MIX_BYTES, h0, h1);
+        if (rel >= 0 && i < n) {
+          uint32_t* to = layers.p[out_log + rel] + 8 * (((size_t)u << rel) + i);
+          uint32_t* s = reinterpret_cast<uint32_t*>(buf[cur] + 2 * i);
+          to[j] = s[j] = h0;
+          to[4 + j] = s[4 + j] = h1;
         }
-        if (rel == -1 && tid == 0) channel_mixed(ch, h, state);
-        qm31 a;
-        if (rel == -2 && !channel_drawn(ch, h, draws, tid == 0, state, felt, a)) {
+        if (rel == 0 && out_log == 0 && tid < 4) {
+          if (root_copy) {
+            root_copy[j] = h0;
+            root_copy[4 + j] = h1;
+          }
+          if (channel) channel_root(ch, j, h0, h1);
+        }
+        if (rel == -1 && tid < 4) channel_mixed(ch, j, h0, h1, state);
+        if (rel == -2 && !channel_drawn(ch, h0, h1, draws, state, felt)) {
           draws++;
-          __syncwarp();
           continue;
         }
       }
-      if (rel > 5) __syncthreads();
+      if (rel > 3) __syncthreads();
       else __syncwarp();
       cur ^= 1;
       rel--;
@@ -347,7 +371,7 @@ __global__ void __launch_bounds__(TH, TH >= 256 ? 4 : 8)
     const uint32_t group_log = out_log > U ? (uint32_t)U : (uint32_t)out_log;
     const uint32_t next_u = u >> group_log;
     if (tid == 0) {
-      __threadfence();  // this unit's root (written by thread 0) before the ticket
+      __threadfence();  // this unit's root (written by lanes 0..3 of this warp) before the ticket
       const uint32_t ticket = atomicInc(counters + cnt_off + next_u, (1u << group_log) - 1u);
       last = ticket == (1u << group_log) - 1u;
     }

@@ -202,8 +202,7 @@ __device__ __forceinline__ void add_columns(uint32_t T[16], const uint32_t e[16]
 }
 
 // T = a·b + (k·p·2^64 + p)·2^192. a, b < 2^255 with a·b < 2^510.
-template <uint32_t K>
-__device__ __forceinline__ void mul_wide8(const Felt& a, const Felt& b, uint32_t T[16]) {
+__device__ __forceinline__ void mul_wide8(uint32_t K, const Felt& a, const Felt& b, uint32_t T[16]) {
   uint32_t e[16], o[16];
 #pragma unroll
   for (int j = 0; j < 4; j++) {
@@ -347,25 +346,23 @@ __device__ __forceinline__ Felt redc(const uint32_t T[16]) {
 
 // a·b / 2^256 mod p: at least (K - 1)·p, below a·b / 2^256 + (K + 1/1000)·p.
 // The top limb of a stays below 2^31.
-template <uint32_t K>
-__device__ __forceinline__ Felt fmul_k(const Felt& a, const Felt& b) {
+__device__ __forceinline__ Felt fmul_k(uint32_t K, const Felt& a, const Felt& b) {
   uint32_t T[16];
-  mul_wide8<K>(a, b, T);
+  mul_wide8(K, a, b, T);
   return redc(T);
 }
 // Below p, for a·b < 0.9·2^256·p (the product is then below 2p).
 __device__ __forceinline__ Felt fmul(const Felt& a, const Felt& b) {
-  Felt r = fmul_k<1>(a, b);
+  Felt r = fmul_k(1, a, b);
   reduce_once(r.v);
   return r;
 }
 // x^3: at least (K - 1)·p. For x <= 11p (below 2^254.5) the square is below
 // (121/32 + 2 + 1/1000)·p < 5.8p and the cube below (5.8·11/32 + K)·p < (K + 2)·p.
-template <uint32_t K>
-__device__ __forceinline__ Felt fcube(const Felt& x) {
+__device__ __forceinline__ Felt fcube(uint32_t K, const Felt& x) {
   uint32_t T[16];
   sqr_wide8(x, T);
-  return fmul_k<K>(x, redc(T));
+  return fmul_k(K, x, redc(T));
 }
 
 
@@ -474,14 +471,14 @@ __device__ __forceinline__ void hades(Felt s[3]) {
 #pragma unroll 1
     for (int r = 0; r < 4; r++) {
 #pragma unroll
-      for (int j = 0; j < 2; j++) s[j] = fcube<1>(ladd(s[j], P252_FULL_RC[3 * (4 * half + r) + j]));
-      s[2] = fcube<3>(s[2]);
+      for (int j = 0; j < 2; j++) s[j] = fcube(1, ladd(s[j], P252_FULL_RC[3 * (4 * half + r) + j]));
+      s[2] = fcube(3, s[2]);
       mds(s, P252_S2_NEXT[half ? 87 + r : r]);
     }
     if (half == 0)
 #pragma unroll 1
       for (int k = 0; k < 83; k++) {
-        s[2] = fcube<3>(s[2]);
+        s[2] = fcube(3, s[2]);
         mds(s, P252_S2_NEXT[4 + k]);
       }
   }
@@ -500,7 +497,7 @@ __device__ __forceinline__ void to_be_words(const Felt& x, uint32_t w[8]) {
   for (int k = 0; k < 8; k++) w[k] = __byte_perm(x.v[7 - k], 0, 0x0123);
 }
 // any 256-bit x, to below 2p (below 1.1p for x < p)
-__device__ __forceinline__ Felt to_mont(const Felt& x) { return fmul_k<1>(P252_R2, x); }
+__device__ __forceinline__ Felt to_mont(const Felt& x) { return fmul_k(1, P252_R2, x); }
 __device__ __forceinline__ Felt from_mont(const Felt& x) {
   Felt one{};
   one.v[0] = 1;
@@ -571,6 +568,107 @@ __global__ void __launch_bounds__(128) poseidon252_layer_kernel(uint32_t log_siz
   }
 }
 
+// Node levels with few nodes, where one permutation's latency is the whole
+// time: a block of three warps takes 32 nodes, lane i node i, and in a full
+// round warp w cubes state element w, so a full round costs one cube and an
+// exchange through shared memory instead of three cubes. In a partial round
+// only s2 is cubed: warp 0 does that and nothing else, while warp 1 updates s0
+// and s1 with the cube of the round before and forms s0 + s1 + constant; one
+// barrier of the two a round, where warp 1 has always arrived first. With
+// at most 32 nodes the block goes on to the root, the hashes of a level
+// handed to the next in Montgomery form. One level: 60 -> 43 us
+// (two cubes fewer to wait for in each full round, the rest the additions).
+struct Levels252 {
+  uint8_t* p[6];  // level L: 2^L hashes
+};
+__global__ void __launch_bounds__(96) poseidon252_trio_kernel(uint32_t log_size, const uint8_t* __restrict__ prev,
+                                                              uint8_t* out, Levels252 up, uint32_t to_root) {
+  __shared__ uint32_t ex[2][3][8][32];
+  __shared__ uint32_t part[2][2][8][32];  // warp 0's cubes, warp 1's sums
+  __shared__ uint32_t hashes[8][32];
+  const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  int cur = 0;
+  auto put_to = [&](uint32_t (&s)[8][32], const Felt& x) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) s[q][lane] = x.v[q];
+  };
+  auto get_from = [&](const uint32_t (&s)[8][32]) {
+    Felt x;
+#pragma unroll
+    for (int q = 0; q < 8; q++) x.v[q] = s[q][lane];
+    return x;
+  };
+  auto put = [&](const Felt& x) { put_to(ex[cur][w], x); };
+  auto get = [&](uint32_t e) { return get_from(ex[cur][e]); };
+  // warps 0 and 1 alone; __syncthreads is barrier 0
+  auto pair_sync = []() { asm volatile("bar.sync 1, 64;" ::: "memory"); };
+  for (uint32_t L = log_size;; L--) {
+    const uint32_t n = 1u << L, i = 32 * blockIdx.x + lane;
+    Felt e;  // this warp's state element; s2 with its round's constant added
+    if (w == 2) {
+      e = ladd(P252_TWO, P252_FULL_RC[2]);
+    } else if (L == log_size) {
+      e = load_hash(prev, 2 * (size_t)(i < n ? i : 0) + w);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; q++) e.v[q] = hashes[q][(2 * lane + w) & 31u];
+    }
+#pragma unroll 1
+    for (int r = 0; r < 8; r++) {
+      e = w == 2 ? e : ladd(e, P252_FULL_RC[3 * r + w]);
+      e = fcube(w == 2 ? 3 : 1, e);
+      put(e);
+      __syncthreads();
+      // the MDS, an element per warp (bounds: mds())
+      const Felt s0 = get(0), s1 = get(1), s2 = get(2);
+      if (w == 0) e = lreduce(ladd(ladd(ladd(s0, s2), ladd(s0, s1)), s0));
+      else if (w == 1) e = lreduce(lsub(ladd(s0, s2), s1));
+      else e = lsub(lsub(ladd(ladd(s0, s1), P252_S2_NEXT[r < 4 ? r : 83 + r]), s2), s2);
+      cur ^= 1;
+      if (r == 3) {  // the partial rounds
+        put(e);
+        __syncthreads();
+        if (w == 0) {
+          Felt x = get(2);
+#pragma unroll 1
+          for (int k = 0; k < 83; k++) {
+            const Felt y = fcube(3, x);
+            put_to(part[k & 1][0], y);
+            pair_sync();
+            x = lsub(lsub(get_from(part[k & 1][1]), y), y);
+          }
+          put_to(ex[cur ^ 1][2], x);
+        } else if (w == 1) {
+          Felt s0 = get(0), s1 = e;
+#pragma unroll 1
+          for (int k = 0; k < 83; k++) {
+            put_to(part[k & 1][1], ladd(ladd(s0, s1), P252_S2_NEXT[4 + k]));
+            pair_sync();
+            const Felt y = get_from(part[k & 1][0]);
+            const Felt u = ladd(s0, y), v = ladd(s0, s1);
+            const Felt a0 = ladd(ladd(u, v), s0), a1 = lsub(u, s1);
+            s0 = lreduce(a0);
+            s1 = lreduce(a1);
+          }
+          put_to(ex[cur ^ 1][0], s0);
+          put_to(ex[cur ^ 1][1], s1);
+        }
+        cur ^= 1;
+        __syncthreads();
+        e = get(w);
+        cur ^= 1;
+      }
+    }
+    if (w == 0) {
+      if (i < n) store_hash(L == log_size ? out : up.p[L], i, e);
+#pragma unroll
+      for (int q = 0; q < 8; q++) hashes[q][lane] = e.v[q];
+    }
+    if (!to_root || L == 0) return;
+    __syncthreads();
+  }
+}
+
 // A batch of permutations: states of 3 big-endian hashes each (tests).
 __global__ void poseidon252_permute_kernel(const uint8_t* __restrict__ in, uint32_t n, uint8_t* __restrict__ out) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -581,6 +679,30 @@ __global__ void poseidon252_permute_kernel(const uint8_t* __restrict__ in, uint3
   }
 }
 
+// Up to here a level is at most two blocks per SM and bound by latency. The
+// line could lie anywhere from 4096 to 16384 nodes (node levels of a 2^16
+// Wide-Fibonacci proof: 12.26, 12.22, 12.22 ms); a thread per node at every
+// size took 14.25.
+constexpr size_t P252_TRIO_NODES = 8192;
+
+int poseidon252_commit_nodes(cudaStream_t st, uint32_t top_log, uint32_t* const* layers) {
+  for (int L = (int)top_log - 1; L >= 0; L--) {
+    const uint8_t* prev = (const uint8_t*)layers[L + 1];
+    if (L > 5) {
+      GS_TRY(poseidon252_commit_on_layer(st, (uint32_t)L, prev, Cols(), 0, (uint8_t*)layers[L]));
+      continue;
+    }
+    for (int k = 0; k <= L; k++) GS_REQUIRE(((uintptr_t)layers[k] & 15) == 0, "hash buffers must be 16-byte aligned");
+    Levels252 up{};
+    for (int k = 0; k < L; k++) up.p[k] = (uint8_t*)layers[k];
+    poseidon252_trio_kernel<<<1, 96, 0, st>>>((uint32_t)L, prev, (uint8_t*)layers[L], up, 1u);
+    note_launch();
+    GS_CUDA_TRY(cudaGetLastError());
+    break;
+  }
+  return OK;
+}
+
 int poseidon252_commit_on_layer(cudaStream_t st, uint32_t log_size, const uint8_t* d_prev,
                                 Cols cols, uint32_t n_cols, uint8_t* d_out) {
   GS_REQUIRE(log_size <= 30, "layer log size out of range");
@@ -588,6 +710,12 @@ int poseidon252_commit_on_layer(cudaStream_t st, uint32_t log_size, const uint8_
   GS_REQUIRE(n_cols == 0 || cols.given(), "null column table");
   GS_REQUIRE(((uintptr_t)d_out & 15) == 0 && ((uintptr_t)d_prev & 15) == 0, "hash buffers must be 16-byte aligned");
   const size_t n = (size_t)1 << log_size;
+  if (d_prev && n_cols == 0 && n <= P252_TRIO_NODES) {
+    poseidon252_trio_kernel<<<(unsigned)((n + 31) / 32), 96, 0, st>>>(log_size, d_prev, d_out, Levels252{}, 0u);
+    note_launch();
+    GS_CUDA_TRY(cudaGetLastError());
+    return OK;
+  }
   size_t blocks = (n + 127) / 128;
   const size_t cap = (size_t)num_sms() * 16;
   if (blocks > cap) blocks = cap;

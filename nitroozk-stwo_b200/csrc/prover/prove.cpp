@@ -35,9 +35,7 @@ static int fri_commit_p252(Prover& pv, uint32_t* quot[4], uint32_t lifting, FriL
     Cols cols;
     GS_TRY(pv.ctx.columns(L.planes, 4, &cols));
     GS_TRY(poseidon252_commit_on_layer(st, L.log, nullptr, cols, 4, (uint8_t*)L.layers[L.log]));
-    for (int k = (int)L.log - 1; k >= 0; k--)
-      GS_TRY(poseidon252_commit_on_layer(st, (uint32_t)k, (const uint8_t*)L.layers[k + 1], Cols(), 0,
-                                         (uint8_t*)L.layers[k]));
+    GS_TRY(poseidon252_commit_nodes(st, L.log, L.layers.data()));
     if (!busy_done && while_busy) while_busy();  // overlaps the first tree
     busy_done = true;
     GS_TRY(pv.ctx.read_back(L.layers[0], 32, L.root.data()));

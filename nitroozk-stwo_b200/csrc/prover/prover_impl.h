@@ -113,11 +113,9 @@ struct Prover {
     t.layers.assign(t.eval_log + 1, nullptr);
     for (uint32_t L = 0; L <= t.eval_log; L++) GS_TRY(A.alloc_n((size_t)8 << L, &t.layers[L]));
     const Cols tab = t.eval_cols();
-    if (ch.p252) {  // Poseidon252MerkleHasher: one launch per layer
+    if (ch.p252) {  // Poseidon252MerkleHasher
       GS_TRY(poseidon252_commit_on_layer(st, t.eval_log, nullptr, tab, t.n_cols, (uint8_t*)t.layers[t.eval_log]));
-      for (int L = (int)t.eval_log - 1; L >= 0; L--)
-        GS_TRY(poseidon252_commit_on_layer(st, (uint32_t)L, (const uint8_t*)t.layers[L + 1], Cols(), 0,
-                                           (uint8_t*)t.layers[L]));
+      GS_TRY(poseidon252_commit_nodes(st, t.eval_log, t.layers.data()));
     } else {
       GS_TRY(commit_on_layer(st, t.eval_log, nullptr, tab, t.n_cols, t.layers[t.eval_log], true));
       if (ctx.d_mail) {  // the tree kernel writes the root into mailbox slot 0 itself

@@ -310,6 +310,8 @@ int lifted_leaves(cudaStream_t st, uint32_t lift, const uint32_t* const* d_cols,
 
 // poseidon252.cu: Poseidon252 Merkle layers and permutations; hashes are
 // felt252 values as 32 big-endian bytes.
+// Every node level below top_log (layers[L]: 2^L hashes; layers[top_log] given).
+int poseidon252_commit_nodes(cudaStream_t st, uint32_t top_log, uint32_t* const* layers);
 int poseidon252_commit_on_layer(cudaStream_t st, uint32_t log_size, const uint8_t* d_prev,
                                 Cols cols, uint32_t n_cols, uint8_t* d_out);
 int poseidon252_permute(cudaStream_t st, const uint8_t* d_in, uint32_t n, uint8_t* d_out);

@@ -573,10 +573,9 @@ __global__ void __launch_bounds__(128) poseidon252_layer_kernel(uint32_t log_siz
 // round warp w cubes state element w, so a full round costs one cube and an
 // exchange through shared memory instead of three cubes. In a partial round
 // only s2 is cubed: warp 0 does that and nothing else, while warp 1 updates s0
-// and s1 with the cube of the round before and forms s0 + s1 + constant; one
-// barrier of the two a round, where warp 1 has always arrived first. With
-// at most 32 nodes the block goes on to the root, the hashes of a level
-// handed to the next in Montgomery form. One level: 60 -> 43 us
+// and s1 with the cube of the round before and hands back s0 + s1 + constant,
+// which warp 0 picks up between its square and its product. With at most 32 nodes the block goes on to the root, the hashes of a level
+// handed to the next in Montgomery form. One level: 60 -> 39 us
 // (two cubes fewer to wait for in each full round, the rest the additions).
 struct Levels252 {
   uint8_t* p[6];  // level L: 2^L hashes
@@ -584,7 +583,7 @@ struct Levels252 {
 __global__ void __launch_bounds__(96) poseidon252_trio_kernel(uint32_t log_size, const uint8_t* __restrict__ prev,
                                                               uint8_t* out, Levels252 up, uint32_t to_root) {
   __shared__ uint32_t ex[2][3][8][32];
-  __shared__ uint32_t part[2][2][8][32];  // warp 0's cubes, warp 1's sums
+  __shared__ uint32_t part[2][8][32];  // warp 0's cubes, warp 1's sums
   __shared__ uint32_t hashes[8][32];
   const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   int cur = 0;
@@ -600,8 +599,12 @@ __global__ void __launch_bounds__(96) poseidon252_trio_kernel(uint32_t log_size,
   };
   auto put = [&](const Felt& x) { put_to(ex[cur][w], x); };
   auto get = [&](uint32_t e) { return get_from(ex[cur][e]); };
-  // warps 0 and 1 alone; __syncthreads is barrier 0
-  auto pair_sync = []() { asm volatile("bar.sync 1, 64;" ::: "memory"); };
+  // Barriers of warps 0 and 1 (__syncthreads is barrier 0): 1, a cube is there
+  // (warp 0 arrives and goes on, warp 1 waits); 2, a sum is there (the other
+  // way round). They alternate: a warp arrives at one only after a wait at the
+  // other, which its partner reaches past its own wait at the first.
+  auto bar_arrive = [](int id) { asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory"); };
+  auto bar_sync = [](int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); };
   for (uint32_t L = log_size;; L--) {
     const uint32_t n = 1u << L, i = 32 * blockIdx.x + lane;
     Felt e;  // this warp's state element; s2 with its round's constant added
@@ -632,19 +635,29 @@ __global__ void __launch_bounds__(96) poseidon252_trio_kernel(uint32_t log_size,
           Felt x = get(2);
 #pragma unroll 1
           for (int k = 0; k < 83; k++) {
-            const Felt y = fcube(3, x);
-            put_to(part[k & 1][0], y);
-            pair_sync();
-            x = lsub(lsub(get_from(part[k & 1][1]), y), y);
+            uint32_t T[16];
+            sqr_wide8(x, T);
+            const Felt q = redc(T);
+            bar_sync(2);
+            const Felt sum = get_from(part[1]);
+            const Felt y = fmul_k(3, x, q);
+            put_to(part[0], y);
+            bar_arrive(1);
+            Felt y2;
+            y2.v[0] = y.v[0] << 1;
+#pragma unroll
+            for (int j = 1; j < 8; j++) y2.v[j] = __funnelshift_l(y.v[j - 1], y.v[j], 1);
+            x = lsub(sum, y2);
           }
           put_to(ex[cur ^ 1][2], x);
         } else if (w == 1) {
           Felt s0 = get(0), s1 = e;
 #pragma unroll 1
           for (int k = 0; k < 83; k++) {
-            put_to(part[k & 1][1], ladd(ladd(s0, s1), P252_S2_NEXT[4 + k]));
-            pair_sync();
-            const Felt y = get_from(part[k & 1][0]);
+            put_to(part[1], ladd(ladd(s0, s1), P252_S2_NEXT[4 + k]));
+            bar_arrive(2);
+            bar_sync(1);
+            const Felt y = get_from(part[0]);
             const Felt u = ladd(s0, y), v = ladd(s0, s1);
             const Felt a0 = ladd(ladd(u, v), s0), a1 = lsub(u, s1);
             s0 = lreduce(a0);
@@ -680,8 +693,8 @@ __global__ void poseidon252_permute_kernel(const uint8_t* __restrict__ in, uint3
 }
 
 // Up to here a level is at most two blocks per SM and bound by latency. The
-// line could lie anywhere from 4096 to 16384 nodes (node levels of a 2^16
-// Wide-Fibonacci proof: 12.26, 12.22, 12.22 ms); a thread per node at every
+// line could lie anywhere from 4096 to 16384 nodes (the hashing of a 2^16
+// Wide-Fibonacci proof differs by 0.04 of 11.5 ms); a thread per node at every
 // size took 14.25.
 constexpr size_t P252_TRIO_NODES = 8192;
 

@@ -40,6 +40,7 @@ __host__ __device__ __forceinline__ uint32_t seeded_m31(uint64_t seed, uint64_t 
 
 // ------------------------------------------------------------ wide fibonacci
 __global__ void wf_trace_kernel(uint32_t* cols, uint32_t log_n, uint32_t n_cols, uint64_t seed, uint32_t mode) {
+  after_previous();
   const size_t n = (size_t)1 << log_n;
   for (size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x; r < n; r += (size_t)gridDim.x * blockDim.x) {
     // mode 0: the reference's inputs (a = 1, b = row); 1: seeded; 2: preloaded columns 0-1
@@ -86,6 +87,8 @@ struct TableCols {
   __device__ __forceinline__ const uint32_t* col(uint32_t c) const { return tab[c]; }
   __device__ __forceinline__ Cursor cursor(uint32_t c, size_t r) const { return Cursor{tab + c, r}; }
 };
+__device__ __forceinline__ void shift_one(ContigCols& c, size_t z) { c.base += z; }
+__device__ __forceinline__ void shift_one(TableCols& c, size_t z) { c.tab += z; }
 
 // Writes (accumulate == 0) or adds to (accumulate != 0) the output planes.
 __device__ __forceinline__ void store_quotient(const Planes& out, size_t r, const uint32_t v[4], uint32_t accumulate) {
@@ -97,6 +100,7 @@ template <class Cols>
 __global__ void __launch_bounds__(256) wf_constraints_kernel(Cols cols, uint32_t n_cols, uint32_t eval_log,
                                                              uint32_t trace_log, ConstraintParams prm, Planes out,
                                                              uint32_t accumulate) {
+  after_previous(cols);
   const size_t n = (size_t)1 << eval_log;
   for (size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x; r < n; r += (size_t)gridDim.x * blockDim.x) {
     auto cur = cols.cursor(0, r);
@@ -171,6 +175,7 @@ __host__ __device__ __forceinline__ void p2_internal(uint32_t* s) {
 __host__ __device__ __forceinline__ uint32_t pow5(uint32_t x) { uint32_t x2 = sqr(x); return mul(sqr(x2), x); }
 
 __global__ void poseidon_trace_kernel(uint32_t* cols, uint32_t log_n, uint64_t seed, uint32_t mode) {
+  after_previous();
   const size_t n = (size_t)1 << log_n;
   for (size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x; r < n; r += (size_t)gridDim.x * blockDim.x) {
     uint32_t s[16];
@@ -242,6 +247,7 @@ __device__ __forceinline__ uint32_t coset_index(uint32_t i, uint32_t log_n) {
 template <class InitCols, class FinalCols>
 __global__ void logup_fraction_kernel(InitCols init, uint32_t c_init, FinalCols fin, uint32_t c_final, uint32_t log_n,
                                       LookupParams lp, uint4* __restrict__ coset_vals) {
+  after_previous(init, fin);
   const size_t n = (size_t)1 << log_n;
   for (size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x; r < n; r += (size_t)gridDim.x * blockDim.x) {
     qm31 d0 = combine16(lp, init, c_init, r);
@@ -261,6 +267,7 @@ struct AddQM {
 // shift = S[n - 1] / n (the claimed sum over n, inv_n = 1/n mod p), read here
 // so that the host need not wait for the sum first.
 __global__ void logup_finalize_kernel(const uint4* __restrict__ scan, uint32_t log_n, uint32_t inv_n, Planes out) {
+  after_previous(scan);
   const size_t n = (size_t)1 << log_n;
   const uint4 total = scan[n - 1];
   const qm31 shift = qm_mul_m31(qm_make(total.x, total.y, total.z, total.w), inv_n);
@@ -297,6 +304,7 @@ __global__ void __launch_bounds__(128, 7) poseidon_constraints_kernel(TraceCols 
                                                                    uint32_t trace_log, ConstraintParams prm,
                                                                    LookupParams lp, qm31 cumsum_shift, Planes out,
                                                                    uint32_t accumulate) {
+  after_previous(trace, inter);
   const size_t n = (size_t)1 << eval_log;
   for (size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x; r < n; r += (size_t)gridDim.x * blockDim.x) {
     uint64_t acc[4] = {0, 0, 0, 0};
@@ -374,7 +382,7 @@ static unsigned grid_rows(size_t n, int threads) {
 
 int wf_trace(cudaStream_t st, uint32_t* cols, uint32_t log_n, uint32_t n_cols, uint64_t seed, uint32_t mode) {
   GS_REQUIRE(n_cols >= 2 && log_n <= 28, "bad wide fibonacci shape");
-  wf_trace_kernel<<<grid_rows((size_t)1 << log_n, 256), 256, 0, st>>>(cols, log_n, n_cols, seed, mode);
+  launch_after(wf_trace_kernel, grid_rows((size_t)1 << log_n, 256), 256, 0, st, cols, log_n, n_cols, seed, mode);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;
@@ -383,8 +391,9 @@ int wf_trace(cudaStream_t st, uint32_t* cols, uint32_t log_n, uint32_t n_cols, u
 int wf_constraints(cudaStream_t st, const uint32_t* cols, uint32_t n_cols, uint32_t eval_log, uint32_t trace_log,
                    const ConstraintParams& prm, Planes out) {
   GS_REQUIRE(n_cols >= 3 && n_cols - 2 <= MAX_CONSTRAINTS, "bad wide fibonacci width");
-  wf_constraints_kernel<<<grid_rows((size_t)1 << eval_log, 256), 256, 0, st>>>(
-      ContigCols{cols, (size_t)1 << eval_log}, n_cols, eval_log, trace_log, prm, out, 0u);
+  launch_after(wf_constraints_kernel<ContigCols>,
+               grid_rows((size_t)1 << eval_log, 256), 256, 0, st, ContigCols{cols, (size_t)1 << eval_log},
+               n_cols, eval_log, trace_log, prm, out, 0u);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;
@@ -394,8 +403,9 @@ int wf_constraints_table(cudaStream_t st, const uint32_t* const* d_cols, uint32_
                          uint32_t trace_log, const ConstraintParams& prm, Planes out, bool accumulate) {
   GS_REQUIRE(n_cols >= 3 && n_cols - 2 <= MAX_CONSTRAINTS, "bad wide fibonacci width");
   GS_REQUIRE(eval_log > trace_log && eval_log - trace_log <= 3 && eval_log <= 30, "bad domain sizes");
-  wf_constraints_kernel<<<grid_rows((size_t)1 << eval_log, 256), 256, 0, st>>>(
-      TableCols{d_cols}, n_cols, eval_log, trace_log, prm, out, accumulate ? 1u : 0u);
+  launch_after(wf_constraints_kernel<TableCols>,
+               grid_rows((size_t)1 << eval_log, 256), 256, 0, st, TableCols{d_cols}, n_cols,
+               eval_log, trace_log, prm, out, accumulate ? 1u : 0u);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;
@@ -403,7 +413,7 @@ int wf_constraints_table(cudaStream_t st, const uint32_t* const* d_cols, uint32_
 
 int poseidon_trace(cudaStream_t st, uint32_t* cols, uint32_t log_n, uint64_t seed, uint32_t mode) {
   GS_REQUIRE(log_n <= 28, "bad poseidon size");
-  poseidon_trace_kernel<<<grid_rows((size_t)1 << log_n, 128), 128, 0, st>>>(cols, log_n, seed, mode);
+  launch_after(poseidon_trace_kernel, grid_rows((size_t)1 << log_n, 128), 128, 0, st, cols, log_n, seed, mode);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;
@@ -434,12 +444,13 @@ static int interaction_impl(cudaStream_t st, InitCols init, uint32_t c_init, Fin
   void* temp = (void*)(scan + n);
   size_t temp_bytes = 0;
   cub::DeviceScan::InclusiveScan(nullptr, temp_bytes, (const uint4*)nullptr, (uint4*)nullptr, AddQM(), (int)n);
-  logup_fraction_kernel<<<grid_rows(n, 128), 128, 0, st>>>(init, c_init, fin, c_final, log_n, lp, vals);
+  launch_after(logup_fraction_kernel<InitCols, FinalCols>, grid_rows(n, 128), 128, 0, st, init, c_init, fin, c_final,
+               log_n, lp, vals);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   GS_CUDA_TRY(cub::DeviceScan::InclusiveScan(temp, temp_bytes, (const uint4*)vals, scan, AddQM(), (int)n, st));
   note_launch();
-  logup_finalize_kernel<<<grid_rows(n, 256), 256, 0, st>>>(scan, log_n, inv((uint32_t)(n % P)), out);
+  launch_after(logup_finalize_kernel, grid_rows(n, 256), 256, 0, st, scan, log_n, inv((uint32_t)(n % P)), out);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   if (claimed_sum) {
@@ -558,8 +569,8 @@ int poseidon_constraints(cudaStream_t st, const uint32_t* trace, const uint32_t*
                          Planes out) {
   GS_REQUIRE(eval_log > trace_log, "poseidon constraints need an extended domain");
   const size_t n = (size_t)1 << eval_log;
-  poseidon_constraints_kernel<<<grid_rows(n, 128), 128, 0, st>>>(ContigCols{trace, n}, ContigCols{inter, n}, eval_log,
-                                                                  trace_log, prm, lp, cumsum_shift, out, 0u);
+  launch_after(poseidon_constraints_kernel<ContigCols, ContigCols>, grid_rows(n, 128), 128, 0, st, ContigCols{trace, n},
+               ContigCols{inter, n}, eval_log, trace_log, prm, lp, cumsum_shift, out, 0u);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;
@@ -569,8 +580,9 @@ int poseidon_constraints_table(cudaStream_t st, const uint32_t* const* d_trace, 
                                uint32_t eval_log, uint32_t trace_log, const ConstraintParams& prm,
                                const LookupParams& lp, qm31 cumsum_shift, Planes out, bool accumulate) {
   GS_REQUIRE(eval_log > trace_log && eval_log - trace_log <= 3 && eval_log <= 30, "bad domain sizes");
-  poseidon_constraints_kernel<<<grid_rows((size_t)1 << eval_log, 128), 128, 0, st>>>(
-      TableCols{d_trace}, TableCols{d_inter}, eval_log, trace_log, prm, lp, cumsum_shift, out, accumulate ? 1u : 0u);
+  launch_after(poseidon_constraints_kernel<TableCols, TableCols>,
+               grid_rows((size_t)1 << eval_log, 128), 128, 0, st, TableCols{d_trace},
+               TableCols{d_inter}, eval_log, trace_log, prm, lp, cumsum_shift, out, accumulate ? 1u : 0u);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;

@@ -18,11 +18,12 @@ struct Factors { qm31 f[31]; };
 
 // W[j] = prod over set bits b < s of j of F_b, for j < 2^s (one thread each).
 __global__ void eap_weights_kernel(Factors fs, uint32_t s, uint32_t* w /* [j][4] */) {
-  uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= (1u << s)) return;
+  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   qm31 acc = qm_one();
   for (uint32_t b = 0; b < s; b++)
     if ((j >> b) & 1u) acc = qm_mul(acc, fs.f[b]);
+  after_previous();  // (the products need no memory)
+  if (j >= (1u << s)) return;
   w[4 * j + 0] = acc.x.a; w[4 * j + 1] = acc.x.b; w[4 * j + 2] = acc.y.a; w[4 * j + 3] = acc.y.b;
 }
 
@@ -34,6 +35,7 @@ __global__ void eap_weights_kernel(Factors fs, uint32_t s, uint32_t* w /* [j][4]
 __global__ void __launch_bounds__(256) eap_chunk_kernel(Cols polys, uint32_t log_n,
                                                         uint32_t s, const uint32_t* __restrict__ w, Factors fs,
                                                         uint32_t* partials, bool vec) {
+  after_previous(polys, w);
   __shared__ uint32_t red[4][256 / 32];
   const uint32_t poly = blockIdx.y;
   const uint32_t chunk = blockIdx.x;
@@ -108,6 +110,7 @@ __global__ void __launch_bounds__(256) eap_chunk_multi_kernel(Cols polys,
                                                               uint32_t n_polys, uint32_t log_n,
                                                               const uint32_t* __restrict__ w, Factors fs,
                                                               uint32_t* partials) {
+  after_previous(polys, w);
   __shared__ uint32_t red[K][4][8];
   const uint32_t chunk = blockIdx.x, p0 = blockIdx.y * K;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -177,6 +180,7 @@ __global__ void __launch_bounds__(256) eap_chunk_multi_kernel(Cols polys,
 // order does not change the result).
 __global__ void __launch_bounds__(128) eap_finalize_kernel(const uint32_t* partials, uint32_t n_chunks, uint32_t n_polys,
                                                            uint32_t* out) {
+  after_previous(partials);
   __shared__ uint4 red[4];
   const uint32_t poly = blockIdx.x;
   const uint4* p = reinterpret_cast<const uint4*>(partials) + (size_t)poly * n_chunks;
@@ -235,22 +239,22 @@ int batch_eval_at_point(cudaStream_t st, Cols polys, uint32_t n_polys, uint32_t 
   uint32_t* w = d_scratch;
   // one chunk per polynomial: its sum is the value
   uint32_t* partials = chunks == 1 ? d_out : d_scratch + 4 * (1u << s);
-  eap_weights_kernel<<<((1u << s) + 255) / 256, 256, 0, st>>>(fs, s, w);
+  launch_after(eap_weights_kernel, ((1u << s) + 255) / 256, 256, 0, st, fs, s, w);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   if (vec && s == EAP_MULTI_LOG) {
     // four polynomials per block (two: L1-bound again, 84 µs on the Poseidon2
     // 2^18 trace; eight: register-bound, 75 µs; four: 54 µs)
     dim3 grid(chunks, (n_polys + 3) / 4);
-    eap_chunk_multi_kernel<4><<<grid, 256, 0, st>>>(polys, n_polys, log_n, w, fs, partials);
+    launch_after(eap_chunk_multi_kernel<4>, grid, 256, 0, st, polys, n_polys, log_n, w, fs, partials);
   } else {
     dim3 grid(chunks, n_polys);
-    eap_chunk_kernel<<<grid, 256, 0, st>>>(polys, log_n, s, w, fs, partials, vec);
+    launch_after(eap_chunk_kernel, grid, 256, 0, st, polys, log_n, s, w, fs, partials, vec);
   }
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   if (chunks == 1) return OK;
-  eap_finalize_kernel<<<n_polys, 128, 0, st>>>(partials, chunks, n_polys, d_out);
+  launch_after(eap_finalize_kernel, n_polys, 128, 0, st, partials, chunks, n_polys, d_out);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;

@@ -236,6 +236,7 @@ __host__ __device__ constexpr uint32_t padw(uint32_t e) { return e + (e >> 5); }
 template <bool INV, int L, int C>
 __global__ void __launch_bounds__(256) fft_tile_kernel(Cols src_tab, MutCols dst_tab,
                                                        const uint32_t* __restrict__ tw, FftPass a) {
+  after_previous(src_tab, tw);
   extern __shared__ uint32_t sm[];
   constexpr int R = 5, NQ = 32;
   constexpr int T = L + C;
@@ -394,6 +395,7 @@ struct StreamGrid {
 template <bool INV, int L, int C, int TB>
 __global__ void __launch_bounds__(1 << (TB - 5), (StreamShape<INV, L, C, TB>::PER_SM))
     fft_stream_kernel(Cols src_tab, MutCols dst_tab, const uint32_t* __restrict__ tw, FftPass a, StreamGrid g) {
+  after_previous(tw);
   using Shape = StreamShape<INV, L, C, TB>;
   constexpr int R = 5, NQ = 32, T = C > 0 ? TB : L;  // T: tile bits of one transform
   constexpr int K = (L + R - 1) / R;
@@ -769,7 +771,7 @@ static void launch_tile(cudaStream_t st, dim3 grid, uint32_t threads, Cols s, Mu
                         const uint32_t* tw, const FftPass& a) {
   const uint32_t words = 1u << (a.t + a.tile_shift);
   const size_t smem = (size_t)4 * (words + (words >> 5));
-  fft_tile_kernel<INV, L, C><<<grid, threads, smem, st>>>(s, d, tw, a);
+  launch_after(fft_tile_kernel<INV, L, C>, grid, threads, smem, st, s, d, tw, a);
   note_launch();
 }
 
@@ -805,7 +807,7 @@ static int launch_stream(cudaStream_t st, uint32_t n_cols, Cols s, MutCols d,
   g.sets_first = C == 0 || a.src_mask != 0xffffffffu;
   const uint32_t per = stream_tiles(g.set_log, g.units, Shape::PER_SM);
   g.group = (g.units + per - 1) / per;
-  fft_stream_kernel<INV, L, C, TB><<<g.group << g.set_log, Shape::THREADS, Shape::SMEM, st>>>(s, d, tw, a, g);
+  launch_after(fft_stream_kernel<INV, L, C, TB>, g.group << g.set_log, Shape::THREADS, Shape::SMEM, st, s, d, tw, a, g);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;

@@ -50,6 +50,7 @@ __device__ __forceinline__ void load_pair(CPlanes s, size_t i, qm31& a, qm31& b)
 // written by the device channel; overrides `alpha`.
 __global__ void fold_line_kernel(CPlanes src, uint32_t log_n, qm31 alpha, Planes dst, const uint32_t* __restrict__ itw,
                                  uint32_t tw_len, uint32_t* leaf_out, const uint32_t* __restrict__ d_alpha, uint32_t one) {
+  after_previous(src, itw, d_alpha);
   const size_t half = (size_t)1 << (log_n - 1);
   if (d_alpha) alpha = qm_make(d_alpha[0], d_alpha[1], d_alpha[2], d_alpha[3]);
   const uint32_t* lvl = itw + (tw_len - (1u << log_n));
@@ -71,6 +72,7 @@ __global__ void fold_circle_kernel(CPlanes src, uint32_t log_n, qm31 alpha, qm31
                                    const uint32_t* __restrict__ itw, uint32_t tw_len, SmallInvY small,
                                    uint32_t* leaf_out, const uint32_t* __restrict__ d_alpha, uint32_t one,
                                    uint32_t fresh) {
+  after_previous(src, itw, d_alpha);
   const size_t half = (size_t)1 << (log_n - 1);
   if (d_alpha) {
     alpha = qm_make(d_alpha[0], d_alpha[1], d_alpha[2], d_alpha[3]);
@@ -111,8 +113,8 @@ static int fold_line_launch(cudaStream_t st, CPlanes src, uint32_t log_n, qm31 a
                             const uint32_t* d_itw, uint32_t tw_log, uint32_t* leaf_out, const uint32_t* d_alpha) {
   GS_REQUIRE(log_n >= 1 && log_n <= tw_log, "fold_line: line domain must fit the twiddle tree");
   size_t half = (size_t)1 << (log_n - 1);
-  fold_line_kernel<<<grid_for(half, 256), 256, 0, st>>>(src, log_n, alpha, dst, d_itw, 1u << tw_log, leaf_out,
-                                                        d_alpha, 1u);
+  launch_after(fold_line_kernel, grid_for(half, 256), 256, 0, st, src, log_n, alpha, dst, d_itw,
+               1u << tw_log, leaf_out, d_alpha, 1u);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;
@@ -152,8 +154,8 @@ static int fold_circle_launch(cudaStream_t st, CPlanes src, uint32_t log_n, qm31
   }
   qm31 alpha_sq = qm_mul(alpha, alpha);
   size_t half = (size_t)1 << (log_n - 1);
-  fold_circle_kernel<<<grid_for(half, 256), 256, 0, st>>>(src, log_n, alpha, alpha_sq, dst, d_itw, 1u << tw_log, small,
-                                                          leaf_out, d_alpha, 1u, fresh ? 1u : 0u);
+  launch_after(fold_circle_kernel, grid_for(half, 256), 256, 0, st, src, log_n, alpha, alpha_sq, dst, d_itw,
+               1u << tw_log, small, leaf_out, d_alpha, 1u, fresh ? 1u : 0u);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;
@@ -193,13 +195,14 @@ __device__ __forceinline__ void bar_sync_128() { asm volatile("bar.sync 1, 128;"
 __global__ void __launch_bounds__(1024) fri_tail_cta_kernel(FriTail a, uint32_t* state,
                                                             const uint32_t* __restrict__ itw, uint32_t tw_len,
                                                             uint32_t one) {
+  const uint32_t zero = (uint32_t)after_previous(itw);
   extern __shared__ uint4 tsm[];
   __shared__ ChannelWords ch;
   __shared__ uint32_t quad_tab[40];
   auto hashes = [&](int i) { return tsm + 2048 * i; };
   auto vals = [&](uint32_t i) { return tsm + 4096 + 1024 * i; };
   uint4* const msgs = tsm + 6144;
-  const uint32_t tid = threadIdx.x, j = tid & 3u;
+  const uint32_t tid = threadIdx.x + zero, j = tid & 3u;
   blake2s_quad_table(quad_tab);
   if (tid < 32) {
     channel_begin(ch, state);  // read by warp 0 after a root
@@ -308,7 +311,7 @@ int fri_tail(cudaStream_t st, const FriTail& a, uint32_t* d_state, const uint32_
   static const cudaError_t attr =
       cudaFuncSetAttribute(fri_tail_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_CTA_SMEM);
   GS_CUDA_TRY(attr);
-  fri_tail_cta_kernel<<<1, 1024, TAIL_CTA_SMEM, st>>>(a, d_state, d_itw, 1u << tw_log, 1u);
+  launch_after(fri_tail_cta_kernel, 1, 1024, TAIL_CTA_SMEM, st, a, d_state, d_itw, 1u << tw_log, 1u);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;

@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(256) gather_all_kernel(const ColGather* __rest
                                                          uint32_t X, const uint32_t* __restrict__ positions,
                                                          uint32_t* words, const HashRun* __restrict__ runs,
                                                          const uint32_t* __restrict__ idx, uint32_t* hashes) {
+  after_previous(blocks, positions, runs, idx);
   const uint32_t bid = blockIdx.x;
   if (bid < n_blocks * X) {
     const ColGather b = blocks[bid / X];
@@ -87,8 +88,8 @@ int gather_all(cudaStream_t st, const ColGather* d_blocks, uint32_t n_blocks, ui
   if (grid == 0) return OK;
   GS_REQUIRE(grid <= 0x7fffffffu, "too many gather blocks");
   GS_REQUIRE(n_runs == 0 || ((uintptr_t)d_hashes & 15) == 0, "hash gather output must be 16-byte aligned");
-  gather_all_kernel<<<(unsigned)grid, 256, 0, st>>>(d_blocks, n_blocks, X, d_positions, d_words, d_runs, d_idx,
-                                                    d_hashes);
+  launch_after(gather_all_kernel, (unsigned)grid, 256, 0, st, d_blocks, n_blocks, X, d_positions, d_words, d_runs,
+               d_idx, d_hashes);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;

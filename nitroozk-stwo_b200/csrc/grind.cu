@@ -40,6 +40,7 @@ constexpr uint32_t GRIND_LOW_LOG = 20, GRIND_STEP = 256;
 // earlier kernel of the stream; `d` is used when it is null.
 __global__ void __launch_bounds__(GRIND_STEP) grind_kernel(Digest8 d, const uint32_t* d_prefix, uint32_t hi,
                                                            uint32_t pow_bits, uint32_t* result) {
+  after_previous();
   const volatile uint32_t* best = result;
   if (d_prefix)
 #pragma unroll
@@ -82,7 +83,7 @@ int grind_blake2s(cudaStream_t st, const uint32_t prefixed_digest[8], uint32_t p
   const uint32_t max_hi = grind_max_hi();
   for (uint32_t hi = hi0; hi < max_hi; hi++) {
     GS_CUDA_TRY(cudaMemsetAsync(d_scratch, 0xff, 4, st));
-    grind_kernel<<<blocks, GRIND_STEP, 0, st>>>(d, nullptr, hi, pow_bits, d_scratch);
+    launch_after(grind_kernel, blocks, GRIND_STEP, 0, st, d, nullptr, hi, pow_bits, d_scratch);
     note_launch();
     GS_CUDA_TRY(cudaGetLastError());
     uint32_t local = 0;
@@ -136,6 +137,7 @@ size_t fri_last_layer_pow_words(uint32_t bound_log) { return ((size_t)4 << bound
 // backend/simd/grind.rs). The host restates every step and compares.
 __global__ void fri_last_layer_prefix_kernel(const uint32_t* last, LastLayerArgs a, const uint32_t* state,
                                              uint32_t* out) {
+  after_previous();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   const uint32_t n = 1u << a.log;
   qm31 v[1u << FRI_POW_MAX_LOG];
@@ -211,12 +213,12 @@ int fri_last_layer_pow(cudaStream_t st, const uint32_t* d_last, uint32_t log, ui
     }
     off += 1u << (l - 1);
   }
-  fri_last_layer_prefix_kernel<<<1, 32, 0, st>>>(d_last, a, d_state, d_out);
+  launch_after(fri_last_layer_prefix_kernel, 1, 32, 0, st, d_last, a, d_state, d_out);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   const uint32_t* d_prefix = d_out + ((size_t)4 << bound_log) + 8;
   uint32_t* d_best = d_out + ((size_t)4 << bound_log) + 16;
-  grind_kernel<<<grind_blocks(pow_bits), GRIND_STEP, 0, st>>>(Digest8{}, d_prefix, 0, pow_bits, d_best);
+  launch_after(grind_kernel, grind_blocks(pow_bits), GRIND_STEP, 0, st, Digest8{}, d_prefix, 0, pow_bits, d_best);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;

@@ -87,6 +87,7 @@ template <bool PREV>
 __global__ void __launch_bounds__(32 * COL_WARPS, 8)
     merkle_columns_kernel(uint32_t log_size, const uint32_t* __restrict__ prev,
                           Cols cols, uint32_t n_cols, uint32_t* __restrict__ out, uint32_t one) {
+  after_previous(prev);
   __shared__ uint4 stage[COL_WARPS][2][16 * 8];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t n_tiles = 1u << (log_size - 5), n_warps = gridDim.x * COL_WARPS;
@@ -207,9 +208,9 @@ int commit_on_layer(cudaStream_t st, uint32_t log_size, const uint32_t* d_prev, 
     const size_t resident = (size_t)num_sms() * 8;  // one wave; a warp walks its tiles, copies crossing from one to the next
     const unsigned grid = (unsigned)(tiles < resident ? tiles : resident);
     if (d_prev)
-      merkle_columns_kernel<true><<<grid, 32 * COL_WARPS, 0, st>>>(log_size, d_prev, cols, n_cols, d_out, 1u);
+      launch_after(merkle_columns_kernel<true>, grid, 32 * COL_WARPS, 0, st, log_size, d_prev, cols, n_cols, d_out, 1u);
     else
-      merkle_columns_kernel<false><<<grid, 32 * COL_WARPS, 0, st>>>(log_size, d_prev, cols, n_cols, d_out, 1u);
+      launch_after(merkle_columns_kernel<false>, grid, 32 * COL_WARPS, 0, st, log_size, d_prev, cols, n_cols, d_out, 1u);
   } else if (alu_only)
     merkle_layer_kernel<false><<<(unsigned)blocks, threads, 0, st>>>(log_size, d_prev, cols, n_cols, d_out, 1u);
   else
@@ -286,6 +287,7 @@ template <int U, int TH>
 __global__ void __launch_bounds__(TH, TH >= 256 ? 4 : 8)
     merkle_tree_kernel(uint32_t top, TreePtrs layers, uint32_t* counters, uint32_t* state, uint32_t* root_copy,
                        uint32_t* felt, uint32_t one) {
+  const uint32_t zero = (uint32_t)after_previous();
   static_assert(TH >= 128, "four lanes for each of 32 nodes");
   __shared__ uint4 buf[2][1 << U];
   __shared__ ChannelWords ch;
@@ -293,7 +295,7 @@ __global__ void __launch_bounds__(TH, TH >= 256 ? 4 : 8)
   const uint32_t tid = threadIdx.x, j = tid & 3u;
   blake2s_quad_table(quad_tab);
   uint32_t in_log = top;
-  uint32_t u = blockIdx.x;
+  uint32_t u = blockIdx.x + zero;
   uint32_t cnt_off = 0;
   for (;;) {
     const int out_log = in_log > U ? (int)in_log - U : 0;
@@ -583,8 +585,8 @@ int commit_node_layers_ch(cudaStream_t st, uint32_t top_log, uint32_t* const* la
       GS_REQUIRE(need <= TREE_COUNTERS, "tree too large for the ticket counters");
     }
     const uint32_t blocks = top > (uint32_t)unit ? 1u << (top - unit) : 1u;
-    merkle_tree_kernel<unit, TREE_THREADS><<<blocks, TREE_THREADS, 0, st>>>(top, tp, d_counters, d_state,
-                                                                           d_root_copy, d_felt, 1u);
+    launch_after(merkle_tree_kernel<unit, TREE_THREADS>, blocks, TREE_THREADS, 0, st, top, tp, d_counters, d_state,
+                 d_root_copy, d_felt, 1u);
     note_launch();
     GS_CUDA_TRY(cudaGetLastError());
     return OK;

@@ -548,6 +548,7 @@ __device__ __forceinline__ Felt node_value(uint32_t k, size_t i, const uint8_t* 
 __global__ void __launch_bounds__(128) poseidon252_layer_kernel(uint32_t log_size, const uint8_t* __restrict__ prev,
                                                                 Cols cols, uint32_t n_cols,
                                                                 uint8_t* __restrict__ out) {
+  after_previous(prev, cols);
   const size_t n = (size_t)1 << log_size;
   const bool node_only = prev && n_cols == 0;
   const uint32_t m = (prev ? 2u : 0u) + (n_cols + 7) / 8;  // values
@@ -582,6 +583,7 @@ struct Levels252 {
 };
 __global__ void __launch_bounds__(96) poseidon252_trio_kernel(uint32_t log_size, const uint8_t* __restrict__ prev,
                                                               uint8_t* out, Levels252 up, uint32_t to_root) {
+  after_previous(prev);
   __shared__ uint32_t ex[2][3][8][32];
   __shared__ uint32_t part[2][8][32];  // warp 0's cubes, warp 1's sums
   __shared__ uint32_t hashes[8][32];
@@ -708,7 +710,7 @@ int poseidon252_commit_nodes(cudaStream_t st, uint32_t top_log, uint32_t* const*
     for (int k = 0; k <= L; k++) GS_REQUIRE(((uintptr_t)layers[k] & 15) == 0, "hash buffers must be 16-byte aligned");
     Levels252 up{};
     for (int k = 0; k < L; k++) up.p[k] = (uint8_t*)layers[k];
-    poseidon252_trio_kernel<<<1, 96, 0, st>>>((uint32_t)L, prev, (uint8_t*)layers[L], up, 1u);
+    launch_after(poseidon252_trio_kernel, 1, 96, 0, st, (uint32_t)L, prev, (uint8_t*)layers[L], up, 1u);
     note_launch();
     GS_CUDA_TRY(cudaGetLastError());
     break;
@@ -724,7 +726,8 @@ int poseidon252_commit_on_layer(cudaStream_t st, uint32_t log_size, const uint8_
   GS_REQUIRE(((uintptr_t)d_out & 15) == 0 && ((uintptr_t)d_prev & 15) == 0, "hash buffers must be 16-byte aligned");
   const size_t n = (size_t)1 << log_size;
   if (d_prev && n_cols == 0 && n <= P252_TRIO_NODES) {
-    poseidon252_trio_kernel<<<(unsigned)((n + 31) / 32), 96, 0, st>>>(log_size, d_prev, d_out, Levels252{}, 0u);
+    launch_after(poseidon252_trio_kernel, (unsigned)((n + 31) / 32), 96, 0, st, log_size, d_prev, d_out, Levels252{},
+                 0u);
     note_launch();
     GS_CUDA_TRY(cudaGetLastError());
     return OK;
@@ -732,7 +735,7 @@ int poseidon252_commit_on_layer(cudaStream_t st, uint32_t log_size, const uint8_
   size_t blocks = (n + 127) / 128;
   const size_t cap = (size_t)num_sms() * 16;
   if (blocks > cap) blocks = cap;
-  poseidon252_layer_kernel<<<(unsigned)blocks, 128, 0, st>>>(log_size, d_prev, cols, n_cols, d_out);
+  launch_after(poseidon252_layer_kernel, (unsigned)blocks, 128, 0, st, log_size, d_prev, cols, n_cols, d_out);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;

@@ -135,10 +135,11 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // entries (k = g, g + EG, ...). In a round the RG warps of an entry group
 // read 512·RG contiguous bytes of one column, which keeps HBM pages open.
 template <int EG>
-__global__ void __launch_bounds__(256, 4) accumulate_numerators_split_kernel(const NumEntry* __restrict__ entries,
+__global__ void __launch_bounds__(256, 4) accumulate_numerators_split_kernel(const NumEntry* entries,
                                                                              uint32_t n_entries, qm31 b_sum,
                                                                              uint32_t log_size, Planes out,
-                                                                             const uint32_t* __restrict__ bsum_dev) {
+                                                                             const uint32_t* bsum_dev) {
+  after_previous();
   if (bsum_dev) b_sum = qm_make(bsum_dev[0], bsum_dev[1], bsum_dev[2], bsum_dev[3]);
   constexpr uint32_t RG = 8 / EG, TILE = 128 * RG, STRIDE = EG * ACC_ROUND;
   extern __shared__ uint4 dyn[];  // [warp][slot][entry][lane] in the loop; part[group][q][row] after it
@@ -245,8 +246,8 @@ int accumulate_numerators(cudaStream_t st, const void* d_entries, uint32_t n_ent
     static const cudaError_t attr = cudaFuncSetAttribute(
         accumulate_numerators_split_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ACC_DYN_SMEM);
     GS_CUDA_TRY(attr);
-    accumulate_numerators_split_kernel<1><<<grid, 256, ACC_DYN_SMEM, st>>>((const NumEntry*)d_entries, n_entries,
-                                                                         b_sum, log_size, out, d_bsum);
+    launch_after(accumulate_numerators_split_kernel<1>, grid, 256, ACC_DYN_SMEM, st, (const NumEntry*)d_entries,
+                 n_entries, b_sum, log_size, out, d_bsum);
   } else if (R == 4)
     accumulate_numerators_kernel<4><<<(unsigned)blocks, threads, 0, st>>>((const NumEntry*)d_entries, n_entries,
                                                                          b_sum, log_size, out, d_bsum);
@@ -283,6 +284,7 @@ __global__ void __launch_bounds__(512) quot_line_coeffs_kernel(const LineTerm* _
                                                                const uint32_t* batch_point, uint32_t n_batches,
                                                                uint32_t* bsums, QuotAcc* accs, uint32_t n_points,
                                                                uint32_t* scratch) {
+  after_previous(terms, vals, points);
   __shared__ qm31 asum[QUOT_MAX_BATCHES];
   for (uint32_t i = threadIdx.x; i < n_terms; i += blockDim.x) {
     const LineTerm t = terms[i];
@@ -336,8 +338,8 @@ int quot_line_coeffs(cudaStream_t st, const LineTerm* d_terms, uint32_t n_terms,
   GS_REQUIRE(n_batches <= QUOT_MAX_BATCHES && n_points <= QUOT_MAX_POINTS, "too many quotient batches or points");
   GS_REQUIRE(n_terms == 0 || (d_terms && d_vals && d_points && d_entries && d_scratch), "null buffer");
   GS_REQUIRE(d_batch_first && d_batch_point && d_bsums && d_accs, "null buffer");
-  quot_line_coeffs_kernel<<<1, 512, 0, st>>>(d_terms, n_terms, d_vals, d_points, alpha, d_entries, d_batch_first,
-                                             d_batch_point, n_batches, d_bsums, d_accs, n_points, d_scratch);
+  launch_after(quot_line_coeffs_kernel, 1, 512, 0, st, d_terms, n_terms, d_vals, d_points, alpha, d_entries,
+               d_batch_first, d_batch_point, n_batches, d_bsums, d_accs, n_points, d_scratch);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;
@@ -349,6 +351,7 @@ constexpr int QUOT_MAXK = 4;   // sample points per inversion chunk
 
 __global__ void __launch_bounds__(128) quotients_kernel(const QuotAcc* __restrict__ accs, uint32_t n_accs,
                                                         DomainTables dt, Planes out) {
+  after_previous(accs, dt);
   const size_t n = (size_t)1 << dt.lift;
   const size_t n_groups = n / QUOT_ROWS;
   for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < n_groups; g += (size_t)gridDim.x * blockDim.x) {
@@ -452,7 +455,7 @@ int compute_quotients_and_combine(cudaStream_t st, const void* d_accs, uint32_t 
   size_t blocks = (groups + threads - 1) / threads;
   size_t cap = (size_t)num_sms() * 16;
   if (blocks > cap) blocks = cap;
-  quotients_kernel<<<(unsigned)blocks, threads, 0, st>>>((const QuotAcc*)d_accs, n_accs, dt, out);
+  launch_after(quotients_kernel, (unsigned)blocks, threads, 0, st, (const QuotAcc*)d_accs, n_accs, dt, out);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;

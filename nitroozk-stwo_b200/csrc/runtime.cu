@@ -345,6 +345,7 @@ int Context::read_buffer(size_t bytes, void** out) {
 // Device words into mapped pinned memory: 16-byte stores where source and
 // destination allow, single words for the rest.
 __global__ void publish_kernel(const uint32_t* __restrict__ src, uint32_t* dst, size_t n_words) {
+  after_previous(src);
   const size_t n16 = n_words / 4;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   const size_t t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -363,7 +364,7 @@ int Context::publish(const void* d_src, size_t bytes, const void** host) {
     const size_t cap = (size_t)num_sms() * 4;
     if (blocks > cap) blocks = cap;
     if (blocks == 0) blocks = 1;
-    publish_kernel<<<(unsigned)blocks, 256, 0, stream>>>((const uint32_t*)d_src, (uint32_t*)d_read, bytes / 4);
+    launch_after(publish_kernel, (unsigned)blocks, 256, 0, stream, (const uint32_t*)d_src, (uint32_t*)d_read, bytes / 4);
     note_launch();
     GS_CUDA_TRY(cudaGetLastError());
   } else if (bytes) {

@@ -102,18 +102,32 @@ __device__ __forceinline__ void bfly(uint32_t& a, uint32_t& b, uint32_t w) {
   }
 }
 
-// The same with the twiddle already doubled.
-template <bool INV>
-__device__ __forceinline__ void bfly_b2(uint32_t& a, uint32_t& b, uint32_t w2) {
-  if (INV) {
-    uint32_t t0 = a;
-    a = add(t0, b);
-    b = mul_b2(sub(t0, b), w2);
-  } else {
-    uint32_t t0 = mul_b2(b, w2);
-    b = sub(a, t0);
-    a = add(a, t0);
-  }
+// Butterflies with one reduction less than three: on centred twiddles (s = 2w,
+// less 2p where w > p/2: an even word in [2 - p, p - 1] as a signed one) the
+// product of a signed b in [-p, p] comes out as t = b w (mod p) in [-p, p - 1]
+// without any: b s + 2^31 - 2^62 has the high word b w / 2^31, rounded, less
+// 2^30, and the low word half of which is the rest, plus 2^30.
+__host__ __device__ __forceinline__ uint32_t centred2(uint32_t w) { return 2u * (w + (w >> 30)); }
+__device__ __forceinline__ uint32_t mul_centred(uint32_t b, uint32_t s) {
+  const int64_t p = (int64_t)(int32_t)b * (int32_t)s + ((1ll << 31) - (1ll << 62));
+  return (uint32_t)((uint64_t)p >> 32) + ((uint32_t)p >> 1);
+}
+// Inverse, a and b canonical before and after: a - b needs no reduction.
+__device__ __forceinline__ void bfly_inv(uint32_t& a, uint32_t& b, uint32_t s) {
+  const uint32_t t = mul_centred(a - b, s);
+  a = add(a, b);
+  b = __viaddmin_u32(t, P, t);
+}
+// Forward: t goes to [-p, -1] and a to [0, p - 1], one step each, so that a + t
+// is a signed word in [-p, p - 2] and a - t an unsigned one in [1, 2p - 1]. The
+// next layer is told which of the two forms its operands have.
+template <bool UNSIGNED>
+__device__ __forceinline__ void bfly_fwd(uint32_t& a, uint32_t& b, uint32_t s) {
+  uint32_t t = mul_centred(UNSIGNED ? b - P : b, s);
+  t = __viaddmax_u32(t, 0u - P, t);
+  const uint32_t r = __viaddmin_u32(a, UNSIGNED ? 0u - P : P, a);
+  a = r + t;
+  b = r - t;
 }
 
 // XOR swizzle over the block's shared-memory index (tile offset included, so
@@ -345,7 +359,7 @@ __global__ void __launch_bounds__(256) fft_tile_kernel(Cols src_tab, MutCols dst
 // warps wait for the tile's loads. So a block fixes the part of the index
 // that selects twiddles and walks the columns (and, in a strided pass, the
 // tiles) that share it:
-//  * the twiddles, already doubled for mul_b2, sit in shared memory, built once
+//  * the twiddles, centred and doubled for mul_centred, sit in shared memory, built once
 //    per block: layer section of size s at [s, 2s), so a thread's 2^k
 //    consecutive twiddles are 16-byte shared loads at offsets computed once;
 //  * the next tile arrives by 16-byte cp.async while the current one is in its
@@ -362,9 +376,11 @@ __global__ void __launch_bounds__(256) fft_tile_kernel(Cols src_tab, MutCols dst
 // threads read and write 32 consecutive words as 16-byte vectors; e + e / 32
 // in the second buffer.
 // Extension of 158 columns, 2^18 coefficients to 2^20 points: 740 us in 9 + 9
-// layers through fft_tile_kernel, 593 us in 8 + 10 here (8.9 against 11.2
-// instructions per butterfly); interpolation 198 -> 167 us. The extension's
-// memory traffic alone, without a butterfly, takes 400 of the 593.
+// layers through fft_tile_kernel, 588 us in 8 + 10 here with three reductions
+// per butterfly (8.9 against 11.2 instructions), 562 us with two;
+// interpolation 198 -> 166 -> 150 us. The extension's memory traffic alone,
+// without a butterfly, takes 400 us, the integer ALU pipe's share (three
+// two-cycle instructions per butterfly) 240 us: they overlap in part only.
 // ---------------------------------------------------------------------------
 template <bool INV, int C>
 __device__ __host__ constexpr uint32_t in_pad(uint32_t e) {
@@ -429,19 +445,19 @@ __global__ void __launch_bounds__(1 << (TB - 5), (StreamShape<INV, L, C, TB>::PE
   // the next tile's column, one tile ahead of its copies
   const uint32_t* next_src = unit + g.group < g.units ? src_tab[(unit + g.group) >> mid_bits] : nullptr;
 
-  // the block's twiddles, doubled
+  // the block's twiddles, centred and doubled
   if (C > 0) {
     for (uint32_t i = tid; i < (1u << L); i += THREADS) {
       if (i == 0) continue;
       const uint32_t lg = 31 - __clz(i);  // section of 2^lg twiddles: layer lo + L - 1 - lg
-      tab[i] = __ldg(tw + (a.tw_len - (1u << (a.n - a.lo - (L - 1) + lg))) + (set << lg) + (i - (1u << lg))) << 1;
+      tab[i] = centred2(__ldg(tw + (a.tw_len - (1u << (a.n - a.lo - (L - 1) + lg))) + (set << lg) + (i - (1u << lg))));
     }
   } else {
     // layers 1 .. L - 1; the circle layer 0 takes its twiddles from layer 1's
     for (uint32_t i = tid; i < (1u << (TB - 1)); i += THREADS) {
       if (i < (1u << (TB - L))) continue;
       const uint32_t lg = 31 - __clz(i);  // layer TB - 1 - lg
-      tab[i] = __ldg(tw + (a.tw_len - (1u << (a.n - (TB - 1) + lg))) + (set << lg) + (i - (1u << lg))) << 1;
+      tab[i] = centred2(__ldg(tw + (a.tw_len - (1u << (a.n - (TB - 1) + lg))) + (set << lg) + (i - (1u << lg))));
     }
   }
 
@@ -507,10 +523,10 @@ __global__ void __launch_bounds__(1 << (TB - 5), (StreamShape<INV, L, C, TB>::PE
             w1[4] = v.x; w1[5] = v.y; w1[6] = v.z; w1[7] = v.w;
           }
 #pragma unroll
-          for (int q = 0; q < 4; q++) {  // [y, -y, -x, x], doubled: 2 (p - w) = 2p - 2w
+          for (int q = 0; q < 4; q++) {  // [y, -y, -x, x]
             w[4 * q] = w1[2 * q + 1];
-            w[4 * q + 1] = 2u * P - w1[2 * q + 1];
-            w[4 * q + 2] = 2u * P - w1[2 * q];
+            w[4 * q + 1] = 0u - w1[2 * q + 1];
+            w[4 * q + 2] = 0u - w1[2 * q];
             w[4 * q + 3] = w1[2 * q];
           }
         } else if (C == 0 && layer == 1 && INV) {
@@ -539,9 +555,17 @@ __global__ void __launch_bounds__(1 << (TB - 5), (StreamShape<INV, L, C, TB>::PE
 #pragma unroll
         for (int q = 0; q < NQ; q++) {
           if (q & (1 << j)) continue;
-          bfly_b2<INV>(x[q], x[q | (1 << j)], w[q >> (j + 1)]);
+          if (INV) bfly_inv(x[q], x[q | (1 << j)], w[q >> (j + 1)]);
+          else if (j + 1 < jb && (q >> (j + 1)) & 1) bfly_fwd<true>(x[q], x[q | (1 << j)], w[q >> (j + 1)]);
+          else bfly_fwd<false>(x[q], x[q | (1 << j)], w[q >> (j + 1)]);
         }
       }
+      // a stage ends with layer j = 0 of its window: signed words go on to the
+      // next stage, canonical ones to memory
+      if (!INV)
+#pragma unroll
+        for (int q = 0; q < NQ; q++)
+          x[q] = k + 1 == K ? __viaddmin_u32(x[q], q & 1 ? 0u - P : P, x[q]) : q & 1 ? x[q] - P : x[q];
       if (k + 1 < K) {
         if (INV && C == 0 && k == 0) {
           uint4* p = reinterpret_cast<uint4*>(in + in_pad<INV, C>(ebase));

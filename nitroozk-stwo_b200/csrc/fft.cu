@@ -377,10 +377,11 @@ __global__ void __launch_bounds__(256) fft_tile_kernel(Cols src_tab, MutCols dst
 // in the second buffer.
 // Extension of 158 columns, 2^18 coefficients to 2^20 points: 740 us in 9 + 9
 // layers through fft_tile_kernel, 588 us in 8 + 10 here with three reductions
-// per butterfly (8.9 against 11.2 instructions), 562 us with two;
-// interpolation 198 -> 166 -> 150 us. The extension's memory traffic alone,
-// without a butterfly, takes 400 us, the integer ALU pipe's share (three
-// two-cycle instructions per butterfly) 240 us: they overlap in part only.
+// per butterfly (8.9 against 11.2 instructions), 562 us with two, 553 us with
+// stepped addresses in the strided pass; interpolation 198 -> 166 -> 148 us. The extension's memory traffic alone,
+// without a butterfly, takes 400 us, the integer ALU pipe's share (4.2
+// two-cycle instructions per butterfly, 3 of them in it) 330 us: they overlap
+// in part only.
 // ---------------------------------------------------------------------------
 template <bool INV, int C>
 __device__ __host__ constexpr uint32_t in_pad(uint32_t e) {
@@ -432,12 +433,17 @@ __global__ void __launch_bounds__(1 << (TB - 5), (StreamShape<INV, L, C, TB>::PE
   };
   auto issue = [&](uint32_t u, const uint32_t* src) {
     const uint32_t base = tile_base(u);
+    // a strided pass's rows lie below the coefficients' size: the mask cuts the
+    // tile's base alone, and the row steps are pointer steps
+    const uint32_t e0 = 4 * tid;
+    const uint32_t* p = src + ((base & a.src_mask) | ((e0 >> C) << a.lo) | (e0 & CMASK));
+    const size_t step = (size_t)(4 * THREADS >> C) << a.lo;
 #pragma unroll
     for (int q = 0; q < 8; q++) {
-      const uint32_t e = 4 * tid + 4 * THREADS * q;
-      const uint32_t v = base | (C > 0 ? ((e >> C) << a.lo) | (e & CMASK) : e);
       const uint32_t d = (uint32_t)__cvta_generic_to_shared(in + in_pad<INV, C>(4 * tid) + in_pad<INV, C>(4 * THREADS * q));
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + (v & a.src_mask)) : "memory");
+      if (C == 0) p = src + ((base | (e0 + 4 * THREADS * q)) & a.src_mask);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(p) : "memory");
+      if (C > 0) p += step;
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -600,12 +606,18 @@ __global__ void __launch_bounds__(1 << (TB - 5), (StreamShape<INV, L, C, TB>::PE
           const uint32_t e = 4 * tid + 4 * THREADS * q;
           d[tid + THREADS * q] = *reinterpret_cast<const uint4*>(ex + e + 4 * (e >> 5));
         }
-      } else {
-        const uint32_t v = tile_base(unit) | (C > 0 ? ((ebase >> C) << a.lo) | (ebase & CMASK) : ebase);
-        uint32_t* p0 = dst + v;
-        const uint32_t stride = C > 0 ? 1u << (s0 - C + a.lo) : 1u << s0;
+      } else if (C > 0) {
+        // byte offsets in 32 bits (columns of up to 2^30 words), stepped by a
+        // two-input add: 64-bit addresses cost two ALU instructions a word
+        uint32_t at = 4u * (tile_base(unit) | ((ebase >> C) << a.lo) | (ebase & CMASK));
+        const uint32_t step = 4u << (s0 - C + a.lo);
+        char* const d = reinterpret_cast<char*>(dst);
 #pragma unroll
-        for (int q = 0; q < NQ; q++) p0[(size_t)q * stride] = x[q];
+        for (int q = 0; q < NQ; q++, at += step) *reinterpret_cast<uint32_t*>(d + at) = x[q];
+      } else {
+        uint32_t* p0 = dst + (tile_base(unit) | ebase);
+#pragma unroll
+        for (int q = 0; q < NQ; q++) p0[(size_t)q << s0] = x[q];
       }
     }
   }

@@ -120,3 +120,73 @@ def test_stream_pass_twiddle_sections(n, lo, L, C, TB):
         some = [(s << (lo + L)) | (m << C) | (row << lo) for s in {0, n_sets - 1} for m in {0, mids - 1}]
         assert max(x.max() for x in some) + (1 << C) <= 1 << n
         assert all(np.all(x % 4 == 0) for x in some)
+
+
+@pytest.mark.parametrize("L,C,TB", STRIDED)
+@pytest.mark.parametrize("ext", [0, 1, 3])
+def test_stream_pass_addresses_step(L, C, TB, ext):
+    """Row steps from one address, the mask on the tile's base alone, give the
+    masked word of every 16-byte load; byte offsets of the stores fit 32 bits."""
+    threads = 1 << (TB - 5)
+    tid = np.arange(threads)
+    for lo in {C, C + 1, 13, 30 - ext - L}:
+        coeff, n = lo + L, lo + L + ext
+        mask = (1 << coeff) - 1
+        sets, mids = 1 << ext, 1 << (lo - C)
+        for st in {0, sets - 1}:
+            for mid in {0, mids - 1}:
+                base = (st << (lo + L)) | (mid << C)
+                e0 = 4 * tid
+                p = (base & mask) | ((e0 >> C) << lo) | (e0 & ((1 << C) - 1))
+                for k in range(8):
+                    e = e0 + 4 * threads * k
+                    v = base | ((e >> C) << lo) | (e & ((1 << C) - 1))
+                    assert np.array_equal(v & mask, p + k * ((4 * threads >> C) << lo))
+                for s0, _, _ in (stages(False, L, C, TB)[-1], stages(True, L, C, TB)[-1]):
+                    ebase = ((tid >> s0) << (s0 + R)) | (tid & ((1 << s0) - 1))
+                    at = 4 * (base | ((ebase >> C) << lo) | (ebase & ((1 << C) - 1)))
+                    for k in range(NQ):
+                        e = ebase | (k << s0)
+                        v = base | ((e >> C) << lo) | (e & ((1 << C) - 1))
+                        assert np.array_equal(at + k * (4 << (s0 - C + lo)), 4 * v) and v.max() < 1 << n
+                        assert 4 * v.max() < 1 << 32
+
+
+def test_butterflies_on_centred_twiddles():
+    """bfly_fwd / bfly_inv in 32-bit words at the edges of their ranges and at
+    random: both forms of the operands, results within their ranges and equal
+    to the butterfly mod p."""
+    P, M = 2**31 - 1, 2**32
+    edge = np.array([0, 1, 2, P - 1, P - 2, 2**30, 2**30 - 1, 2**30 + 1, 2**16], dtype=object)
+    rng = np.random.default_rng(3)
+    rand = np.array([int(v) for v in rng.integers(0, P, 9)], dtype=object)
+    vals = np.concatenate([edge, rand])
+    a, b, w = (g.ravel() for g in np.meshgrid(vals, vals, vals, indexing="ij"))
+    signed = lambda x: np.where(x >= M // 2, x - M, x)
+
+    def mul_centred(x, s):
+        p = signed(x) * signed(s) + 2**31 - 2**62
+        assert p.min() >= -2**63 and p.max() < 2**63
+        p = p % 2**64
+        return ((p >> 32) + (p % M >> 1)) % M
+
+    s = 2 * (w + (w >> 30)) % M
+    add_min = lambda x, c: np.minimum((x + c) % M, x)
+    add_max = lambda x, c: np.maximum((x + c) % M, x)
+    t = mul_centred((a - b) % M, s)
+    assert np.array_equal(add_min(t, P), (a - b) * w % P)
+    for unsigned in (False, True):
+        # the same residues in the form's range: [-p, p - 1] or [1, 2p - 1]
+        forms = [lambda x: x, lambda x: x - P] if not unsigned else [lambda x: np.where(x > 0, x, P), lambda x: x + P]
+        for fa in forms:
+            for fb in forms:
+                x, y = fa(a) % M, fb(b) % M
+                t = mul_centred((y - P) % M if unsigned else y, s)
+                assert signed(t).min() >= -P and signed(t).max() < P
+                t = add_max(t, -P)
+                r = add_min(x, -P if unsigned else P)
+                assert signed(t).max() < 0 and r.max() < P
+                lo, hi = (r + t) % M, (r - t) % M
+                assert signed(lo).min() >= -P and signed(lo).max() < P and hi.min() >= 1 and hi.max() < 2 * P
+                assert np.array_equal(add_min(lo, P), (a + b * w) % P)
+                assert np.array_equal(add_min(hi, -P), (a - b * w) % P)

@@ -613,7 +613,7 @@ def proof_roofline(args, log_n, wl, ctx, clk=None):
             inst = recs.get("inst_lde_%s_%d" % (wl, log_n))
         except Exception:
             traffic = inst = None
-    out = {"kernel": "fft_tile_kernel (LDE %d cols 2^%d -> 2^%d, 2 launches)" % (cols, log_n, target), "bound": "hbm",
+    out = {"kernel": "fft_stream_kernel (LDE %d cols 2^%d -> 2^%d, 2 launches)" % (cols, log_n, target), "bound": "hbm",
            "achieved": round(achieved, 1), "peak": hbm_peak, "peak_kind": peak_kind, "unit": "GB/s",
            "frac": round(achieved / hbm_peak, 4), "traffic": traffic, "algorithmic_bytes": alg,
            "avg_ms": round(ms, 4)}

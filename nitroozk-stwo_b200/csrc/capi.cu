@@ -406,12 +406,32 @@ int gs_batch_eval_at_point(gs_ctx* ctx, const uint32_t* const* polys, uint32_t n
   for (uint32_t i = 0; i < n_polys; i++) vec = vec && ((uintptr_t)polys[i] & 15) == 0;
   GS_TRY(batch_eval_at_point(ctx->c.stream, c, n_polys, log_size, p, d_out, (uint32_t*)scratch,
                              12, vec));
-  GS_CUDA_TRY(cudaMemcpyAsync(out, d_out, 16 * (size_t)n_polys, cudaMemcpyDeviceToHost, ctx->c.stream));
-  GS_CUDA_TRY(cudaStreamSynchronize(ctx->c.stream));
-  return OK;
+  return ctx->c.read_back_published(d_out, 16 * (size_t)n_polys, out);
 }
 
 // ------------------------------------------------------ per-trait operations
+// Where a gather stores: the context's mapped read buffer, up to the size that
+// it starts with, else scratch that is copied back (as it is where host memory
+// cannot be mapped). Stored in place, 1 MiB takes 125 us a call against 141.
+struct GatherTarget {
+  void *dev = nullptr, *host = nullptr;
+  size_t bytes = 0;
+  int open(Context& c, size_t n) {
+    bytes = n;
+    if (n <= (1u << 20)) {
+      GS_TRY(c.read_buffer(n, &host));
+      dev = c.d_read;
+    }
+    return dev ? OK : c.get_scratch(n, &dev);
+  }
+  int read(Context& c, void* out) const {
+    if (dev != c.d_read) return c.read_back(dev, bytes, out);
+    GS_TRY(stream_sync(c.stream));
+    memcpy(out, host, bytes);
+    return OK;
+  }
+};
+
 int gs_batch_gather_multi_uint32(gs_ctx* ctx, const uint32_t* const* cols, uint32_t n_cols, size_t col_len,
                                  const uint32_t* indices, uint32_t n_indices, uint32_t* out) {
   CTX_REQUIRED(ctx);
@@ -424,12 +444,11 @@ int gs_batch_gather_multi_uint32(gs_ctx* ctx, const uint32_t* const* cols, uint3
   const void* d_idx = nullptr;
   GS_TRY(ctx->c.stage_ptrs((const void* const*)cols, n_cols, &d_cols));
   GS_TRY(ctx->c.stage_bytes(indices, 4 * (size_t)n_indices, &d_idx));
-  size_t bytes = 4 * (size_t)n_cols * n_indices;
-  void* d_out = nullptr;
-  GS_TRY(ctx->c.get_scratch(bytes, &d_out));
+  GatherTarget to;
+  GS_TRY(to.open(ctx->c, 4 * (size_t)n_cols * n_indices));
   GS_TRY(gather_multi(ctx->c.stream, (const uint32_t* const*)d_cols, n_cols, (const uint32_t*)d_idx, n_indices,
-                      (uint32_t*)d_out));
-  return ctx->c.read_back(d_out, bytes, out);
+                      (uint32_t*)to.dev));
+  return to.read(ctx->c, out);
 }
 
 int gs_batch_get_blake2s_hash(gs_ctx* ctx, const uint32_t* layer, size_t n_hashes, const uint32_t* indices,
@@ -440,12 +459,13 @@ int gs_batch_get_blake2s_hash(gs_ctx* ctx, const uint32_t* layer, size_t n_hashe
   GS_REQUIRE(((uintptr_t)layer & 15) == 0, "hash layer must be 16-byte aligned");
   for (uint32_t i = 0; i < n_indices; i++) GS_REQUIRE(indices[i] < n_hashes, "hash index out of range");
   const void* d_idx = nullptr;
-  GS_TRY(ctx->c.stage_bytes(indices, 4 * (size_t)n_indices, &d_idx));
-  size_t bytes = 32 * (size_t)n_indices;
-  void* d_out = nullptr;
-  GS_TRY(ctx->c.get_scratch(bytes, &d_out));
-  GS_TRY(gather_hashes(ctx->c.stream, layer, (const uint32_t*)d_idx, n_indices, (uint32_t*)d_out));
-  return ctx->c.read_back(d_out, bytes, out);
+  FewIndices few{};
+  if (n_indices <= sizeof(few.v) / 4) memcpy(few.v, indices, 4 * (size_t)n_indices);
+  else GS_TRY(ctx->c.stage_bytes(indices, 4 * (size_t)n_indices, &d_idx));
+  GatherTarget to;
+  GS_TRY(to.open(ctx->c, 32 * (size_t)n_indices));
+  GS_TRY(gather_hashes(ctx->c.stream, layer, (const uint32_t*)d_idx, few, n_indices, (uint32_t*)to.dev));
+  return to.read(ctx->c, out);
 }
 
 int gs_barycentric_weights(gs_ctx* ctx, uint32_t log_size, gs_point_qm31 point, uint32_t* const weights[4]) {

@@ -446,7 +446,10 @@ int secure_powers(cudaStream_t st, qm31 felt, size_t n, Planes out);
 // gather.cu: Column::batch_at_multi (row-major) and hashes of one layer
 int gather_multi(cudaStream_t st, const uint32_t* const* d_cols, uint32_t n_cols, const uint32_t* d_idx,
                  uint32_t n_idx, uint32_t* d_out);
-int gather_hashes(cudaStream_t st, const uint32_t* d_layer, const uint32_t* d_idx, uint32_t n_idx, uint32_t* d_out);
+// d_idx null: the indices of `few`.
+struct FewIndices { uint32_t v[16]; };
+int gather_hashes(cudaStream_t st, const uint32_t* d_layer, const uint32_t* d_idx, const FewIndices& few,
+                  uint32_t n_idx, uint32_t* d_out);
 
 // grind.cu
 // hi0: the first high word searched (a search whose chunk hi = 0 already ran

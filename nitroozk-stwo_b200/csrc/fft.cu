@@ -731,10 +731,11 @@ static void split_layers(uint32_t layers, FftTuning tn, std::vector<std::pair<ui
 // best for each size. Fewest passes, then fewest register stages
 // (of up to 5 layers), then the wider rows of 12/5 (whole 128-byte lines).
 // 13/4, whose strided passes hold 9 layers in tiles of 2^13, only where it
-// saves a pass: 9 + 9 layers measured 345 + 193 us (extension by 2 and
-// interpolation of 158 columns of 2^18: 638 + 194), 10 + 8 (12/4) 328 + 177
-// (600 + 176); 2^19, 12 + 7 (12/5) 280 + 155 against 290 + 162 for 10 + 9;
-// 2^22, 13 + 9 345 + 178 against three passes' 387 + 256.
+// saves a pass. Measured with fft_stream_kernel and butterflies of three
+// reductions: 158 columns of 2^18 extended by 2 and interpolated, 9 + 9 layers
+// (13/4) 625 + 171 us, 10 + 8 (12/4) 589 + 166; eight columns of 2^22, 13 + 9
+// 341 + 173 against three passes' 366 + 248. 2^19, with an earlier form of it,
+// 12 + 7 (12/5) 280 + 155 against 290 + 162 for 10 + 9.
 static FftTuning default_tuning(uint32_t layers) {
   FftTuning best{13, 4};
   size_t best_passes = 99, best_stages = 0;

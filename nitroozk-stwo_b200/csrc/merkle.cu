@@ -279,8 +279,9 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(1024) merkle_tail_ke
 struct TreePtrs { uint32_t* p[TREE_MAX_LOG + 1]; };
 // Threads per 512-child unit: 128, each hashing two nodes of the unit's first
 // level (452 us of tree kernels per Poseidon2 2^18 proof, against 464 us
-// with 256 threads and 568 us with 64): half the warps wait at the barriers
-// of the upper levels, and twice as many units fit on an SM.
+// with 256 threads and 568 us with 64, all with a thread per node): half the
+// warps wait at the barriers of the upper levels, and twice as many units fit
+// on an SM.
 constexpr int TREE_THREADS = 128;
 
 template <int U, int TH>

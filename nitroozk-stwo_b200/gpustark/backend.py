@@ -9,8 +9,10 @@ are lists of 4 such tensors (coordinate planes); a hash layer is an int32
 tensor of 8 words per node. Every call enqueues on the context's stream,
 which is torch's current stream unless another is given.
 """
+import array
 import ctypes as C
 import hashlib
+import itertools
 import struct
 from dataclasses import dataclass
 
@@ -75,6 +77,26 @@ def qm31(v):
     return L.QM31(*v)
 
 
+def _integer_words(values):
+    """A list of rows of 4 integers as an array of words, mod 2^32 as in a
+    ctypes field; None for rows of other lengths or values of other types,
+    which a conversion per value takes or refuses. Of integers alone: numpy
+    turns NaN, infinities and complex numbers into integers, int() does not."""
+    try:
+        if isinstance(values[0], np.ndarray):
+            a = np.array(values)
+            if a.dtype.kind not in "biu" or a.shape != (len(values), 4):
+                return None
+        elif set(map(len, values)) == {4}:
+            a = np.frombuffer(array.array("q", list(itertools.chain.from_iterable(values))), np.int64)
+            a = a.reshape(-1, 4)
+        else:
+            return None
+    except Exception:
+        return None
+    return a.astype(np.uint32)
+
+
 def qm31_array(values, n=None):
     """QM31 values (4 ints each) as a host array of n gs_qm31, zeros after the
     last: (address, array to keep alive)."""
@@ -84,15 +106,11 @@ def qm31_array(values, n=None):
         raise ValueError(f"{len(values)} values for {n} places")
     out = np.zeros((max(n, 1), 4), np.uint32)
     if values:
-        try:  # one conversion for the whole list; words wrap mod 2^32, as in a ctypes field
-            a = np.array(values, dtype=np.int64)
-        except (OverflowError, TypeError, ValueError):
-            a = None
-        if a is not None and a.shape == (len(values), 4):
-            out[:len(values)] = a.astype(np.uint32)
-        else:
+        words = _integer_words(values)
+        if words is None:
             arr = (L.QM31 * len(values))(*[qm31(v) for v in values])
-            out[:len(values)] = np.frombuffer(arr, np.uint32).reshape(-1, 4)
+            words = np.frombuffer(arr, np.uint32).reshape(-1, 4)
+        out[:len(values)] = words
     return out.ctypes.data, out
 
 

@@ -123,7 +123,14 @@ _MERKLE_ITEM = np.dtype([("cols", "u8"), ("n_cols", "u4"), ("log_size", "u4"), (
 _ONE_BUFFER_TREE_LOG = 10
 
 
+def _log_word(t):
+    """The tensor's log size as a C word: 2^32 - 1, which the library refuses, where it has no words."""
+    return (t.numel().bit_length() - 1) & 0xFFFFFFFF
+
+
 def _tree_layers(log):
+    if log > 31:  # no size at all (_log_word)
+        return []
     if log > _ONE_BUFFER_TREE_LOG:
         return [torch.empty(8 << lg, dtype=torch.int32, device="cuda") for lg in range(log + 1)]
     sizes = [8 << lg for lg in range(log + 1)]
@@ -202,8 +209,8 @@ class GpuBackend:
         if items:
             arr["src"] = [src.data_ptr() for _, src, _ in items]
             arr["dst"] = [dst.data_ptr() for _, _, dst in items]
-            arr["log_size"] = [dst.numel().bit_length() - 1 for _, _, dst in items]
-            arr["coeffs_log_size"] = [src.numel().bit_length() - 1 for _, src, _ in items]
+            arr["log_size"] = [_log_word(dst) for _, _, dst in items]
+            arr["coeffs_log_size"] = [_log_word(src) for _, src, _ in items]
             arr["inverse"] = [kind == "interpolate" for kind, _, _ in items]
         L.check(L.lib().gs_fft_worklist(ctx.handle, arr.ctypes.data, len(items), _p(twiddles.twiddles), _p(twiddles.itwiddles),
                                         twiddles.root_log), "fft_worklist")
@@ -275,7 +282,7 @@ class GpuBackend:
         trees: lists of columns (tensors of 2^log words each, at least one per
         tree); returns per tree its layers, layers[L] of 2^L x 8 words."""
         ctx = ctx or default_context()
-        logs = [cols[0].numel().bit_length() - 1 for cols in trees]
+        logs = [_log_word(cols[0]) for cols in trees]
         out = [_tree_layers(log) for log in logs]
         ptrs, at = [], []  # every tree's column and layer pointers in one array; where they start
         for cols, layers in zip(trees, out):

@@ -45,3 +45,42 @@ def test_qm31_array_equals_one_conversion_per_value(k):
         _, got = backend.qm31_array(vals, len(vals) + 2)
         assert got.shape == (len(vals) + 2, 4) and not got[len(vals):].any()
         assert np.array_equal(got[:len(vals)], want)
+
+
+class _Library:
+    """Stands for the C library: keeps what a call was given."""
+
+    def __init__(self, name, types):
+        self.args = None
+
+        def call(*args):
+            self.args = [t(a) if t else a for t, a in zip(types, args)]
+            return 0
+
+        setattr(self, name, call)
+
+
+class _Context:
+    handle = None
+
+
+def _host_tensors(monkeypatch):
+    empty = torch.empty
+    monkeypatch.setattr(backend.torch, "empty", lambda *a, device=None, **k: empty(*a, **k))
+
+
+def test_worklist_sizes_reach_the_library_as_they_are(monkeypatch):
+    """A tensor of no words has no log size; the library refuses it (2^32 - 1)."""
+    _host_tensors(monkeypatch)
+    some, none = torch.zeros(8, dtype=torch.int32), torch.zeros(0, dtype=torch.int32)
+    tw = backend.TwiddleTree(3, some, some)
+    lib = _Library("gs_fft_worklist", [None, lambda a: np.ctypeslib.as_array(
+        backend.C.cast(a, backend.C.POINTER(backend.C.c_uint32)), (16,)).copy()])
+    monkeypatch.setattr(L, "lib", lambda: lib)
+    backend.GpuBackend.fft_worklist([("interpolate", some, none), ("evaluate", none, some)], tw, ctx=_Context())
+    assert list(lib.args[1][4:7]) == [2**32 - 1, 3, 1] and list(lib.args[1][12:15]) == [3, 2**32 - 1, 0]
+    lib = _Library("gs_merkle_worklist", [None, lambda a: np.ctypeslib.as_array(
+        backend.C.cast(a, backend.C.POINTER(backend.C.c_uint32)), (12,)).copy()])
+    layers = backend.GpuBackend.merkle_worklist([[some, some], [none]], ctx=_Context())
+    assert list(lib.args[1][2:4]) == [2, 3] and list(lib.args[1][8:10]) == [1, 2**32 - 1]
+    assert [len(x) for x in layers] == [4, 0]

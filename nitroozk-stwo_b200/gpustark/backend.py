@@ -365,7 +365,7 @@ class GpuBackend:
         out = [torch.empty(1 << log_size, dtype=torch.int32, device="cuda") for _ in range(4)]
         cp, k1 = L.ptr_array([c.data_ptr() for c in columns])
         n = len(column_indices)
-        idx = np.array([int(i) for i in column_indices] or [0], dtype=np.int64).astype(np.uint32)
+        idx = np.array([int(i) & 0xFFFFFFFF for i in column_indices] or [0], dtype=np.uint32)
         bs, kb = qm31_array(line_coeffs_b, n)
         cs, kc = qm31_array(line_coeffs_c, n)
         op, k2 = L.ptr_array([t.data_ptr() for t in out])

@@ -84,3 +84,13 @@ def test_worklist_sizes_reach_the_library_as_they_are(monkeypatch):
     layers = backend.GpuBackend.merkle_worklist([[some, some], [none]], ctx=_Context())
     assert list(lib.args[1][2:4]) == [2, 3] and list(lib.args[1][8:10]) == [1, 2**32 - 1]
     assert [len(x) for x in layers] == [4, 0]
+
+
+def test_column_indices_wrap_as_a_ctypes_word(monkeypatch):
+    _host_tensors(monkeypatch)
+    indices = [0, -1, 2**32 + 1, 2**63, -2**70 + 5, np.int64(3)]
+    lib = _Library("gs_accumulate_numerators", [None] * 4 + [lambda a: [a[k] for k in range(len(indices))]])
+    monkeypatch.setattr(L, "lib", lambda: lib)
+    cols = [torch.zeros(8, dtype=torch.int32)]
+    backend.GpuBackend.accumulate_numerators(cols, 3, indices, [[0] * 4] * 6, [[0] * 4] * 6, ctx=_Context())
+    assert lib.args[4] == [backend.C.c_uint32(int(i)).value for i in indices]

@@ -835,9 +835,8 @@ template <bool INV, int L, int C, int TB>
 static int launch_stream(cudaStream_t st, uint32_t n_cols, Cols s, MutCols d,
                          const uint32_t* tw, const FftPass& a) {
   using Shape = StreamShape<INV, L, C, TB>;
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      fft_stream_kernel<INV, L, C, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape::SMEM);
-  GS_CUDA_TRY(attr);
+  static OncePerDevice smem;
+  GS_CUDA_TRY(allow_smem(smem, fft_stream_kernel<INV, L, C, TB>, Shape::SMEM));
   StreamGrid g;
   g.set_log = C > 0 ? a.n - a.lo - L : a.n - TB;
   g.units = C > 0 ? n_cols << (a.lo - C) : n_cols;
@@ -1094,9 +1093,8 @@ int fft_worklist(Context& ctx, const FftItem* items, uint32_t n_items, const uin
     d = owned;
   }
   const size_t smem = (size_t)4 << wl.front().log;
-  static const cudaError_t attr = cudaFuncSetAttribute(fft_worklist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       4 << FFT_WL_MAX_LOG);
-  GS_CUDA_TRY(attr);
+  static OncePerDevice limit;
+  GS_CUDA_TRY(allow_smem(limit, fft_worklist_kernel, (size_t)4 << FFT_WL_MAX_LOG));
   const uint32_t per_sm = (uint32_t)std::min<size_t>(8, (200u << 10) / smem);
   const uint32_t grid = (uint32_t)std::min<size_t>(wl.size(), (size_t)num_sms() * (per_sm ? per_sm : 1));
   fft_worklist_kernel<<<grid, 256, smem, st>>>((const FftWlItem*)d, (uint32_t)wl.size(), d_twiddles, d_itwiddles,

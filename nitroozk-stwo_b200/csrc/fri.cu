@@ -308,9 +308,8 @@ int fri_tail(cudaStream_t st, const FriTail& a, uint32_t* d_state, const uint32_
   GS_REQUIRE(a.n >= 1 && a.n <= FRI_TAIL_MAX && a.log0 <= FRI_TAIL_MAX - 1 && a.log0 >= a.n,
              "FRI tail: layer sizes out of range");
   GS_REQUIRE(a.log0 <= tw_log, "FRI tail: line domain must fit the twiddle tree");
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(fri_tail_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_CTA_SMEM);
-  GS_CUDA_TRY(attr);
+  static OncePerDevice smem;
+  GS_CUDA_TRY(allow_smem(smem, fri_tail_cta_kernel, TAIL_CTA_SMEM));
   launch_after(fri_tail_cta_kernel, 1, 1024, TAIL_CTA_SMEM, st, a, d_state, d_itw, 1u << tw_log, 1u);
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());

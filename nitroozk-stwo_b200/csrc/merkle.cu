@@ -514,9 +514,8 @@ int merkle_worklist(Context& ctx, const MerkleItem* items, uint32_t n_items) {
     d = owned;
   }
   const size_t smem = (size_t)3 * 16 << max_log;  // 2^max_log + 2^(max_log - 1) hashes, reserved as 3 * 2^max_log uint4
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      merkle_worklist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(((size_t)3 * 16) << MERKLE_WL_MAX_LOG));
-  GS_CUDA_TRY(attr);
+  static OncePerDevice limit;
+  GS_CUDA_TRY(allow_smem(limit, merkle_worklist_kernel, (size_t)3 * 16 << MERKLE_WL_MAX_LOG));
   const uint32_t per_sm = (uint32_t)std::min<size_t>(8, ((size_t)200 << 10) / smem);
   const uint32_t grid = (uint32_t)std::min<size_t>(wl.size(), (size_t)num_sms() * (per_sm ? per_sm : 1));
   merkle_worklist_kernel<<<grid, 256, smem, st>>>((const MerkleWlItem*)d, (uint32_t)wl.size(),

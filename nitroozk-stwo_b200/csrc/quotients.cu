@@ -243,9 +243,8 @@ int accumulate_numerators(cudaStream_t st, const void* d_entries, uint32_t n_ent
     const size_t tiles = n / 1024;
     const size_t cap2 = (size_t)num_sms() * 8;
     const unsigned grid = (unsigned)(tiles < cap2 ? tiles : cap2);
-    static const cudaError_t attr = cudaFuncSetAttribute(
-        accumulate_numerators_split_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ACC_DYN_SMEM);
-    GS_CUDA_TRY(attr);
+    static OncePerDevice smem;
+    GS_CUDA_TRY(allow_smem(smem, accumulate_numerators_split_kernel<1>, ACC_DYN_SMEM));
     launch_after(accumulate_numerators_split_kernel<1>, grid, 256, ACC_DYN_SMEM, st, (const NumEntry*)d_entries,
                  n_entries, b_sum, log_size, out, d_bsum);
   } else if (R == 4)

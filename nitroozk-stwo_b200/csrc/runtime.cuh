@@ -7,6 +7,7 @@
 #include <string>
 #include <vector>
 #include "m31.cuh"
+#include "once_per_device.h"
 
 namespace gs {
 
@@ -125,6 +126,18 @@ inline void launch_after(void (*kernel)(K...), dim3 grid, dim3 block, size_t sme
   (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);  // (callers check cudaGetLastError)
 }
 #endif
+
+// Up to `bytes` of dynamic shared memory for a kernel on the current device
+// (more than 48 KiB has to be allowed). `set` belongs to the kernel.
+template <class Kernel>
+inline cudaError_t allow_smem(OncePerDevice& set, Kernel* kernel, size_t bytes) {
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  return (cudaError_t)set.run(device, [&] {
+    return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  });
+}
 
 // Count of kernel launches issued by this library (for launch accounting).
 void note_launch(unsigned n = 1);

@@ -78,46 +78,39 @@ def qm31(v):
 
 
 def _integer_words(values):
-    """A list of rows of 4 integers as an array of words, mod 2^32 as in a
-    ctypes field; None for rows of other lengths or values of other types,
-    which a conversion per value takes or refuses. Of integers alone: numpy
-    turns NaN, infinities and complex numbers into integers, int() does not."""
+    """Rows of 4 integers as an array of 32-bit words; None for words of other
+    types and ranges and for rows of other lengths, which a conversion per
+    value takes, wraps or refuses. Of integers alone: numpy turns NaN,
+    infinities and complex numbers into integers, int() does not."""
     try:
         if isinstance(values[0], np.ndarray):
             a = np.array(values)
             if a.dtype.kind not in "biu" or a.shape != (len(values), 4):
                 return None
-        elif set(map(len, values)) == {4}:
-            a = np.frombuffer(array.array("q", list(itertools.chain.from_iterable(values))), np.int64)
-            a = a.reshape(-1, 4)
-        else:
-            return None
+            return array.array("I", a.astype(np.uint32).tobytes())
+        if set(map(len, values)) == {4}:
+            return array.array("I", list(itertools.chain.from_iterable(values)))
     except Exception:
-        return None
-    return a.astype(np.uint32)
+        pass
+    return None
 
 
 def qm31_array(values, n=None):
     """QM31 values (4 ints each) as a host array of n gs_qm31, zeros after the
-    last: (address, array to keep alive)."""
+    last: (address, array to keep alive). Without numpy, whose fixed cost made
+    calls of one to three values slower than a ctypes array."""
     values = list(values)
     n = len(values) if n is None else n
     if len(values) > max(n, 1):
         raise ValueError(f"{len(values)} values for {n} places")
-    out = np.zeros((max(n, 1), 4), np.uint32)
-    if values:
-        words = _integer_words(values)
-        if words is None:
-            arr = (L.QM31 * len(values))(*[qm31(v) for v in values])
-            words = np.frombuffer(arr, np.uint32).reshape(-1, 4)
-        out[:len(values)] = words
-    return out.ctypes.data, out
+    out = _integer_words(values) if values else array.array("I")
+    if out is None:
+        out = array.array("I", bytes((L.QM31 * len(values))(*[qm31(v) for v in values])))
+    if len(values) < max(n, 1):
+        out.frombytes(bytes(16 * (max(n, 1) - len(values))))
+    return out.buffer_info()[0], out
 
 
-# gs_fft_item and gs_merkle_item (include/gpustark.h)
-_FFT_ITEM = np.dtype([("src", "u8"), ("dst", "u8"), ("log_size", "u4"), ("coeffs_log_size", "u4"), ("inverse", "u4"),
-                      ("reserved", "u4")])
-_MERKLE_ITEM = np.dtype([("cols", "u8"), ("n_cols", "u4"), ("log_size", "u4"), ("layers", "u8")])
 # A small tree's layers are one allocation; a larger tree's are separate, so
 # that a caller who keeps only its root keeps only the root's memory.
 _ONE_BUFFER_TREE_LOG = 10
@@ -202,17 +195,13 @@ class GpuBackend:
         (src is dst: in place) or ("evaluate", coeffs, dst) with dst of
         2^log words; returns the dst tensors."""
         ctx = ctx or default_context()
-        for kind, _, _ in items:
+        words = []  # gs_fft_item, as 8-byte words
+        for kind, src, dst in items:
             if kind not in ("interpolate", "evaluate"):
                 raise ValueError(f"unknown work-list item kind {kind!r}")
-        arr = np.zeros(max(len(items), 1), _FFT_ITEM)
-        if items:
-            arr["src"] = [src.data_ptr() for _, src, _ in items]
-            arr["dst"] = [dst.data_ptr() for _, _, dst in items]
-            arr["log_size"] = [_log_word(dst) for _, _, dst in items]
-            arr["coeffs_log_size"] = [_log_word(src) for _, src, _ in items]
-            arr["inverse"] = [kind == "interpolate" for kind, _, _ in items]
-        L.check(L.lib().gs_fft_worklist(ctx.handle, arr.ctypes.data, len(items), _p(twiddles.twiddles), _p(twiddles.itwiddles),
+            words += (src.data_ptr(), dst.data_ptr(), _log_word(dst) | _log_word(src) << 32, kind == "interpolate")
+        arr, keep = L.ptr_array(words)
+        L.check(L.lib().gs_fft_worklist(ctx.handle, arr, len(items), _p(twiddles.twiddles), _p(twiddles.itwiddles),
                                         twiddles.root_log), "fft_worklist")
         return [dst for _, _, dst in items]
 
@@ -290,13 +279,11 @@ class GpuBackend:
             ptrs += [c.data_ptr() for c in cols]
             ptrs += [t.data_ptr() for t in layers]
         base, keep = L.ptr_array(ptrs)
-        arr = np.zeros(max(len(trees), 1), _MERKLE_ITEM)
-        if trees:
-            arr["cols"] = [base + 8 * c for c, _ in at]
-            arr["n_cols"] = [len(cols) for cols in trees]
-            arr["log_size"] = logs
-            arr["layers"] = [base + 8 * l for _, l in at]
-        L.check(L.lib().gs_merkle_worklist(ctx.handle, arr.ctypes.data, len(trees)), "merkle_worklist")
+        words = []  # gs_merkle_item, as 8-byte words
+        for cols, log, (c, l) in zip(trees, logs, at):
+            words += (base + 8 * c, len(cols) | log << 32, base + 8 * l)
+        arr, keep_items = L.ptr_array(words)
+        L.check(L.lib().gs_merkle_worklist(ctx.handle, arr, len(trees)), "merkle_worklist")
         return out
 
     @staticmethod
@@ -365,12 +352,12 @@ class GpuBackend:
         out = [torch.empty(1 << log_size, dtype=torch.int32, device="cuda") for _ in range(4)]
         cp, k1 = L.ptr_array([c.data_ptr() for c in columns])
         n = len(column_indices)
-        idx = np.array([int(i) & 0xFFFFFFFF for i in column_indices] or [0], dtype=np.uint32)
+        idx = array.array("I", [int(i) & 0xFFFFFFFF for i in column_indices] or [0])
         bs, kb = qm31_array(line_coeffs_b, n)
         cs, kc = qm31_array(line_coeffs_c, n)
         op, k2 = L.ptr_array([t.data_ptr() for t in out])
         L.check(L.lib().gs_accumulate_numerators(ctx.handle, log_size, cp, len(columns),
-                                                 idx.ctypes.data_as(L.U32P), bs, cs, n, op),
+                                                 (C.c_uint32 * len(idx)).from_buffer(idx), bs, cs, n, op),
                 "accumulate_numerators")
         return out
 

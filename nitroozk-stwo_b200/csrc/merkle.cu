@@ -27,13 +27,21 @@ __device__ __forceinline__ void store_hash(uint32_t* out, size_t i, const uint32
   o[1] = make_uint4(h[4], h[5], h[6], h[7]);
 }
 
-// FMA: adds of the compression on the FMA pipe (blake2s_compress_f).
-template <bool FMA>
-__global__ void __launch_bounds__(256) merkle_layer_kernel(uint32_t log_size, const uint32_t* __restrict__ prev,
-                                                           Cols cols, uint32_t n_cols, uint32_t* __restrict__ out,
-                                                           uint32_t one) {
+// FMA: adds of the compression on the FMA pipe (blake2s_compress_f). TABLE:
+// columns through the pointer table, else from a base and a stride, chosen at
+// compile time: a choice per word keeps a block's 16 loads from being issued
+// together (64 columns x 2^20 rows, not 16-byte aligned: 308 us, now 196; 100
+// x 2^13 29.5 -> 15.0). Five blocks per SM: 48 registers, where the compiler
+// takes 55 to 59 by itself (2^19 nodes of two children 25.0 -> 23.8 us; 21.8
+// with its launch overlapped).
+template <bool FMA, bool TABLE>
+__global__ void __launch_bounds__(256, 5)
+    merkle_layer_kernel(uint32_t log_size, const uint32_t* __restrict__ prev, const uint32_t* const* __restrict__ tab,
+                        const uint32_t* __restrict__ base, size_t stride, uint32_t n_cols, uint32_t* __restrict__ out,
+                        uint32_t one) {
+  const uint32_t prev_words = prev ? 16u : 0u;  // (before the shift: a null stays null)
+  after_previous(prev, tab, base);
   const size_t n = (size_t)1 << log_size;
-  const uint32_t prev_words = prev ? 16u : 0u;
   const uint32_t total_words = prev_words + n_cols;
   const uint32_t total_bytes = 4u * total_words;
   const uint32_t n_blocks = total_words == 0 ? 1u : (total_words + 15u) / 16u;
@@ -43,7 +51,7 @@ __global__ void __launch_bounds__(256) merkle_layer_kernel(uint32_t log_size, co
     uint32_t m[16];
     uint32_t blk = 0;
     uint32_t col = 0;
-    if (prev) {
+    if (prev_words) {
       const uint4* p = reinterpret_cast<const uint4*>(prev + 16 * i);
       uint4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3);
       m[0] = a.x; m[1] = a.y; m[2] = a.z; m[3] = a.w;
@@ -59,7 +67,7 @@ __global__ void __launch_bounds__(256) merkle_layer_kernel(uint32_t log_size, co
 #pragma unroll
       for (int j = 0; j < 16; j++) {
         uint32_t c = col + j;
-        m[j] = c < n_cols ? __ldg(cols[c] + i) : 0u;
+        m[j] = c < n_cols ? __ldg((TABLE ? tab[c] : base + c * stride) + i) : 0u;
       }
       col += 16;
       uint32_t t = 64u * (blk + 1);
@@ -203,7 +211,12 @@ int commit_on_layer(cudaStream_t st, uint32_t log_size, const uint32_t* d_prev, 
     const char* e = getenv("GS_BLAKE_ALU");
     return e && e[0] == '1';
   }();
-  if (cols_aligned && n_cols > 0 && log_size >= 5 && !alu_only) {
+  // With children and at most 24 columns, large layers stay with a thread per
+  // node: the staged kernel's warps wait for their children once per tile (one
+  // column injected at 2^22 nodes 376 us staged, 352 not; at 2^19 48.3 and
+  // 43.9; at 2^17 12.8 and 16.8; 32 columns at 2^20 142 and 144).
+  const bool staged = cols_aligned && n_cols > 0 && log_size >= 5 && !(d_prev && n_cols <= 24 && log_size >= 18);
+  if (staged && !alu_only) {
     const size_t tiles = n / (32 * COL_WARPS) ? n / (32 * COL_WARPS) : 1;
     const size_t resident = (size_t)num_sms() * 8;  // one wave; a warp walks its tiles, copies crossing from one to the next
     const unsigned grid = (unsigned)(tiles < resident ? tiles : resident);
@@ -211,10 +224,12 @@ int commit_on_layer(cudaStream_t st, uint32_t log_size, const uint32_t* d_prev, 
       launch_after(merkle_columns_kernel<true>, grid, 32 * COL_WARPS, 0, st, log_size, d_prev, cols, n_cols, d_out, 1u);
     else
       launch_after(merkle_columns_kernel<false>, grid, 32 * COL_WARPS, 0, st, log_size, d_prev, cols, n_cols, d_out, 1u);
-  } else if (alu_only)
-    merkle_layer_kernel<false><<<(unsigned)blocks, threads, 0, st>>>(log_size, d_prev, cols, n_cols, d_out, 1u);
-  else
-    merkle_layer_kernel<true><<<(unsigned)blocks, threads, 0, st>>>(log_size, d_prev, cols, n_cols, d_out, 1u);
+  } else {
+    const auto kernel = alu_only ? (cols.tab ? merkle_layer_kernel<false, true> : merkle_layer_kernel<false, false>)
+                                 : (cols.tab ? merkle_layer_kernel<true, true> : merkle_layer_kernel<true, false>);
+    launch_after(kernel, (unsigned)blocks, threads, 0, st, log_size, d_prev, cols.tab, cols.base, cols.stride, n_cols,
+                 d_out, 1u);
+  }
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;

@@ -49,3 +49,20 @@ def test_column_spacings(B, pick, log, off):
         assert all(np.array_equal(host(a), b) for a, b in zip(cols, want))
         rest = [i for i in range(8) if i not in idx]
         assert np.array_equal(host(mat[rest]), words[rest])
+
+
+@pytest.mark.parametrize("log,n_cols", [(4, 3), (9, 17), (12, 40), (17, 24), (18, 1), (18, 24), (18, 25)])
+@pytest.mark.parametrize("off", [0, 1])
+def test_layer_kernels(B, log, n_cols, off):
+    """A layer over children and columns by either kernel (aligned or not, few
+    and more columns, small and large layers), evenly spaced or not."""
+    rng = np.random.default_rng(log * 100 + n_cols)
+    n = 1 << log
+    words = rng.integers(0, O.P, (n_cols, n + 4), dtype=np.int64).astype(np.uint32)
+    prev = rng.integers(0, 256, (2 * n, 32), dtype=np.uint8)
+    mat = torch.from_numpy(words.view(np.int32)).cuda()
+    kids = torch.from_numpy(prev.reshape(-1).view(np.int32)).cuda()
+    for order in (list(range(n_cols)), [0] + list(range(n_cols - 1, 0, -1)) + [0]):
+        ref = [words[i, off:off + n].copy() for i in order]
+        got = B.commit_on_layer(log, kids, [mat[i, off:off + n] for i in order])
+        assert np.array_equal(host(got).view(np.uint8).reshape(-1, 32), O.commit_on_layer(log, prev.reshape(-1), ref))

@@ -293,13 +293,16 @@ def cpu_sweep_sample(threads):
 def fft_autotune(args, hi):
     """Installs the FFT pass splits the library's autotuner picks for log
     sizes 8..hi and LDE extensions 0..2 (set-up, outside every timed region);
-    returns the picks that differ from the default 13/4 as
+    returns the picks that divide the layers otherwise than the split by size as
     {"log+extension": "tile_log/coalesce_bits"}."""
     if args.fft_autotune == "off":
         return "off"
     from gpustark.backend import GpuBackend
+    sizes = [(n, e) for n in range(8, min(hi, 27) + 1) for e in range(3)]
+    passes = lambda: [[p[:2] for p in GpuBackend.fft_passes(n + e, n)] for n, e in sizes]  # noqa: E731
+    before = passes()
     picks = GpuBackend.fft_autotune(8, min(hi, 27), 2)
-    return {"%d+%d" % k: "%d/%d" % v for k, v in picks.items() if v != (13, 4)}
+    return {"%d+%d" % k: "%d/%d" % picks[k] for k, a, b in zip(sizes, before, passes()) if a != b}
 
 
 def run_kernels(args, world, rank, local):

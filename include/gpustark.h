@@ -131,12 +131,20 @@ int gs_fft_worklist(gs_ctx* ctx, const gs_fft_item* items, uint32_t n_items, con
  * set-up calls: no other FFT may be in flight. gs_fft_set_tuning installs one
  * split (log_size 0: every size; extension > 3: every extension; tile_log in
  * [6, 13], coalesce_bits <= min(5, tile_log - 5)); gs_fft_get_tuning reads
- * it. The default, 13 / 4, takes the split measured best for the size within
- * tiles of 2^13 (12 / 5, 12 / 4 or 13 / 4). */
+ * it. Where nothing is installed, the split goes by the size (12 / 5, 12 / 4 or
+ * 13 / 4, within tiles of 2^13) and reads as 13 / 4; gs_fft_reset_tuning goes
+ * back to that for every size. gs_fft_passes lists the passes that an FFT of
+ * n_cols columns (16-byte aligned; coeffs_log_size = log_size for an
+ * interpolation, `inverse`) takes with the splits installed, in the order of
+ * launch: three words each, first layer, layers, and kernel (0 generic, 1 a
+ * tile per block, 2 streaming), at most 8 of them. */
 int gs_fft_autotune(gs_ctx* ctx, uint32_t min_log, uint32_t max_log, uint32_t max_extension, uint32_t* tile_logs,
                     uint32_t* coalesce_bits);
 int gs_fft_set_tuning(uint32_t log_size, uint32_t extension, uint32_t tile_log, uint32_t coalesce_bits);
 int gs_fft_get_tuning(uint32_t log_size, uint32_t extension, uint32_t* tile_log, uint32_t* coalesce_bits);
+int gs_fft_reset_tuning(void);
+int gs_fft_passes(uint32_t log_size, uint32_t coeffs_log_size, uint32_t n_cols, uint32_t inverse, uint32_t* passes,
+                  uint32_t* n_passes);
 
 /* -------------------------------------------------------------- MerkleOps */
 /* commit_on_first_layer / commit_on_layer_with_previous (bindings.rs:262-275);

@@ -199,6 +199,16 @@ int gs_fft_set_tuning(uint32_t log_size, uint32_t extension, uint32_t tile_log, 
   return set_fft_tuning(log_size, extension, tile_log, coalesce_bits);
 }
 
+int gs_fft_reset_tuning(void) {
+  reset_fft_tuning();
+  return OK;
+}
+
+int gs_fft_passes(uint32_t log_size, uint32_t coeffs_log_size, uint32_t n_cols, uint32_t inverse, uint32_t* passes,
+                  uint32_t* n_passes) {
+  return fft_passes(log_size, coeffs_log_size, n_cols, inverse != 0, passes, n_passes);
+}
+
 int gs_fft_get_tuning(uint32_t log_size, uint32_t extension, uint32_t* tile_log, uint32_t* coalesce_bits) {
   GS_REQUIRE(log_size < 32 && tile_log && coalesce_bits, "bad arguments");
   get_fft_tuning(log_size, extension, tile_log, coalesce_bits);

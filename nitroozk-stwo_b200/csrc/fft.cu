@@ -717,26 +717,29 @@ static int launch_small(cudaStream_t st, Cols src, MutCols dst, uint32_t n_cols,
 }
 
 struct FftTuning {
-  uint32_t tile_log;       // log2 of the shared-memory tile (elements), <= 13
+  uint32_t tile_log;       // log2 of the shared-memory tile (elements), <= 13; 0: by size
   uint32_t coalesce_bits;  // contiguous low bits per strided tile row
 };
 // Per number of computed layers (an FFT of 2^n, or an LDE from 2^n
 // coefficients, computes n layers) and extension (domain log size minus
 // layers: 0 for an FFT, the blowup for an LDE; capped at FFT_MAX_EXT). Written
-// at set-up (set_fft_tuning, fft_autotune), read by every launch.
+// at set-up (set_fft_tuning, fft_autotune, reset_fft_tuning), read by every
+// launch. Zero, as at the start: the split by size.
 constexpr uint32_t FFT_MAX_EXT = 3;
+static FftTuning g_fft_tuning[32][FFT_MAX_EXT + 1];
 static void split_layers(uint32_t layers, FftTuning tn, std::vector<std::pair<uint32_t, uint32_t>>& parts);
 
-// What the default, 13/4, stands for: within tiles of 2^13, the split measured
-// best for each size. Fewest passes, then fewest register stages
-// (of up to 5 layers), then the wider rows of 12/5 (whole 128-byte lines).
-// 13/4, whose strided passes hold 9 layers in tiles of 2^13, only where it
-// saves a pass. Measured with fft_stream_kernel and butterflies of three
-// reductions: 158 columns of 2^18 extended by 2 and interpolated, 9 + 9 layers
-// (13/4) 625 + 171 us, 10 + 8 (12/4) 589 + 166; eight columns of 2^22, 13 + 9
-// 341 + 173 against three passes' 366 + 248. 2^19, with an earlier form of it,
-// 12 + 7 (12/5) 280 + 155 against 290 + 162 for 10 + 9.
-static FftTuning default_tuning(uint32_t layers) {
+// The split by size, within tiles of 2^13. Fewest passes, then fewest register
+// stages (of up to 5 layers), then the wider rows of 12/5 (whole 128-byte
+// lines). 13/4, whose strided passes hold 9 layers in tiles of 2^13, only where
+// it saves a pass. 158 columns of 2^18: 9 + 9 layers (13/4) 167 us interpolated
+// and 306 extended by 1, 10 + 8 (12/4) 159 and 292; 17 layers of 128 columns,
+// 10 + 7 against 8 + 9, 63 against 72. Over 13..24 layers of 1 to 256 columns,
+// extended by 0 to 2, it is within 7% (mostly 3%) of the best of 13/4, 12/4,
+// 12/5, 13/5, 11/5 and 10/4, except at 22 layers of up to 4 columns: three
+// passes (10/4 or 11/5) take 0.90 to 0.97 of 13 + 9. 13/4 at every size takes
+// up to 1.19 times as long.
+static FftTuning split_by_size(uint32_t layers) {
   FftTuning best{13, 4};
   size_t best_passes = 99, best_stages = 0;
   for (FftTuning tn : {FftTuning{12, 5}, FftTuning{12, 4}, FftTuning{13, 4}}) {
@@ -752,26 +755,23 @@ static FftTuning default_tuning(uint32_t layers) {
   }
   return best;
 }
-struct FftTunings {
-  FftTuning by_size[32];
-  FftTuning at[32][FFT_MAX_EXT + 1];  // as installed
-  FftTunings() {
-    for (uint32_t l = 0; l < 32; l++) {
-      by_size[l] = default_tuning(l);
-      for (uint32_t e = 0; e <= FFT_MAX_EXT; e++) at[l][e] = {13, 4};
-    }
+struct SplitsBySize {
+  FftTuning of[32];
+  SplitsBySize() {
+    for (uint32_t l = 0; l < 32; l++) of[l] = split_by_size(l);
   }
-  FftTuning* operator[](uint32_t l) { return at[l]; }
 };
-static FftTunings g_fft_tuning;
 static uint32_t ext_slot(uint32_t layers, uint32_t n) {
   return n - layers < FFT_MAX_EXT ? n - layers : FFT_MAX_EXT;
 }
 static FftTuning tuning_for(uint32_t layers, uint32_t n) {
+  static const SplitsBySize by_size;
   const uint32_t l = layers < 32 ? layers : 31;
   const FftTuning t = g_fft_tuning[l][ext_slot(layers, n)];
-  return t.tile_log == 13 && t.coalesce_bits == 4 ? g_fft_tuning.by_size[l] : t;
+  return t.tile_log ? t : by_size.of[l];
 }
+// An entry as it is read back: 13/4 where nothing was installed.
+static FftTuning reported(FftTuning t) { return t.tile_log ? t : FftTuning{13, 4}; }
 
 // Splits layers [0, layers) into balanced passes (lo, L): the first pass has
 // the whole tile for layers, later ones reserve `coalesce_bits` of it.
@@ -855,9 +855,10 @@ static int launch_stream(cudaStream_t st, uint32_t n_cols, Cols s, MutCols d,
 // A contiguous pass builds a table of half a tile's words per block, which
 // takes 4 tiles to pay (one column of 2^24, a tile per block: 46 -> 77 us).
 constexpr uint32_t STREAM_MIN_TILES = 4;
+// Without `launch` it only says so.
 template <bool INV>
 static int launch_stream_any(cudaStream_t st, uint32_t n_cols, Cols s, MutCols d,
-                             const uint32_t* tw, const FftPass& a, bool* taken) {
+                             const uint32_t* tw, const FftPass& a, bool* taken, bool launch = true) {
   *taken = false;
   if (fft_generic() || !a.vec_ok || (uint64_t)n_cols << a.n >= 1ull << 40) return OK;
 #define GS_STREAM(LL, CC, TB)                                                   \
@@ -866,7 +867,7 @@ static int launch_stream_any(cudaStream_t st, uint32_t n_cols, Cols s, MutCols d
     if (CC == 0 && stream_tiles(a.n - TB, n_cols, StreamShape<INV, LL, CC, TB>::PER_SM) < STREAM_MIN_TILES) \
       return OK;                                                                \
     *taken = true;                                                              \
-    return launch_stream<INV, LL, CC, TB>(st, n_cols, s, d, tw, a);
+    return launch ? launch_stream<INV, LL, CC, TB>(st, n_cols, s, d, tw, a) : OK;
   if (a.lo == 0) {
     switch (a.L) { GS_STREAM(5, 0, 12) GS_STREAM(6, 0, 12) GS_STREAM(7, 0, 12) GS_STREAM(8, 0, 12) GS_STREAM(9, 0, 12)
                    GS_STREAM(10, 0, 12) GS_STREAM(11, 0, 12) GS_STREAM(12, 0, 12) GS_STREAM(13, 0, 13)
@@ -879,13 +880,16 @@ static int launch_stream_any(cudaStream_t st, uint32_t n_cols, Cols s, MutCols d
 
 // The specialised kernel covers first passes (C = 0, 5..13 layers) and later
 // passes with 16 or 32 contiguous words per tile row (C = 4 with 5..9 layers,
-// C = 5 with 5..8); anything else runs the generic pass.
+// C = 5 with 5..8); anything else runs the generic pass. Without `launch` it
+// only says which.
 template <bool INV>
 static bool launch_tile_any(cudaStream_t st, dim3 grid, uint32_t threads, Cols s,
-                            MutCols d, const uint32_t* tw, const FftPass& a) {
+                            MutCols d, const uint32_t* tw, const FftPass& a, bool launch = true) {
   if (fft_generic()) return false;
-#define GS_TILE(LL, CC) \
-  case LL: launch_tile<INV, LL, CC>(st, grid, threads, s, d, tw, a); return true;
+#define GS_TILE(LL, CC)                                                   \
+  case LL:                                                                \
+    if (launch) launch_tile<INV, LL, CC>(st, grid, threads, s, d, tw, a); \
+    return true;
   if (a.c == 0) {
     switch (a.L) { GS_TILE(5, 0) GS_TILE(6, 0) GS_TILE(7, 0) GS_TILE(8, 0) GS_TILE(9, 0) GS_TILE(10, 0)
                    GS_TILE(11, 0) GS_TILE(12, 0) GS_TILE(13, 0) default: return false; }
@@ -906,31 +910,37 @@ static thread_local bool g_cols_aligned = true;
 void fft_set_columns_aligned(bool aligned) { g_cols_aligned = aligned; }
 
 template <bool INV>
+static FftPass pass_of(uint32_t n, uint32_t layers, std::pair<uint32_t, uint32_t> part, bool first, bool last,
+                       uint32_t src_mask, uint32_t tw_len, bool aligned) {
+  FftPass a{};
+  a.n = n;
+  a.lo = part.first;
+  a.L = part.second;
+  a.c = std::min(tuning_for(layers, n).coalesce_bits, a.lo);
+  a.t = a.c + a.L;
+  const uint32_t R = std::min<uint32_t>(5, a.L);
+  a.K = (a.L + R - 1) / R;
+  a.src_mask = first ? src_mask : 0xffffffffu;
+  a.tw_len = tw_len;
+  a.has_scale = (INV && last) ? 1u : 0u;
+  a.scale = a.has_scale ? inv(1u << n) : 1u;
+  a.vec_ok = aligned ? 1u : 0u;
+  const uint32_t tpt_log = a.t - R, tiles_log = n - a.t;
+  a.tile_shift = std::min(tpt_log < 7 ? 7 - tpt_log : 0u, tiles_log);
+  return a;
+}
+
+template <bool INV>
 static int run_passes(cudaStream_t st, Cols src, MutCols dst, uint32_t n_cols, uint32_t n,
                       uint32_t layers, uint32_t src_mask, const uint32_t* tw, uint32_t tw_len) {
   std::vector<std::pair<uint32_t, uint32_t>> parts;
   fft_partition(layers, n, parts);
   if (!INV) std::reverse(parts.begin(), parts.end());
   for (size_t p = 0; p < parts.size(); p++) {
-    FftPass a{};
-    a.n = n;
-    a.lo = parts[p].first;
-    a.L = parts[p].second;
-    a.c = std::min(tuning_for(layers, n).coalesce_bits, a.lo);
-    a.t = a.c + a.L;
-    const uint32_t R = std::min<uint32_t>(5, a.L);
-    a.K = (a.L + R - 1) / R;
-    a.src_mask = (p == 0) ? src_mask : 0xffffffffu;
-    a.tw_len = tw_len;
-    a.has_scale = (INV && p + 1 == parts.size()) ? 1u : 0u;
-    a.scale = a.has_scale ? inv(1u << n) : 1u;
-    a.vec_ok = g_cols_aligned ? 1u : 0u;
-    const uint32_t tpt_log = a.t - R;
+    const FftPass a = pass_of<INV>(n, layers, parts[p], p == 0, p + 1 == parts.size(), src_mask, tw_len, g_cols_aligned);
+    const uint32_t R = std::min<uint32_t>(5, a.L), tile_shift = a.tile_shift;
     const uint32_t tiles_log = n - a.t;
-    uint32_t tile_shift = tpt_log < 7 ? 7 - tpt_log : 0;
-    if (tile_shift > tiles_log) tile_shift = tiles_log;
-    a.tile_shift = tile_shift;
-    const uint32_t threads = 1u << (tpt_log + tile_shift);
+    const uint32_t threads = 1u << (a.t - R + tile_shift);
     const size_t smem = (size_t)4 << (a.t + tile_shift);
     dim3 grid(1u << (tiles_log - tile_shift), n_cols);
     Cols s = (p == 0) ? src : Cols(dst);
@@ -950,6 +960,37 @@ static int run_passes(cudaStream_t st, Cols src, MutCols dst, uint32_t n_cols, u
     }
     GS_CUDA_TRY(cudaGetLastError());
   }
+  return OK;
+}
+
+// The passes of an FFT of n_cols aligned columns, in the order of launch: first
+// layer, layers, kernel (0 generic, 1 a tile per block, 2 streaming).
+template <bool INV>
+static void list_passes(uint32_t n, uint32_t layers, uint32_t n_cols, uint32_t* out, uint32_t* n_out) {
+  std::vector<std::pair<uint32_t, uint32_t>> parts;
+  fft_partition(layers, n, parts);
+  if (!INV) std::reverse(parts.begin(), parts.end());
+  for (size_t p = 0; p < parts.size(); p++) {
+    const FftPass a = pass_of<INV>(n, layers, parts[p], p == 0, p + 1 == parts.size(),
+                                   layers == n ? 0xffffffffu : (1u << layers) - 1u, 1u << (n - 1), true);
+    bool streams = false;
+    (void)launch_stream_any<INV>(nullptr, n_cols, Cols(), MutCols(), nullptr, a, &streams, false);
+    const bool tile = a.L >= 5 && launch_tile_any<INV>(nullptr, dim3(), 0, Cols(), MutCols(), nullptr, a, false);
+    out[3 * p] = a.lo;
+    out[3 * p + 1] = a.L;
+    out[3 * p + 2] = streams ? 2u : tile ? 1u : 0u;
+  }
+  *n_out = (uint32_t)parts.size();
+}
+int fft_passes(uint32_t log_n, uint32_t coeff_log, uint32_t n_cols, bool inverse, uint32_t* out, uint32_t* n_out) {
+  GS_REQUIRE(log_n >= 1 && log_n <= 30 && coeff_log >= 1 && coeff_log <= log_n, "log size out of range");
+  GS_REQUIRE(n_cols >= 1 && n_cols <= 65535, "number of columns out of range");
+  GS_REQUIRE(!inverse || coeff_log == log_n, "an interpolation computes every layer");
+  GS_REQUIRE(out && n_out, "null output");
+  *n_out = 0;
+  if (log_n <= 2) return OK;  // closed forms
+  if (inverse) list_passes<true>(log_n, coeff_log, n_cols, out, n_out);
+  else list_passes<false>(log_n, coeff_log, n_cols, out, n_out);
   return OK;
 }
 
@@ -1120,6 +1161,11 @@ int set_fft_tuning(uint32_t layers, uint32_t ext, uint32_t tile_log, uint32_t co
   return OK;
 }
 
+void reset_fft_tuning() {
+  for (auto& row : g_fft_tuning)
+    for (FftTuning& t : row) t = FftTuning{0, 0};
+}
+
 // Picks, for every FFT log size n in [lo, hi] and extension e in [0,
 // max_ext], the tile size and coalesced row width whose pass split is
 // fastest, and installs it. e = 0 times an evaluate + interpolate round trip
@@ -1129,7 +1175,8 @@ int set_fft_tuning(uint32_t layers, uint32_t ext, uint32_t tile_log, uint32_t co
 // whose output exceeds the scratch keep their tuning. Each split is timed with
 // CUDA events as the best of 3 trials of 3 runs; the installed split (first
 // in the list) is replaced only by one at least 2% faster, so timing noise
-// does not move it. Candidates that give the same pass split as an earlier
+// does not move it; the split by size, where it stays, is installed as what it
+// is. Candidates that give the same pass split as an earlier
 // one are not timed again. Every candidate computes the same values; only the
 // split, and so the speed, differ. Not thread-safe against concurrent
 // launches (a set-up step). Outputs: (hi - lo + 1) x (max_ext + 1), by size.
@@ -1162,8 +1209,8 @@ int fft_autotune(cudaStream_t st, uint32_t lo, uint32_t hi, uint32_t max_ext, co
       const uint32_t dn = n + e;  // domain log size
       const size_t slot = (size_t)(n - lo) * (max_ext + 1) + e;
       if (dn > w_log || tw_log + 1 < dn) {
-        if (out_tile) out_tile[slot] = g_fft_tuning[n][e].tile_log;
-        if (out_coalesce) out_coalesce[slot] = g_fft_tuning[n][e].coalesce_bits;
+        if (out_tile) out_tile[slot] = reported(g_fft_tuning[n][e]).tile_log;
+        if (out_coalesce) out_coalesce[slot] = reported(g_fft_tuning[n][e]).coalesce_bits;
         continue;
       }
       const uint32_t cols = (uint32_t)std::min<size_t>(words >> dn, max_cols);
@@ -1179,7 +1226,7 @@ int fft_autotune(cudaStream_t st, uint32_t lo, uint32_t hi, uint32_t max_ext, co
         rc = ERR_CUDA;
         break;
       }
-      const FftTuning keep = g_fft_tuning[n][e];
+      const FftTuning before = g_fft_tuning[n][e], keep = tuning_for(n, dn);
       float best = 1e30f, keep_ms = 1e30f;
       FftTuning pick = keep;
       std::vector<std::vector<std::pair<uint32_t, uint32_t>>> seen;
@@ -1190,8 +1237,7 @@ int fft_autotune(cudaStream_t st, uint32_t lo, uint32_t hi, uint32_t max_ext, co
         g_fft_tuning[n][e] = c;
         std::vector<std::pair<uint32_t, uint32_t>> parts;
         fft_partition(n, dn, parts);
-        const uint32_t cb = tuning_for(n, dn).coalesce_bits;
-        for (auto& pr : parts) pr.first = std::min(cb, pr.first) | (pr.first << 8);
+        for (auto& pr : parts) pr.first = std::min(c.coalesce_bits, pr.first) | (pr.first << 8);
         if (std::find(seen.begin(), seen.end(), parts) != seen.end()) continue;
         seen.push_back(parts);
         float ms = 1e30f;
@@ -1223,7 +1269,7 @@ int fft_autotune(cudaStream_t st, uint32_t lo, uint32_t hi, uint32_t max_ext, co
         }
       }
       if (best > 0.98f * keep_ms) pick = keep;
-      g_fft_tuning[n][e] = rc == OK ? pick : keep;
+      g_fft_tuning[n][e] = rc == OK ? pick : before;
       if (out_tile) out_tile[slot] = g_fft_tuning[n][e].tile_log;
       if (out_coalesce) out_coalesce[slot] = g_fft_tuning[n][e].coalesce_bits;
     }
@@ -1240,7 +1286,7 @@ int fft_autotune(cudaStream_t st, uint32_t lo, uint32_t hi, uint32_t max_ext, co
 }
 
 void get_fft_tuning(uint32_t layers, uint32_t ext, uint32_t* tile_log, uint32_t* coalesce_bits) {
-  const FftTuning t = g_fft_tuning[layers < 32 ? layers : 31][ext < FFT_MAX_EXT ? ext : FFT_MAX_EXT];
+  const FftTuning t = reported(g_fft_tuning[layers < 32 ? layers : 31][ext < FFT_MAX_EXT ? ext : FFT_MAX_EXT]);
   *tile_log = t.tile_log;
   *coalesce_bits = t.coalesce_bits;
 }

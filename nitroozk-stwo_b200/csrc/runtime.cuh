@@ -325,6 +325,8 @@ int bit_reverse(cudaStream_t st, uint32_t* d, uint32_t log_n);
 // Pass-split tuning per number of computed layers and extension (domain log
 // size minus layers), process-wide, written at set-up time.
 int set_fft_tuning(uint32_t layers, uint32_t ext, uint32_t tile_log, uint32_t coalesce_bits);
+void reset_fft_tuning();
+int fft_passes(uint32_t log_n, uint32_t coeff_log, uint32_t n_cols, bool inverse, uint32_t* out, uint32_t* n_out);
 void get_fft_tuning(uint32_t layers, uint32_t ext, uint32_t* tile_log, uint32_t* coalesce_bits);
 int fft_autotune(cudaStream_t st, uint32_t lo, uint32_t hi, uint32_t max_ext, const uint32_t* tw, const uint32_t* itw,
                  uint32_t tw_log, uint32_t* out_tile, uint32_t* out_coalesce);

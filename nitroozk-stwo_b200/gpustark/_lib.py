@@ -72,6 +72,8 @@ _PROTOS = {
     "gs_fft_autotune": [C.c_void_p, C.c_uint32, C.c_uint32, C.c_uint32, U32P, U32P],
     "gs_fft_set_tuning": [C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32],
     "gs_fft_get_tuning": [C.c_uint32, C.c_uint32, U32P, U32P],
+    "gs_fft_reset_tuning": [],
+    "gs_fft_passes": [C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, U32P, U32P],
     "gs_commit_on_layer": [C.c_void_p, C.c_uint32, C.c_void_p, C.c_uint32, VPP, C.c_void_p],
     "gs_commit_node_layers": [C.c_void_p, C.c_uint32, VPP],
     "gs_merkle_worklist": [C.c_void_p, C.c_void_p, C.c_uint32],

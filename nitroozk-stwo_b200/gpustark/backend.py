@@ -231,6 +231,20 @@ class GpuBackend:
         L.check(L.lib().gs_fft_get_tuning(log_size, extension, C.byref(t), C.byref(c)), "fft_get_tuning")
         return t.value, c.value
 
+    @staticmethod
+    def fft_reset_tuning():
+        """Back to the splits by size, for every size."""
+        L.check(L.lib().gs_fft_reset_tuning(), "fft_reset_tuning")
+
+    @staticmethod
+    def fft_passes(log_size, coeffs_log_size=None, n_columns=1, inverse=False):
+        """The passes that an FFT of aligned columns takes as tuned now, in the
+        order of launch: (first layer, layers, "generic" | "tile" | "stream")."""
+        out, n = (C.c_uint32 * 24)(), C.c_uint32()
+        L.check(L.lib().gs_fft_passes(log_size, log_size if coeffs_log_size is None else coeffs_log_size, n_columns,
+                                      int(inverse), out, C.byref(n)), "fft_passes")
+        return [(out[3 * k], out[3 * k + 1], ("generic", "tile", "stream")[out[3 * k + 2]]) for k in range(n.value)]
+
     # ------------------------------------------------------------ MerkleOps
     @staticmethod
     def commit_on_layer(log_size, prev_layer, columns, ctx=None, out=None):

@@ -1,10 +1,12 @@
 """FFT pass splits and the kernels of their passes, as the library reports
-them without a GPU: the split by size, installed ones (13/4 among them) and
-the way back."""
+them without a GPU: the split by size, installed ones (13/4 among them), the
+way back, and that the cases of test_gpu_fft_stream.py reach every shape of
+the streaming kernel."""
 import pytest
 
 pytest.importorskip("torch")
 
+import test_gpu_fft_stream as stream  # noqa: E402
 from gpustark.backend import GpuBackend as B  # noqa: E402
 
 
@@ -45,3 +47,17 @@ def test_passes_are_refused_outside_the_range():
         with pytest.raises(GpuStarkError):
             B.fft_passes(*bad)
     assert B.fft_passes(1) == [] and B.fft_passes(2, 1) == []  # closed forms
+
+
+def test_the_stream_cases_reach_every_shape():
+    want = {(lo, n) for lo, sizes in ((False, range(5, 14)), (True, range(5, 10))) for n in sizes}
+    seen = {False: set(), True: set()}
+    for log, ext, n_cols, tile, coalesce in stream.SHAPES:
+        B.fft_set_tuning(0, tile, coalesce)
+        seen[False] |= {(lo > 0, n) for lo, n, k in B.fft_passes(log + ext, log, n_cols) if k == "stream"}
+    for log, n_cols, tile, coalesce, sizes in stream.INVERSE:
+        B.fft_set_tuning(0, tile, coalesce)
+        passes = B.fft_passes(log, log, n_cols, True)
+        assert [p[1] for p in passes] == sizes and passes[0][2] == passes[-1][2] == "stream"
+        seen[True] |= {(lo > 0, n) for lo, n, k in B.fft_passes(log, log, n_cols, True) if k == "stream"}
+    assert seen[False] == want and seen[True] == want

@@ -185,7 +185,8 @@ __device__ __forceinline__ void blake2s_quad_table(uint32_t tab[40]) {
   GS_QUAD_ROW(5); GS_QUAD_ROW(6); GS_QUAD_ROW(7); GS_QUAD_ROW(8); GS_QUAD_ROW(9);
 #undef GS_QUAD_ROW
 }
-// h0, h1: words j and 4 + j of the hash. All 32 lanes take part.
+// h0, h1: words j and 4 + j of the hash. All 32 lanes take part; a barrier lies
+// between the stores of the message (and the table) by other lanes and this.
 __device__ __forceinline__ void blake2s_quad(const uint32_t* tab, const uint4* msg, uint32_t bytes, uint32_t& h0,
                                              uint32_t& h1) {
   const uint32_t j = threadIdx.x & 3u;
@@ -198,7 +199,7 @@ __device__ __forceinline__ void blake2s_quad(const uint32_t* tab, const uint4* m
 #pragma unroll
     for (int k = 0; k < 4; k++) at[k] = __dp4a(offsets, 1u << (8 * k), base);
 #pragma unroll
-    for (int k = 0; k < 4; k++) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[k]) : "r"(at[k]));
+    for (int k = 0; k < 4; k++) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[k]) : "r"(at[k]) : "memory");
   };
   uint32_t m[4], next[4];
   fetch(tab[j], m);

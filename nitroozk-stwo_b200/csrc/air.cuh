@@ -60,8 +60,6 @@ struct HashRun {
   uint32_t first, count;
   uint32_t out, pad;
 };
-int gather_hash_runs(cudaStream_t st, const HashRun* d_runs, uint32_t n_runs, const uint32_t* d_idx,
-                     uint32_t* d_out);
 // Values of n_cols columns at a list of positions, written position-major
 // (for each position, every column): columns given explicitly (n_cols <= 4)
 // or as base + c * stride.
@@ -73,9 +71,7 @@ struct ColGather {
   uint64_t pos_off;  // first position in the shared position list
   uint64_t out_off;  // first output word
 };
-int gather_cols(cudaStream_t st, const ColGather* d_blocks, uint32_t n_blocks, uint32_t max_items,
-                const uint32_t* d_positions, uint32_t* d_out);
-// Both gathers in one launch: the column values to d_words, the hashes to
+// Both in one launch: the column values to d_words, the hashes to
 // d_hashes (16-byte aligned). The outputs may be mapped host memory.
 int gather_all(cudaStream_t st, const ColGather* d_blocks, uint32_t n_blocks, uint32_t max_items,
                const uint32_t* d_positions, uint32_t* d_words, const HashRun* d_runs, uint32_t n_runs,

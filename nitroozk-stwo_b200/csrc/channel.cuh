@@ -1,7 +1,8 @@
 // Device-side Fiat-Shamir step of the Blake2s channel (Blake2sChannel::
 // mix_root followed by draw_secure_felt, crates/stwo/src/core/channel/
-// blake2s.rs), shared by the stand-alone channel kernel and the fused FRI
-// tail kernel. Run by one warp, four lanes per compression.
+// blake2s.rs), run at the end of a tree's launch (merkle_tree_kernel, the legacy
+// merkle_tail_kernel) and between the layers of the fused FRI tail. Run by one
+// warp, four lanes per compression.
 //
 //   mix_root:    digest <- Blake2s(digest || root), n_draws <- 0
 //   draw_u32s:   Blake2s(digest || n_draws (LE u32) || 0x00), n_draws += 1

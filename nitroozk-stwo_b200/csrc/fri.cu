@@ -31,12 +31,6 @@ __device__ __forceinline__ void leaf_hash4(uint32_t* leaf_out, size_t i, qm31 v,
   o[1] = make_uint4(h[4], h[5], h[6], h[7]);
 }
 
-__device__ __forceinline__ void store_hash8(uint32_t* out, size_t i, const uint32_t h[8]) {
-  uint4* o = reinterpret_cast<uint4*>(out + 8 * i);
-  o[0] = make_uint4(h[0], h[1], h[2], h[3]);
-  o[1] = make_uint4(h[4], h[5], h[6], h[7]);
-}
-
 __device__ __forceinline__ void load_pair(CPlanes s, size_t i, qm31& a, qm31& b) {
   uint2 p0 = __ldg(reinterpret_cast<const uint2*>(s.p[0]) + i);
   uint2 p1 = __ldg(reinterpret_cast<const uint2*>(s.p[1]) + i);
@@ -314,15 +308,6 @@ int fri_tail(cudaStream_t st, const FriTail& a, uint32_t* d_state, const uint32_
   note_launch();
   GS_CUDA_TRY(cudaGetLastError());
   return OK;
-}
-
-int fold_line(cudaStream_t st, CPlanes src, uint32_t log_n, qm31 alpha, Planes dst, const uint32_t* d_itwiddles,
-              uint32_t tw_log) {
-  return fold_line_fused(st, src, log_n, alpha, dst, d_itwiddles, tw_log, nullptr);
-}
-int fold_circle_into_line(cudaStream_t st, CPlanes src, uint32_t log_n, qm31 alpha, Planes dst,
-                          const uint32_t* d_itwiddles, uint32_t tw_log) {
-  return fold_circle_into_line_fused(st, src, log_n, alpha, dst, d_itwiddles, tw_log, nullptr);
 }
 
 }  // namespace gs

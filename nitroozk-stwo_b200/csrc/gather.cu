@@ -6,54 +6,10 @@
 
 namespace gs {
 
-// One block per run: the run's witnesses are spread over its threads, each
-// copying one 32-byte hash as two 16-byte vectors.
-__global__ void gather_hash_runs_kernel(const HashRun* __restrict__ runs, const uint32_t* __restrict__ idx,
-                                        uint32_t* __restrict__ out) {
-  const HashRun r = runs[blockIdx.x];
-  for (uint32_t k = threadIdx.x; k < r.count; k += blockDim.x) {
-    const uint4* s = reinterpret_cast<const uint4*>(r.src + 8 * (size_t)__ldg(idx + (size_t)r.first + k));
-    uint4* o = reinterpret_cast<uint4*>(out + 8 * ((size_t)r.out + k));
-    o[0] = __ldg(s);
-    o[1] = __ldg(s + 1);
-  }
-}
-
-// grid.y = descriptor, grid.x covers its n_pos * n_cols outputs.
-__global__ void gather_cols_kernel(const ColGather* __restrict__ blocks, const uint32_t* __restrict__ positions,
-                                   uint32_t* __restrict__ out) {
-  const ColGather b = blocks[blockIdx.y];
-  const uint32_t n = b.n_pos * b.n_cols;
-  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    const uint32_t p = t / b.n_cols, c = t - p * b.n_cols;
-    const uint32_t* src = b.n_cols <= 4 ? b.cols[c] : b.base + c * b.stride;
-    out[b.out_off + t] = __ldg(src + positions[b.pos_off + p]);
-  }
-}
-
-int gather_cols(cudaStream_t st, const ColGather* d_blocks, uint32_t n_blocks, uint32_t max_items,
-                const uint32_t* d_positions, uint32_t* d_out) {
-  if (n_blocks == 0 || max_items == 0) return OK;
-  GS_REQUIRE(n_blocks <= 65535, "too many gather descriptors");
-  dim3 grid((max_items + 255) / 256 < 64 ? (max_items + 255) / 256 : 64, n_blocks);
-  gather_cols_kernel<<<grid, 256, 0, st>>>(d_blocks, d_positions, d_out);
-  note_launch();
-  GS_CUDA_TRY(cudaGetLastError());
-  return OK;
-}
-
-int gather_hash_runs(cudaStream_t st, const HashRun* d_runs, uint32_t n_runs, const uint32_t* d_idx,
-                     uint32_t* d_out) {
-  if (n_runs == 0) return OK;
-  GS_REQUIRE(((uintptr_t)d_out & 15) == 0, "hash gather output must be 16-byte aligned");
-  gather_hash_runs_kernel<<<n_runs, 128, 0, st>>>(d_runs, d_idx, d_out);
-  note_launch();
-  GS_CUDA_TRY(cudaGetLastError());
-  return OK;
-}
-
-// The two gathers above in one grid: blocks [0, n_blocks * X) take the
-// column descriptors (X blocks each), the rest one hash run each.
+// One grid: blocks [0, n_blocks * X) take the column descriptors (X blocks
+// each, spread over the descriptor's n_pos * n_cols outputs), the rest one hash
+// run each, its witnesses spread over the block's threads (32 bytes as two
+// 16-byte vectors).
 __global__ void __launch_bounds__(256) gather_all_kernel(const ColGather* __restrict__ blocks, uint32_t n_blocks,
                                                          uint32_t X, const uint32_t* __restrict__ positions,
                                                          uint32_t* words, const HashRun* __restrict__ runs,

@@ -586,7 +586,7 @@ int commit_node_layers_ch(cudaStream_t st, uint32_t top_log, uint32_t* const* la
       GS_REQUIRE(((uintptr_t)layers[k] & 15) == 0, "hash buffers must be 16-byte aligned");
       tp.p[k] = layers[k];
     }
-    // units of 2^9 children (256 threads): 2^8 (440 -> 464 us of tree
+    // units of 2^9 children (timed with 256 threads): 2^8 (440 -> 464 us of tree
     // kernels per Poseidon2 2^18 proof), 2^7 (854 us) and 2^10 (449 us) were
     // slower
     constexpr int unit = 9;

@@ -12,8 +12,6 @@
 namespace gs {
 int fold_line_fused(cudaStream_t st, CPlanes src, uint32_t log_n, qm31 alpha, Planes dst, const uint32_t* d_itw,
                     uint32_t tw_log, uint32_t* leaf_out);
-int fold_circle_into_line_fused(cudaStream_t st, CPlanes src, uint32_t log_n, qm31 alpha, Planes dst,
-                                const uint32_t* d_itw, uint32_t tw_log, uint32_t* leaf_out);
 int fold_line_dev_alpha(cudaStream_t st, CPlanes src, uint32_t log_n, const uint32_t* d_alpha, Planes dst,
                         const uint32_t* d_itw, uint32_t tw_log, uint32_t* leaf_out);
 int fold_circle_fresh(cudaStream_t st, CPlanes src, uint32_t log_n, qm31 alpha, Planes dst, const uint32_t* d_itw,
@@ -270,8 +268,6 @@ struct Prover {
     return OK;
   }
 };
-
-static bool pt_eq(const ptq& a, const ptq& b) { return qm_eq(a.x, b.x) && qm_eq(a.y, b.y); }
 
 // Line interpolation of the last FRI layer (prover/line.rs:45-70) on
 // half_odds(log) from bit-reversed values; returns LinePoly coefficients in

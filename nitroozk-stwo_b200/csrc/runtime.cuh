@@ -300,7 +300,7 @@ int precompute_twiddles(cudaStream_t st, uint32_t initial_index, uint32_t step_i
                         uint32_t* d_twiddles, uint32_t* d_itwiddles);
 int batch_inverse(cudaStream_t st, const uint32_t* d_in, uint32_t* d_out, size_t n);
 
-// fft.cu (columns given by a device table of pointers)
+// fft.cu
 int interpolate_columns(cudaStream_t st, MutCols cols, uint32_t n_cols, uint32_t log_n,
                         const uint32_t* d_itwiddles, uint32_t tw_log);
 // One FFT of a work-list: interpolate (inverse != 0) 2^log evaluations, or
@@ -399,12 +399,6 @@ struct FriTail {
   uint32_t* felts = nullptr;  // 8 words per committed layer (challenge, square)
 };
 int fri_tail(cudaStream_t st, const FriTail& a, uint32_t* d_state, const uint32_t* d_itw, uint32_t tw_log);
-
-// fri.cu
-int fold_line(cudaStream_t st, CPlanes src, uint32_t log_n, qm31 alpha, Planes dst, const uint32_t* d_itwiddles,
-              uint32_t tw_log);
-int fold_circle_into_line(cudaStream_t st, CPlanes src, uint32_t log_n, qm31 alpha, Planes dst,
-                          const uint32_t* d_itwiddles, uint32_t tw_log);
 
 // quotients.cu
 // vec: every column pointer and output plane is 16-byte aligned (4 rows per

@@ -735,10 +735,10 @@ static void split_layers(uint32_t layers, FftTuning tn, std::vector<std::pair<ui
 // it saves a pass. 158 columns of 2^18: 9 + 9 layers (13/4) 167 us interpolated
 // and 306 extended by 1, 10 + 8 (12/4) 159 and 292; 17 layers of 128 columns,
 // 10 + 7 against 8 + 9, 63 against 72. Over 13..24 layers of 1 to 256 columns,
-// extended by 0 to 2, it is within 7% (mostly 3%) of the best of 13/4, 12/4,
-// 12/5, 13/5, 11/5 and 10/4, except at 22 layers of up to 4 columns: three
-// passes (10/4 or 11/5) take 0.90 to 0.97 of 13 + 9. 13/4 at every size takes
-// up to 1.19 times as long.
+// extended by 0 to 2, it is within 8% of the best of 13/4, 12/4, 12/5, 13/5,
+// 11/5 and 10/4, at nine shapes in ten within 3%, except at 22 layers of few
+// columns, where its two passes take 1.03 to 1.11 times as long as three. 13/4
+// at every size takes up to 1.19 times as long.
 static FftTuning split_by_size(uint32_t layers) {
   FftTuning best{13, 4};
   size_t best_passes = 99, best_stages = 0;

@@ -76,3 +76,28 @@ def test_captured_and_replayed(B):
         graph.replay()
         torch.cuda.synchronize()
         assert all(torch.equal(a, b) for a, b in zip(out[0] + out[1], want[0] + want[1]))
+
+
+@pytest.mark.parametrize("log,n,off", [(6, 3, 1), (13, 20, 1), (18, 4, 0), (18, 4, 1)])
+def test_layers_right_behind_the_kernels_they_read(B, log, n, off):
+    """Layers of a thread per node, over columns and children that the kernels
+    before them in the stream write."""
+    tw = B.precompute_twiddles(log)
+    for seed in range(4):
+        got = []
+        for idle in (False, True):
+            rows = torch.stack(columns(log, n, seed))
+            mem = torch.zeros(n, (1 << log) + 4, dtype=torch.int32, device="cuda")
+            cols = [r[off:off + (1 << log)] for r in mem]
+            mem[:, off:off + (1 << log)] = rows
+            kids = torch.zeros(16 << log, dtype=torch.int32, device="cuda")
+            torch.cuda.synchronize()
+            B.interpolate_columns(cols, log, tw)
+            B.commit_on_layer(log + 1, None, [torch.cat([c, c]) for c in cols], out=kids)
+            if idle:
+                torch.cuda.synchronize()
+            layer = B.commit_on_layer(log, kids, cols)
+            if idle:
+                torch.cuda.synchronize()
+            got.append(B.commit_on_layer(log - 1, layer, []))
+        assert torch.equal(*got)
